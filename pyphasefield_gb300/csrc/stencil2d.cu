@@ -155,82 +155,152 @@ __global__ void __launch_bounds__(kThreads)
 // Lean depth-1 kernel: a warp owns WW = 32 V columns (V cells of one
 // 16-byte vector per lane) and kRB rows. It requests the kRB + 2 rows it
 // reads (band plus halo rows) as vector loads up front, takes the west /
-// east neighbours across lanes by shuffles (lanes 0 and 31 load the strip's
-// outer neighbours), and writes each output row as one vector per lane: no
-// shared memory, no barriers. Edge bands use the generic ghost rule.
-constexpr int kRB = 8;
+// east neighbours across lanes by shuffles (the strip's outer neighbours are
+// loaded by its first and last lane), and writes each output row as one
+// vector per lane: no shared memory, no barriers.
+//
+// Bound: HBM on grids beyond L2, the latency of one round of loads below.
+// The grid's edges therefore take the same path: a ghost row is read from
+// its source row and fixed after the load (RowRule), a ghost column is one
+// more load of the lane beside it (ColumnRule), and a vector that reaches
+// past nx is loaded cell by cell. Fetching every cell of an edge band and its
+// neighbours through the per-cell rule chained up to 160 dependent loads per
+// lane and set the time of every grid (diffusion, us per step, before ->
+// after: 256^2 30.3 -> 2.1, 1024^2 30.2 -> 2.8, 4096^2 52.7 -> 20.5, 8192^2
+// 113.5 -> 77.4, which is 6.9 TB/s).
+//
+// Two rows per warp: the halo rows are shared through the caches, and the
+// four times as many warps hide the latency better than eight rows' deeper
+// batch of loads does (eight rows: 256^2 3.2 us, 1024^2 3.3, 4096^2 22.0,
+// 8192^2 79.7; float64 1024^2 17.6 against 14.7).
+constexpr int kRB = 2;
+
+template <typename T>
+struct RowRule {
+  int src;           // source row
+  bool ghost, fixed;
+  T add;             // Dirichlet value, or the shift added to the loaded value
+  __device__ __forceinline__ RowRule(const Geo& g, const Bc<T>& bc, int y) {
+    const int n = g.n[0];
+    src = y;
+    ghost = (unsigned)y >= (unsigned)n;
+    fixed = false;
+    add = T(0);
+    if (!ghost) return;
+    const int side = y < 0 ? 0 : 1;
+    if (bc.type[0] == PPF_BC_PERIODIC) {
+      src = wrap_index(y, n);
+    } else if (bc.type[0] == PPF_BC_NEUMANN) {
+      src = mirror_index(y, n);
+      add = bc.shift[0][0][side];
+    } else {
+      src = y < 0 ? 0 : n - 1;
+      fixed = true;
+      add = bc.shift[0][0][side];
+    }
+  }
+};
+
+// A lane's V cells x .. x + V - 1 of one row: a vector where it lies inside
+// the row and the rows are 16-byte aligned, else the cells below nx one by
+// one (zeros past them).
+template <typename T, int V>
+__device__ __forceinline__ void load_cells(const T* __restrict__ row, int x, int nx, bool vec,
+                                           T (&v)[V]) {
+  using VT = typename Vec16<T>::type;
+  if (vec) {
+    const VT q = __ldg(reinterpret_cast<const VT*>(row + x));
+    const T* pq = reinterpret_cast<const T*>(&q);
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = pq[e];
+  } else {
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = x + e < nx ? __ldg(row + x + e) : T(0);
+  }
+}
+
+template <typename T, int V>
+__device__ __forceinline__ void store_cells(T* row, int x, int nx, bool vec, const T (&v)[V]) {
+  using VT = typename Vec16<T>::type;
+  if (vec) {
+    VT q;
+    T* pq = reinterpret_cast<T*>(&q);
+#pragma unroll
+    for (int e = 0; e < V; ++e) pq[e] = v[e];
+    *reinterpret_cast<VT*>(row + x) = q;
+  } else {
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+      if (x + e < nx) row[x + e] = v[e];
+  }
+}
 
 template <typename T, typename Op>
 __global__ void __launch_bounds__(kThreads)
-    stencil2d_lean_kernel(Op op, Geo g, Bc<T> bc, const T* __restrict__ in, T* __restrict__ out,
-                          int vec_ok) {
+    stencil2d_lean_kernel(Op op, const __grid_constant__ Geo g, const __grid_constant__ Bc<T> bc,
+                          const T* __restrict__ in, T* __restrict__ out, int vec_ok) {
   constexpr int V = Vec16<T>::n;
-  using VT = typename Vec16<T>::type;
-  constexpr int WW = 32 * V;
+  constexpr int WW = 32 * V, RB = kRB;
   const int lane = threadIdx.x;
   const int x0 = blockIdx.x * WW;
-  const int y0 = (blockIdx.y * (kThreads / 32) + threadIdx.y) * kRB;
+  const unsigned band = blockIdx.y + gridDim.y * blockIdx.z;
+  const int y0 = (int)((band * (kThreads / 32) + threadIdx.y) * RB);
   const int ny = g.n[0], nx = g.n[1];
   pdl_wait();
   pdl_launch_next();
   if (y0 >= ny) return;  // whole warp
-  // full strips whose rows y0 - 1 .. y0 + kRB lie inside the grid take the
-  // vector path; the left / right edge strips fetch their one ghost column
-  // through the boundary rule (lanes 0 / 31 only)
-  const bool fast = vec_ok && x0 + WW <= nx && y0 >= 1 && y0 + kRB + 1 <= ny;
-  if (fast) {
-    const T* base = in + (int64_t)(y0 - 1) * g.pitch + x0;
-    VT r[kRB + 2];
+  const int x = x0 + lane * V;
+  const bool vec = vec_ok && x + V <= nx;
+  const bool rows_in = y0 >= 1 && y0 + RB + 1 <= ny;
+  const bool first = lane == 0;                                // loads the west neighbour
+  const bool last = x < nx && (lane == 31 || x + V >= nx);     // loads the east neighbour
+  const ColumnRule<T, 1> wr(g, bc, x0 - 1), er(g, bc, min(x0 + WW, nx));
+  T c[RB + 2][V], wv[RB], ev[RB];
 #pragma unroll
-    for (int j = 0; j < kRB + 2; ++j)
-      r[j] = __ldg(reinterpret_cast<const VT*>(base + (int64_t)j * g.pitch) + lane);
-    T wv[kRB], ev[kRB];
-#pragma unroll
-    for (int j = 0; j < kRB; ++j) {
-      const T* row = base + (int64_t)(j + 1) * g.pitch;
-      if (lane == 0)
-        wv[j] = x0 >= 1 ? __ldg(row - 1) : fetch<T, 2>(in, g, bc, 0, y0 + j, x0 - 1);
-      else
-        wv[j] = T(0);
-      if (lane == 31)
-        ev[j] = x0 + WW + 1 <= nx ? __ldg(row + WW) : fetch<T, 2>(in, g, bc, 0, y0 + j, x0 + WW);
-      else
-        ev[j] = T(0);
+  for (int j = 0; j < RB + 2; ++j) {
+    // rows past the ghost row feed outputs that are not stored
+    const int y = rows_in ? y0 - 1 + j : RowRule<T>(g, bc, min(y0 - 1 + j, ny)).src;
+    const T* row = in + (int64_t)y * g.pitch;
+    load_cells<T, V>(row, x, nx, vec, c[j]);
+    if (j >= 1 && j <= RB) {
+      wv[j - 1] = first ? __ldg(row + wr.xi) : T(0);
+      ev[j - 1] = last ? __ldg(row + er.xi) : T(0);
     }
-    T* obase = out + (int64_t)y0 * g.pitch + x0 + lane * V;
+  }
+  if (!rows_in) {  // ghost rows above and below the grid (uniform across the warp)
 #pragma unroll
-    for (int j = 1; j <= kRB; ++j) {
-      const T* c = reinterpret_cast<const T*>(&r[j]);
-      const T* n = reinterpret_cast<const T*>(&r[j - 1]);
-      const T* sv = reinterpret_cast<const T*>(&r[j + 1]);
-      T wl = __shfl_up_sync(0xffffffffu, c[V - 1], 1);
-      T er = __shfl_down_sync(0xffffffffu, c[0], 1);
-      if (lane == 0) wl = wv[j - 1];
-      if (lane == 31) er = ev[j - 1];
-      VT o;
-      T* ov = reinterpret_cast<T*>(&o);
+    for (int j = 0; j < RB + 2; ++j) {
+      const RowRule<T> r(g, bc, min(y0 - 1 + j, ny));
+      if (r.ghost) {
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        const T w = e == 0 ? wl : c[e - 1];
-        const T ea = e == V - 1 ? er : c[e + 1];
-        ov[e] = op(c[e], w, ea, n[e], sv[e]);
-      }
-      *reinterpret_cast<VT*>(obase + (int64_t)(j - 1) * g.pitch) = o;
-    }
-  } else {
-    for (int j = 0; j < kRB; ++j) {
-      const int row = y0 + j;
-      if (row >= ny) break;
-#pragma unroll
-      for (int e = 0; e < V; ++e) {
-        const int x = x0 + lane * V + e;
-        if (x < nx)
-          out[(int64_t)row * g.pitch + x] =
-              op(fetch<T, 2>(in, g, bc, 0, row, x), fetch<T, 2>(in, g, bc, 0, row, x - 1),
-                 fetch<T, 2>(in, g, bc, 0, row, x + 1), fetch<T, 2>(in, g, bc, 0, row - 1, x),
-                 fetch<T, 2>(in, g, bc, 0, row + 1, x));
+        for (int e = 0; e < V; ++e) c[j][e] = r.fixed ? r.add : c[j][e] + r.add;
       }
     }
+  }
+#pragma unroll
+  for (int j = 0; j < RB; ++j) {
+    wv[j] = wr.value(0, wv[j]);
+    ev[j] = er.value(0, ev[j]);
+    if (last) {  // the ghost column inside the last lane's vector
+#pragma unroll
+      for (int e = 1; e < V; ++e)
+        if (x + e == nx) c[j + 1][e] = ev[j];
+    }
+  }
+#pragma unroll
+  for (int j = 1; j <= RB; ++j) {
+    T wl = __shfl_up_sync(0xffffffffu, c[j][V - 1], 1);
+    T ee = __shfl_down_sync(0xffffffffu, c[j][0], 1);
+    if (first) wl = wv[j - 1];
+    if (last) ee = ev[j - 1];
+    T o[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const T w = e == 0 ? wl : c[j][e - 1];
+      const T ea = e == V - 1 ? ee : c[j][e + 1];
+      o[e] = op(c[j][e], w, ea, c[j - 1][e], c[j + 1][e]);
+    }
+    if (y0 + j - 1 < ny) store_cells<T, V>(out + (int64_t)(y0 + j - 1) * g.pitch, x, nx, vec, o);
   }
 }
 
@@ -572,9 +642,10 @@ int32_t run2d(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b,
   const bool pdl = tiling && tiling->pdl;
   if (t.k == 1 && !(tiling && tiling->tile_x)) {
     constexpr int WW = 32 * Vec16<T>::n;
-    dim3 grid_dim((g.n[1] + WW - 1) / WW,
-                  (g.n[0] + kRB * (kThreads / 32) - 1) / (kRB * (kThreads / 32)));
-    if (grid_dim.y > 65535) return fail(PPF_ERR_INVALID, "too many row bands");
+    if ((g.n[0] + 63) / 64 > 65535) return fail(PPF_ERR_INVALID, "too many row bands");
+    const unsigned bands = (g.n[0] + kRB * (kThreads / 32) - 1) / (kRB * (kThreads / 32));
+    const unsigned by = bands < 65535 ? bands : 65535;
+    const dim3 grid_dim((g.n[1] + WW - 1) / WW, by, (bands + by - 1) / by);
     PPF_TRY_CUDA(launch(stencil2d_lean_kernel<T, Op>, grid_dim, dim3(32, kThreads / 32), 0,
                         (cudaStream_t)stream, pdl, op, g, bc, in, out, vec_ok));
     return PPF_OK;

@@ -1,0 +1,60 @@
+"""2-D Diffusion / Allen-Cahn kernels at the sizes where their edge handling
+changes: rows and columns around a vector, a warp's strip and its bands."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import restate
+from tests.helpers import make_structs, rel_l2, run_single_gpu
+
+pytestmark = pytest.mark.gpu
+
+BCS = ["PERIODIC", "NEUMANN", "DIRCHLET", ["DIRCHLET", "PERIODIC"], ["NEUMANN", "DIRCHLET"]]
+
+
+def face_values(bc, nd=2):
+    bcs = [bc] * nd if isinstance(bc, str) else bc
+    return [[[0.25, 0.5] if b != "PERIODIC" else [0.0, 0.0] for b in bcs]]
+
+
+@pytest.mark.parametrize("shape", [(1, 4), (2, 5), (3, 1), (15, 127), (16, 128), (17, 129),
+                                   (18, 258), (33, 63), (5, 64), (4, 65)])
+@pytest.mark.parametrize("bc", BCS, ids=str)
+def test_single_step_edges(cuda, shape, bc):
+    """Depth 1 against the tile kernel, whose every edge cell goes through the
+    per-cell rule (bit for bit), and the float64 oracle; gradients and fixed
+    values on the faces."""
+    c0 = np.random.default_rng(5).random(shape)
+    vals = face_values(bc)
+    kw = dict(M=0.1, epsilon=1.0, W=1.0)
+    for prec in ("fp32", "fp64"):
+        a = run_single_gpu("allen_cahn", c0, 3, bc, 1.0, 0.1, values=vals, precision=prec, **kw)
+        b = run_single_gpu("allen_cahn", c0, 3, bc, 1.0, 0.1, values=vals, precision=prec,
+                           tile=(64, 8), **kw)
+        np.testing.assert_array_equal(a, b)
+    ref = restate.run_single("allen_cahn", c0, 3, bc, 1.0, 0.1, values=vals, **kw)
+    assert rel_l2(a, ref) < 1e-12
+
+
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_single_step_misaligned_rows(cuda, offset):
+    """Field pointers off the 16-byte boundary take scalar loads and stores,
+    with the same result."""
+    import torch
+    from pyphasefield_gb300 import _lib as L
+    shape = (37, 131)
+    g, b, _, pitch = make_structs(shape, "NEUMANN")
+    c0 = np.random.default_rng(6).random(shape)
+    p = L.PpfDiffusionParams(1.0, 0.1, 1.0)
+    t = L.PpfTiling(depth=1)
+    got = []
+    for off in (0, offset):
+        bufs = [torch.zeros(shape[0] * pitch + 8, device="cuda")[off:off + shape[0] * pitch]
+                for _ in range(2)]
+        bufs[0].view(shape[0], pitch)[:, :shape[1]] = torch.from_numpy(c0)
+        L.call("ppf_diffusion_step_f32", C.byref(p), C.byref(g), C.byref(b),
+               C.c_void_p(bufs[0].data_ptr()), C.c_void_p(bufs[1].data_ptr()), C.byref(t),
+               C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        got.append(bufs[1].view(shape[0], pitch)[:, :shape[1]].cpu().numpy())
+    np.testing.assert_array_equal(got[0], got[1])
