@@ -1,9 +1,11 @@
 // 2-D Diffusion and Allen-Cahn explicit steps, one or several per pass.
 //
 // Kernels: stencil2d_lean_kernel (one step, warp strips of 16-byte
-// vectors, the default), stencil2d_march_kernel (depth 2..8 steps per HBM
-// pass: warps march down column windows fed by TMA, a pipeline of one
-// register stage per step) and stencil2d_tb_kernel (depth steps on a
+// vectors), stencil2d_block_kernel (float, depth 2..8 steps per pass with the
+// block in registers), stencil2d_march_kernel (depth 2..8 in double, and in
+// float where a segment length is asked for: warps march down column windows
+// fed by TMA, a pipeline of one register stage per step) and
+// stencil2d_tb_kernel (depth steps on a
 // TY x TX shared-memory tile with a halo of `depth` cells, used when a tile
 // shape is asked for). Every kernel reads each cell once and writes it once
 // per pass, applying the ghost rule at load time.
@@ -12,6 +14,7 @@
 // engine_CahnAllenExplicit (Engines/CahnAllen.py:128-135), with Field.laplacian
 // (field.py:60-67) as the 5-point stencil.
 #include "ppf_common.cuh"
+#include "ppf_pack.cuh"
 #include "ppf_tma.cuh"
 
 namespace ppf {
@@ -19,13 +22,16 @@ namespace {
 
 // c + dt*D*lap(c). The neighbour sum is grouped ((w+e)+(n+s)) so that a
 // mirrored tile (no-flux ghosts deeper than one cell) evolves bit-identically
-// to the cells it mirrors.
+// to the cells it mirrors. The multiply-adds are written out, so that the
+// scalar and the packed form (two cells; we = w + e, ns = n + s) round alike.
 template <typename T>
 struct DiffusionOp {
   T r;  // dt*D/dx^2
   __device__ __forceinline__ T operator()(T c, T w, T e, T n, T s) const {
-    const T lap = ((w + e) + (n + s)) - T(4) * c;
-    return c + r * lap;
+    return fma(r, fma(T(-4), c, (w + e) + (n + s)), c);
+  }
+  __device__ __forceinline__ F2 pair(F2 c, F2 we, F2 ns) const {
+    return fma2(sp(r), fma2(sp(-4.f), c, we + ns), c);
   }
 };
 
@@ -35,9 +41,14 @@ struct AllenCahnOp {
   T a;  // dt*M*eps^2/dx^2
   T b;  // dt*M*16*W
   __device__ __forceinline__ T operator()(T c, T w, T e, T n, T s) const {
-    const T lap = ((w + e) + (n + s)) - T(4) * c;
-    const T fp = c * (T(2) + c * (T(-6) + T(4) * c));
-    return c + (a * lap - b * fp);
+    const T lap = fma(T(-4), c, (w + e) + (n + s));
+    const T fp = c * fma(c, fma(T(4), c, T(-6)), T(2));
+    return c + fma(a, lap, -b * fp);
+  }
+  __device__ __forceinline__ F2 pair(F2 c, F2 we, F2 ns) const {
+    const F2 lap = fma2(sp(-4.f), c, we + ns);
+    const F2 fp = c * fma2(c, fma2(sp(4.f), c, sp(-6.f)), sp(2.f));
+    return c + fma2(sp(a), lap, sp(-b) * fp);
   }
 };
 
@@ -519,6 +530,127 @@ __global__ void __launch_bounds__(32 * kMWarps, (MarchMinBlocks<T, K>::value))
   }
 }
 
+// ------------------------------------------------------------ register block
+// Several steps per pass with the block in registers (float). A CTA of NW
+// warps owns NW x R rows of a 32 V column window; a lane keeps R rows of one
+// 16-byte vector. Every step a warp leaves its first and last row in shared
+// memory (two buffers by the step's parity, so one barrier per step), takes
+// the rows above and below from its neighbours, west / east cells by shuffles,
+// and advances its cells in place. After `depth` steps the outer `depth` rows
+// and KA = depth rounded up to V columns per side are stale; the CTA stores
+// the cells inside. HBM and L2 see one read and one write per `depth` steps,
+// and a grid that fits the caches runs `depth` steps on one launch.
+//
+// Cells outside the grid are loaded by the boundary rule and then evolve as in
+// the marching kernel: copies (periodic wrap, no-flux mirror) follow their
+// images bit for bit, Dirichlet ghosts keep their value.
+template <typename Op, int R, int NW>
+__global__ void __launch_bounds__(32 * NW, 2)
+    stencil2d_block_kernel(Op op, const __grid_constant__ Geo g,
+                           const __grid_constant__ Bc<float> bc, const float* __restrict__ in,
+                           float* __restrict__ out, int depth, int ka) {
+  constexpr int WW = 128, H = NW * R;
+  __shared__ float4 edge[2][NW][2][32];
+  const int lane = threadIdx.x, wid = threadIdx.y;
+  const int ny = g.n[0], nx = g.n[1];
+  const int xs = (int)blockIdx.x * (WW - 2 * ka) - ka;
+  const int ys = (int)(blockIdx.y + gridDim.y * blockIdx.z) * (H - 2 * depth) - depth;
+  const int x = xs + lane * 4, yw = ys + wid * R;
+  pdl_wait();
+  pdl_launch_next();
+  F2 c[R][2];
+  uint32_t fix = 0;    // this lane's columns that never change
+  bool edges = false;  // the window reaches outside the grid (uniform across the CTA)
+  if (xs >= 0 && xs + WW <= nx && ys >= 0 && ys + H <= ny) {
+    const float* p = in + (int64_t)yw * g.pitch + x;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(p + (int64_t)r * g.pitch));
+      c[r][0] = pk(q.x, q.y), c[r][1] = pk(q.z, q.w);
+    }
+  } else {
+    edges = true;
+    float v[R][4];
+    int src[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) src[r] = RowRule<float>(g, bc, yw + r).src;
+    if (x >= 0 && x + 4 <= nx) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        load_cells<float, 4>(in + (int64_t)src[r] * g.pitch, x, nx, true, v[r]);
+    } else {
+      int col[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        col[e] = ColumnRule<float, 1>(g, bc, x + e).xi;
+        if (bc.type[1] == PPF_BC_DIRCHLET && (unsigned)(x + e) >= (unsigned)nx) fix |= 1u << e;
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[r][e] = __ldg(in + (int64_t)src[r] * g.pitch + col[e]);
+    }
+    if (bc.type[0] == PPF_BC_DIRCHLET) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if ((unsigned)(yw + r) >= (unsigned)ny) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[r][e] = bc.shift[0][0][yw + r < 0 ? 0 : 1];
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (fix & (1u << e)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r][e] = bc.shift[0][1][x + e < 0 ? 0 : 1];
+      }
+#pragma unroll
+    for (int r = 0; r < R; ++r) c[r][0] = pk(v[r][0], v[r][1]), c[r][1] = pk(v[r][2], v[r][3]);
+  }
+  const bool fix_y = edges && bc.type[0] == PPF_BC_DIRCHLET;
+
+#pragma unroll 2
+  for (int s = 1; s <= depth; ++s) {
+    float4(*eb)[2][32] = edge[s & 1];
+    eb[wid][0][lane] = make_float4(lo(c[0][0]), hi(c[0][0]), lo(c[0][1]), hi(c[0][1]));
+    eb[wid][1][lane] =
+        make_float4(lo(c[R - 1][0]), hi(c[R - 1][0]), lo(c[R - 1][1]), hi(c[R - 1][1]));
+    __syncthreads();
+    // rows s .. H - 1 - s of the window can still be computed
+    if (wid * R + R - 1 < s || wid * R > H - 1 - s) continue;
+    // the block's first and last warp read their own row: stale rows
+    const float4 a = eb[wid > 0 ? wid - 1 : 0][1][lane];
+    const float4 b = eb[wid < NW - 1 ? wid + 1 : wid][0][lane];
+    F2 prev[2] = {pk(a.x, a.y), pk(a.z, a.w)};
+    const F2 below[2] = {pk(b.x, b.y), pk(b.z, b.w)};
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float c0 = lo(c[r][0]), c1 = hi(c[r][0]), c2 = lo(c[r][1]), c3 = hi(c[r][1]);
+      const float wl = __shfl_up_sync(0xffffffffu, c3, 1);
+      const float er = __shfl_down_sync(0xffffffffu, c0, 1);
+      F2 nxt[2] = {op.pair(c[r][0], pk(wl + c1, c0 + c2),
+                           prev[0] + (r < R - 1 ? c[r < R - 1 ? r + 1 : r][0] : below[0])),
+                   op.pair(c[r][1], pk(c1 + c3, c2 + er),
+                           prev[1] + (r < R - 1 ? c[r < R - 1 ? r + 1 : r][1] : below[1]))};
+      if (fix) {
+        nxt[0] = pk(fix & 1u ? c0 : lo(nxt[0]), fix & 2u ? c1 : hi(nxt[0]));
+        nxt[1] = pk(fix & 4u ? c2 : lo(nxt[1]), fix & 8u ? c3 : hi(nxt[1]));
+      }
+      if (fix_y && (unsigned)(yw + r) >= (unsigned)ny) nxt[0] = c[r][0], nxt[1] = c[r][1];
+      prev[0] = c[r][0], prev[1] = c[r][1];
+      c[r][0] = nxt[0], c[r][1] = nxt[1];
+    }
+  }
+  if (lane * 4 < ka || lane * 4 >= WW - ka) return;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int wr = wid * R + r;
+    const float v[4] = {lo(c[r][0]), hi(c[r][0]), lo(c[r][1]), hi(c[r][1])};
+    if (wr >= depth && wr < H - depth && yw + r < ny)
+      store_cells<float, 4>(out + (int64_t)(yw + r) * g.pitch, x, nx, x + 4 <= nx, v);
+  }
+}
+
 struct Tile2d {
   int tx, ty, k, ka;
   size_t smem;
@@ -617,6 +749,45 @@ int32_t run_march(Op op, const Geo& g, const Bc<T>& bc, const T* in, T* out, int
   }
 }
 
+template <typename Op, int R, int NW>
+int32_t launch_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, float* out,
+                     int depth, bool pdl, cudaStream_t s) {
+  const int ka = (depth + 3) / 4 * 4;
+  const int ow = 128 - 2 * ka, oh = NW * R - 2 * depth;
+  const unsigned bands = (g.n[0] + oh - 1) / oh, by = bands < 65535 ? bands : 65535;
+  const dim3 grid((g.n[1] + ow - 1) / ow, by, (bands + by - 1) / by);
+  PPF_TRY_CUDA(launch(stencil2d_block_kernel<Op, R, NW>, grid, dim3(32, NW), 0, s, pdl, op, g,
+                      bc, in, out, depth, ka));
+  return PPF_OK;
+}
+
+// Block shapes, smallest first. A pass takes as long as its busiest SM, and a
+// block's own time grows with its rows, so the first shape that leaves at most
+// one block per SM wins (diffusion 256^2, us per step: 0.61 with 12 x 2 rows,
+// 0.69 with 16 x 2, 0.80 and 0.89 with 12 and 16 x 4; 512^2: 0.78 with 12 x 4,
+// 0.90 with 16 x 4), then the first of the four-row shapes whose blocks are all
+// resident at two per SM (777 x 1303 Allen-Cahn: 1.28 with 12 x 4, 1.61 with
+// 16 x 4); larger grids take the tallest, which recomputes the fewest halo rows
+// (8192^2: 33.7, and 38.5 with 12 x 4).
+template <typename Op>
+int32_t run_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, float* out, int depth,
+                  bool pdl, cudaStream_t s) {
+  if (((uintptr_t)in) % 16 || ((uintptr_t)out) % 16 || g.pitch % 4)
+    return fail(PPF_ERR_INVALID, "temporal blocking needs 16-byte aligned rows");
+  int dev = 0, sms = 0;
+  PPF_TRY_CUDA(cudaGetDevice(&dev));
+  PPF_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int ow = 128 - 2 * ((depth + 3) / 4 * 4);
+  auto blocks = [&](int rows) {
+    const int oh = rows - 2 * depth;
+    return (long)((g.n[1] + ow - 1) / ow) * ((g.n[0] + oh - 1) / oh);
+  };
+  if (blocks(24) <= sms) return launch_block<Op, 2, 12>(op, g, bc, in, out, depth, pdl, s);
+  if (blocks(32) <= sms) return launch_block<Op, 2, 16>(op, g, bc, in, out, depth, pdl, s);
+  if (blocks(48) <= 2 * sms) return launch_block<Op, 4, 12>(op, g, bc, in, out, depth, pdl, s);
+  return launch_block<Op, 4, 16>(op, g, bc, in, out, depth, pdl, s);
+}
+
 template <typename T, typename Op>
 int32_t run2d(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b,
               const T* in, T* out, const PpfTiling* tiling, void* stream) {
@@ -630,6 +801,10 @@ int32_t run2d(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b,
     if (depth > 8) return fail(PPF_ERR_INVALID, "depth=%d not in [1, 8]", depth);
     Bc<T> bcm;
     if ((rc = make_bc<T>(b, g, dx, 1, depth, &bcm))) return rc;
+    if constexpr (sizeof(T) == 4) {
+      if (!tiling->tile_y)
+        return run_block<Op>(op, g, bcm, in, out, depth, tiling->pdl != 0, (cudaStream_t)stream);
+    }
     return run_march<T, Op>(op, g, bcm, in, out, depth, tiling->tile_y, tiling->pdl != 0,
                             (cudaStream_t)stream);
   }

@@ -6,52 +6,10 @@
 // :50-92); the exact bulk form and the noise stream are unchanged.
 #pragma once
 
-#include <cstdint>
+#include "ppf_pack.cuh"
 
 namespace ppf {
 namespace w95 {
-
-struct F2 {
-  uint64_t v;
-};
-
-__device__ __forceinline__ F2 pk(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ F2 sp(float a) { return pk(a, a); }
-__device__ __forceinline__ float lo(F2 x) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
-  return a;
-}
-__device__ __forceinline__ float hi(F2 x) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
-  return b;
-}
-__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
-  F2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-// a * b + c, one rounding per half
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
 
 // D~ and Q~ (see point() in w95_core.cuh) for two cells at once.
 __device__ __forceinline__ void point2(const Coef<float>& k, F2 phi, F2 c, F2& Dt, F2& Qt) {

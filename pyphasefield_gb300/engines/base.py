@@ -11,14 +11,15 @@ retrieve_fields_from_GPU / apply_boundary_conditions, ppf_gpu_utils.py:
   in two ping-pong buffer sets; the boundary rule is fused into every
   kernel's tile load, so apply_boundary_conditions is a no-op on device;
 * simulate(n) advances n steps in captured CUDA graphs of `graph_chunk`
-  launches (each launch with programmatic dependent launch), split at
+  steps (each launch with programmatic dependent launch), split at
   autosave boundaries so autosave cadence and time_step_counter behave as in
   the reference;
 * send_fields_to_GPU / retrieve_fields_from_GPU move the interiors between
   Field.data (float64, ghosts refilled on the host) and the device.
 
 User-data keys added to the reference's: precision ("fp32" | "fp64"),
-temporal_depth (steps per HBM pass, 2-D Diffusion/Allen-Cahn), tile
+temporal_depth (steps per HBM pass, 2-D Diffusion/Allen-Cahn; 1, the
+default, leaves the steps per pass to the engine), tile
 ((tile_x, tile_y) or None; Warren1995: (0, rows per warp band), chosen by
 grid size when None), zchunk (planes per CTA, 3-D), autotune (bool: time the
 launch shapes on scratch copies and cache the fastest), bulk_shortcut
@@ -120,6 +121,12 @@ class GB300Engine:
         raise NotImplementedError
 
     def _ppf_max_depth(self) -> int:
+        return 1
+
+    def _ppf_auto_depth(self) -> int:
+        """Steps a pass takes on its own account while temporal_depth is 1:
+        more than 1 where the kernels advance several steps per pass with the
+        results of single steps, bit for bit."""
         return 1
 
     def _ppf_encode(self, j: int, x: np.ndarray) -> np.ndarray:
@@ -453,8 +460,17 @@ class GB300Engine:
                     slot["job"] = None
 
     # ------------------------------------------------------------ stepping
-    def _ppf_passes(self, nsteps: int) -> list[int]:
+    def _ppf_passes(self, nsteps: int, even: bool = False) -> list[int]:
+        """Steps of each pass of a run of nsteps. temporal_depth > 1: passes
+        of that depth and a remainder; else as few passes as the engine's own
+        depth allows, of equal depth within one step (even: an even number of
+        them, so that the field ends in the buffers it began in)."""
         k = max(1, min(int(self.user_data.get("temporal_depth", 1)), self._ppf_max_depth()))
+        if k == 1:
+            m = -(-nsteps // self._ppf_auto_depth())
+            if even:
+                m += m & 1
+            return [nsteps // m + (i < nsteps % m) for i in range(m)]
         passes = [k] * (nsteps // k)
         if nsteps % k:
             passes.append(nsteps % k)
@@ -527,40 +543,38 @@ class GB300Engine:
         if nsteps <= 0:
             return
         self._ppf_done = 0
-        passes = self._ppf_passes(nsteps)
         ud = self.user_data
         chunk = max(2, int(ud.get("graph_chunk", 64)) // 2 * 2)
         s = self._ppf_stream
         sp = C.c_void_p(s.cuda_stream)
-        i = 0
         step = step0
-        if ud.get("use_graph", True) and len(passes) >= chunk:
-            depths = tuple(passes[:chunk])
-            if all(d == depths[0] for d in depths):
-                g = self._ppf_graph(depths)
-                span = sum(depths)
-                with torch.cuda.stream(s):
-                    self._ppf_stepctr.fill_(step)
-                while len(passes) - i >= chunk:
-                    self._ppf_check_status(False)
-                    with nvtx_range(f"ppf.graph {span} steps from {step}"):
-                        L.call("ppf_graph_launch", g, sp)
-                    self._ppf_mark()
-                    self._ppf_segment_end(span, s)
-                    i += chunk
-                    step += span
-                    self._ppf_done += span
-        if i < len(passes):
+        # a graph holds `chunk` passes of temporal_depth steps, or `chunk`
+        # steps in passes of the engine's own depth
+        k = max(1, min(int(ud.get("temporal_depth", 1)), self._ppf_max_depth()))
+        span = chunk * k
+        if ud.get("use_graph", True) and nsteps >= span:
+            g = self._ppf_graph(tuple(self._ppf_passes(span, even=True)))
+            with torch.cuda.stream(s):
+                self._ppf_stepctr.fill_(step)
+            while nsteps >= span:
+                self._ppf_check_status(False)
+                with nvtx_range(f"ppf.graph {span} steps from {step}"):
+                    L.call("ppf_graph_launch", g, sp)
+                self._ppf_mark()
+                self._ppf_segment_end(span, s)
+                nsteps -= span
+                step += span
+                self._ppf_done += span
+        if nsteps:
             self._ppf_check_status(False)
-            rest = passes[i:]
-            with torch.cuda.stream(s), nvtx_range(f"ppf.eager {sum(rest)} steps from {step}"):
-                self._ppf_segment_begin(sum(rest), s)
-                for d in rest:
+            with torch.cuda.stream(s), nvtx_range(f"ppf.eager {nsteps} steps from {step}"):
+                self._ppf_segment_begin(nsteps, s)
+                for d in self._ppf_passes(nsteps):
                     self._ppf_launch_pass(d, step, None)
                     step += d
                 self._ppf_watch(s)
             self._ppf_mark()
-            self._ppf_segment_end(sum(rest), s)
+            self._ppf_segment_end(nsteps, s)
 
     # ------------------------------------------------------------ access
     def device_fields(self) -> list[torch.Tensor]:

@@ -112,6 +112,22 @@ def _stencil_candidates(sim) -> list:
         [{"tile": t} for t in ((64, 16), (32, 16), (128, 8))]
 
 
+def _stencil_auto_depth(sim) -> int:
+    """Steps per pass of the 2-D float kernels on their own account: eight
+    where no tile is asked for and the depth is exact (a ghost cell with a
+    gradient has no image to follow beyond one step). In double a step is
+    bound by the FP64 units, and recomputed halo cells would cost more than
+    the pass saves."""
+    if len(sim._ppf_grid.kshape) != 2 or sim._ppf_dtype != torch.float32 \
+            or sim.user_data.get("tile"):
+        return 1
+    b = sim._ppf_bc
+    if any(b.type[a] == L.PPF_BC_NEUMANN and (b.value[0][a][0] or b.value[0][a][1])
+           for a in range(2)):
+        return 1
+    return 8
+
+
 _SOLVERS = {"explicit": L.PPF_SOLVER_EXPLICIT, "implicit": L.PPF_SOLVER_IMPLICIT,
             "crank-nicolson": L.PPF_SOLVER_CRANK_NICOLSON}
 
@@ -180,6 +196,9 @@ class _DiffusionMixin(GB300Engine):
             return 1
         return 8 if len(self._ppf_grid.kshape) == 2 else 1
 
+    def _ppf_auto_depth(self):
+        return 1 if self._ppf_solver != L.PPF_SOLVER_EXPLICIT else _stencil_auto_depth(self)
+
     def _ppf_tune_candidates(self):
         if self._ppf_solver != L.PPF_SOLVER_EXPLICIT:
             return []
@@ -247,6 +266,9 @@ class _CahnAllenMixin(_ImplicitPhase, GB300Engine):
         if self._ppf_phase_solver is not None:
             return 1
         return 8 if len(self._ppf_grid.kshape) == 2 else 1
+
+    def _ppf_auto_depth(self):
+        return 1 if self._ppf_phase_solver is not None else _stencil_auto_depth(self)
 
     def _ppf_tune_candidates(self):
         return [] if self._ppf_phase_solver is not None else _stencil_candidates(self)

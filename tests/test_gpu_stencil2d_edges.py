@@ -58,3 +58,40 @@ def test_single_step_misaligned_rows(cuda, offset):
                C.c_void_p(torch.cuda.current_stream().cuda_stream))
         got.append(bufs[1].view(shape[0], pitch)[:, :shape[1]].cpu().numpy())
     np.testing.assert_array_equal(got[0], got[1])
+
+
+# one grid per block shape of the several-step kernel, odd sides
+@pytest.mark.parametrize("shape", [(3, 7), (61, 203), (501, 301), (777, 515), (1101, 2103)])
+@pytest.mark.parametrize("depth", [2, 5, 8])
+def test_block_kernel_equals_single_steps(cuda, shape, depth):
+    """Passes of several steps (float) equal single steps bit for bit."""
+    c0 = np.random.default_rng(7).random(shape)
+    for model, kw in (("diffusion", dict(D=1.0)), ("allen_cahn", dict(M=0.1, epsilon=1.0, W=1.0))):
+        for bc in BCS:
+            vals = [[v if b == "DIRCHLET" else [0.0, 0.0]
+                     for v, b in zip(face_values(bc)[0], [bc] * 2 if isinstance(bc, str) else bc)]]
+            a = run_single_gpu(model, c0, depth + 2, bc, 1.0, 0.1, values=vals, precision="fp32", **kw)
+            b = run_single_gpu(model, c0, depth + 2, bc, 1.0, 0.1, values=vals, precision="fp32",
+                               depth=depth, **kw)
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("steps", [1, 7, 50, 100, 131])
+@pytest.mark.parametrize("gradient", [0.0, 0.5])
+def test_engine_default_depth_equals_single_steps(cuda, steps, gradient):
+    """The engine's own steps per pass (graphs and the remainder) against
+    one launch per step; a face gradient keeps single steps."""
+    from pyphasefield_gb300 import DiffusionGB300
+    c0 = np.random.default_rng(8).random((70, 150))
+    vals = [[[gradient, 0.0], [0.0, 0.0]]]
+    sim = DiffusionGB300(dimensions=[70, 150], dx=1.0, dt=0.1, boundary_conditions="NEUMANN",
+                         user_data={"D": 1.0, "graph_chunk": 24})
+    sim.initialize_fields_and_imported_data()
+    sim._boundary_conditions_array[0][0, :] = gradient
+    sim.fields[0].data[1:-1, 1:-1] = c0
+    sim.simulate(steps)
+    assert sim._ppf_auto_depth() == (8 if gradient == 0 else 1)
+    sim.retrieve_fields_from_GPU()
+    ref = run_single_gpu("diffusion", c0, steps, "NEUMANN", 1.0, 0.1, values=vals,
+                         precision="fp32", D=1.0)
+    np.testing.assert_array_equal(sim.fields[0].get_cells(), ref)
