@@ -173,13 +173,13 @@ __device__ __forceinline__ T fetch(const T* __restrict__ f, const Geo& g,
 // loaded)). A strip that crosses the x edge then loads every row straight
 // from one column and fixes its ghost lanes afterwards, instead of a
 // divergent fetch per row. Field f of shift: 0 phi, 1 c (as fetch's fld).
-template <typename T, int NF>
+template <typename T, int NF, int AXIS = 1>
 struct ColumnRule {
   int xi;
   bool ghost, fixed;
   T add[NF];
   __device__ __forceinline__ ColumnRule(const Geo& g, const Bc<T>& bc, int x) {
-    const int n = g.n[1];
+    const int n = g.n[AXIS];
     xi = x;
     ghost = (unsigned)x >= (unsigned)n;
     fixed = false;
@@ -187,18 +187,18 @@ struct ColumnRule {
     for (int f = 0; f < NF; ++f) add[f] = T(0);
     if (!ghost) return;
     const int side = x < 0 ? 0 : 1;
-    const int t = bc.type[1];
+    const int t = bc.type[AXIS];
     if (t == PPF_BC_PERIODIC) {
       xi = wrap_index(x, n);
     } else if (t == PPF_BC_NEUMANN) {
       xi = mirror_index(x, n);
 #pragma unroll
-      for (int f = 0; f < NF; ++f) add[f] = T(0) + bc.shift[f][1][side];
+      for (int f = 0; f < NF; ++f) add[f] = T(0) + bc.shift[f][AXIS][side];
     } else {
       xi = x < 0 ? 0 : n - 1;
       fixed = true;
 #pragma unroll
-      for (int f = 0; f < NF; ++f) add[f] = bc.shift[f][1][side] + T(0);
+      for (int f = 0; f < NF; ++f) add[f] = bc.shift[f][AXIS][side] + T(0);
     }
   }
   __device__ __forceinline__ T value(int f, T loaded) const {

@@ -15,6 +15,7 @@
 // (field.py:60-67) as the 5-point stencil.
 #include "ppf_common.cuh"
 #include "ppf_pack.cuh"
+#include "ppf_rows.cuh"
 #include "ppf_tma.cuh"
 
 namespace ppf {
@@ -50,19 +51,6 @@ struct AllenCahnOp {
     const F2 fp = c * fma2(c, fma2(sp(4.f), c, sp(-6.f)), sp(2.f));
     return c + fma2(sp(a), lap, sp(-b) * fp);
   }
-};
-
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-  using type = float4;
-  static constexpr int n = 4;
-};
-template <>
-struct Vec16<double> {
-  using type = double2;
-  static constexpr int n = 2;
 };
 
 constexpr int kThreads = 256;  // 8 warps; threadIdx.x = lane
@@ -172,7 +160,7 @@ __global__ void __launch_bounds__(kThreads)
 //
 // Bound: HBM on grids beyond L2, the latency of one round of loads below.
 // The grid's edges therefore take the same path: a ghost row is read from
-// its source row and fixed after the load (RowRule), a ghost column is one
+// its source row and fixed after the load (AxisRule), a ghost column is one
 // more load of the lane beside it (ColumnRule), and a vector that reaches
 // past nx is loaded cell by cell. Fetching every cell of an edge band and its
 // neighbours through the per-cell rule chained up to 160 dependent loads per
@@ -185,66 +173,6 @@ __global__ void __launch_bounds__(kThreads)
 // batch of loads does (eight rows: 256^2 3.2 us, 1024^2 3.3, 4096^2 22.0,
 // 8192^2 79.7; float64 1024^2 17.6 against 14.7).
 constexpr int kRB = 2;
-
-template <typename T>
-struct RowRule {
-  int src;           // source row
-  bool ghost, fixed;
-  T add;             // Dirichlet value, or the shift added to the loaded value
-  __device__ __forceinline__ RowRule(const Geo& g, const Bc<T>& bc, int y) {
-    const int n = g.n[0];
-    src = y;
-    ghost = (unsigned)y >= (unsigned)n;
-    fixed = false;
-    add = T(0);
-    if (!ghost) return;
-    const int side = y < 0 ? 0 : 1;
-    if (bc.type[0] == PPF_BC_PERIODIC) {
-      src = wrap_index(y, n);
-    } else if (bc.type[0] == PPF_BC_NEUMANN) {
-      src = mirror_index(y, n);
-      add = bc.shift[0][0][side];
-    } else {
-      src = y < 0 ? 0 : n - 1;
-      fixed = true;
-      add = bc.shift[0][0][side];
-    }
-  }
-};
-
-// A lane's V cells x .. x + V - 1 of one row: a vector where it lies inside
-// the row and the rows are 16-byte aligned, else the cells below nx one by
-// one (zeros past them).
-template <typename T, int V>
-__device__ __forceinline__ void load_cells(const T* __restrict__ row, int x, int nx, bool vec,
-                                           T (&v)[V]) {
-  using VT = typename Vec16<T>::type;
-  if (vec) {
-    const VT q = __ldg(reinterpret_cast<const VT*>(row + x));
-    const T* pq = reinterpret_cast<const T*>(&q);
-#pragma unroll
-    for (int e = 0; e < V; ++e) v[e] = pq[e];
-  } else {
-#pragma unroll
-    for (int e = 0; e < V; ++e) v[e] = x + e < nx ? __ldg(row + x + e) : T(0);
-  }
-}
-
-template <typename T, int V>
-__device__ __forceinline__ void store_cells(T* row, int x, int nx, bool vec, const T (&v)[V]) {
-  using VT = typename Vec16<T>::type;
-  if (vec) {
-    VT q;
-    T* pq = reinterpret_cast<T*>(&q);
-#pragma unroll
-    for (int e = 0; e < V; ++e) pq[e] = v[e];
-    *reinterpret_cast<VT*>(row + x) = q;
-  } else {
-#pragma unroll
-    for (int e = 0; e < V; ++e)
-      if (x + e < nx) row[x + e] = v[e];
-  }
-}
 
 template <typename T, typename Op>
 __global__ void __launch_bounds__(kThreads)
@@ -270,7 +198,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int j = 0; j < RB + 2; ++j) {
     // rows past the ghost row feed outputs that are not stored
-    const int y = rows_in ? y0 - 1 + j : RowRule<T>(g, bc, min(y0 - 1 + j, ny)).src;
+    const int y = rows_in ? y0 - 1 + j : AxisRule<T>(g, bc, 0, min(y0 - 1 + j, ny)).src;
     const T* row = in + (int64_t)y * g.pitch;
     load_cells<T, V>(row, x, nx, vec, c[j]);
     if (j >= 1 && j <= RB) {
@@ -281,7 +209,7 @@ __global__ void __launch_bounds__(kThreads)
   if (!rows_in) {  // ghost rows above and below the grid (uniform across the warp)
 #pragma unroll
     for (int j = 0; j < RB + 2; ++j) {
-      const RowRule<T> r(g, bc, min(y0 - 1 + j, ny));
+      const AxisRule<T> r(g, bc, 0, min(y0 - 1 + j, ny));
       if (r.ghost) {
 #pragma unroll
         for (int e = 0; e < V; ++e) c[j][e] = r.fixed ? r.add : c[j][e] + r.add;
@@ -573,7 +501,7 @@ __global__ void __launch_bounds__(32 * NW, 2)
     float v[R][4];
     int src[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) src[r] = RowRule<float>(g, bc, yw + r).src;
+    for (int r = 0; r < R; ++r) src[r] = AxisRule<float>(g, bc, 0, yw + r).src;
     if (x >= 0 && x + 4 <= nx) {
 #pragma unroll
       for (int r = 0; r < R; ++r)

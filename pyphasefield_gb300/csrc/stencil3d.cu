@@ -1,7 +1,8 @@
 // 3-D explicit steps that march along z: Diffusion / Allen-Cahn (7-point)
 // and Cahn-Hilliard (radius 2 through an on-chip chemical-potential tile).
 //
-// A CTA owns a TY x TX column of the grid and a chunk of ZC planes. Its
+// Diffusion / Allen-Cahn by default: lean7_kernel, warps without a shared tile.
+// Otherwise a CTA owns a TY x TX column of the grid and a chunk of ZC planes. Its
 // z-planes (with an xy halo) are staged by TMA tensor loads into a ring of
 // shared-memory slots, several planes ahead of the plane being computed, so
 // HBM reads overlap the stencil; each plane is read once and written once
@@ -16,6 +17,8 @@
 #include <cmath>
 
 #include "ppf_common.cuh"
+#include "ppf_pack.cuh"
+#include "ppf_rows.cuh"
 #include "ppf_tma.cuh"
 
 namespace ppf {
@@ -28,8 +31,13 @@ template <typename T>
 struct Diffusion7 {
   T r;
   __device__ __forceinline__ T operator()(T c, T w, T e, T n, T s, T d, T u) const {
-    const T lap = (((w + e) + (n + s)) + (d + u)) - T(6) * c;
-    return c + r * lap;
+    const T lap = fma(T(-6), c, ((w + e) + (n + s)) + (d + u));
+    return fma(r, lap, c);
+  }
+  // two cells: the sums of the west / east, north / south and lower / upper
+  // pairs, rounded as above
+  __device__ __forceinline__ F2 pair(F2 c, F2 we, F2 ns, F2 du) const {
+    return fma2(sp(r), fma2(sp(-6.f), c, (we + ns) + du), c);
   }
 };
 
@@ -37,11 +45,36 @@ template <typename T>
 struct AllenCahn7 {
   T a, b;
   __device__ __forceinline__ T operator()(T c, T w, T e, T n, T s, T d, T u) const {
-    const T lap = (((w + e) + (n + s)) + (d + u)) - T(6) * c;
-    const T fp = c * (T(2) + c * (T(-6) + T(4) * c));
-    return c + (a * lap - b * fp);
+    const T lap = fma(T(-6), c, ((w + e) + (n + s)) + (d + u));
+    const T fp = c * fma(c, fma(T(4), c, T(-6)), T(2));
+    return c + fma(a, lap, -b * fp);
+  }
+  __device__ __forceinline__ F2 pair(F2 c, F2 we, F2 ns, F2 du) const {
+    const F2 lap = fma2(sp(-6.f), c, (we + ns) + du);
+    const F2 fp = c * fma2(c, fma2(sp(4.f), c, sp(-6.f)), sp(2.f));
+    return c + fma2(sp(a), lap, sp(-b) * fp);
   }
 };
+
+// One vector of cells from its neighbours: packed in float, cell by cell in double.
+template <typename Op>
+__device__ __forceinline__ void advance(const Op& op, const float (&c)[4], float w, float e,
+                                        const float (&n)[4], const float (&s)[4],
+                                        const float (&d)[4], const float (&u)[4], float (&o)[4]) {
+  const F2 a = op.pair(pk(c[0], c[1]), pk(w + c[1], c[0] + c[2]), pk(n[0], n[1]) + pk(s[0], s[1]),
+                       pk(d[0], d[1]) + pk(u[0], u[1]));
+  const F2 b = op.pair(pk(c[2], c[3]), pk(c[1] + c[3], c[2] + e), pk(n[2], n[3]) + pk(s[2], s[3]),
+                       pk(d[2], d[3]) + pk(u[2], u[3]));
+  o[0] = lo(a), o[1] = hi(a), o[2] = lo(b), o[3] = hi(b);
+}
+template <typename Op>
+__device__ __forceinline__ void advance(const Op& op, const double (&c)[2], double w, double e,
+                                        const double (&n)[2], const double (&s)[2],
+                                        const double (&d)[2], const double (&u)[2],
+                                        double (&o)[2]) {
+  o[0] = op(c[0], w, c[1], n[0], s[0], d[0], u[0]);
+  o[1] = op(c[1], c[0], e, n[1], s[1], d[1], u[1]);
+}
 
 // Shared-memory plane ring fed by TMA. Plane p (p >= pbase) lives in slot
 // (p - pbase) % NS; its k-th use of the slot completes mbarrier phase k.
@@ -319,140 +352,192 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Lean 7-point kernel (the default tile): 32 x 32 cells, 256 threads, each
-// thread owns the 4 xy-columns (ty + 8q, tx) and keeps c(z - 1), c(z) of
-// each in registers while marching along z, so a cell reads only its four
-// xy neighbours and the new plane's centre from shared memory; every shared
-// index is a compile-time offset from one per-thread base and there is one
-// block barrier per plane.
-constexpr int kLTX = 32;
-constexpr int kLTY = 32;
-constexpr int kLQ = kLTY / 8;
-constexpr int kLW = kLTX + 2 * kXOff;  // TMA box width
-constexpr int kNSL = 6;                // planes z, z+1 read; z+2 .. z+4 in flight
+// Lean 7-point kernel (the default): a warp owns 32 V columns (V cells of one
+// 16-byte vector per lane) and R rows and marches along z with planes z - 1, z
+// and z + 1 of its rows in registers; west / east cells come by shuffles. A
+// lane copies its own vectors of the band and of the two rows beside it, D - 1
+// planes ahead, into a ring in shared memory (cp.async) and is the only one to
+// read them back: no barrier, and a warp waits for its own copies alone. The
+// grid's edges take the same path: a ghost row or plane is copied from its
+// source and fixed after the read (AxisRule), a ghost column one of the strip's side
+// cells (ColumnRule), and of a vector that reaches past nx the cells below it.
+//
+// Bound: HBM beyond L2 (512^3: 6.3 TB/s), instruction latency below. us per step
+// against the 32 x 32 shared-memory tiles this replaced, whose edge tiles
+// rewrote their window every plane behind a barrier: Allen-Cahn 320 x 200 x 250
+// no-flux 86 -> 30, diffusion 64^3 22.9 -> 3.8, 256^3 38.2 -> 25.8, 384^3 104 ->
+// 79, 512^3 221 -> 170; float64 200^3 309 -> 260.
+constexpr int kLWarps = 4;
 
-template <typename T, typename Op, bool EDGE_COPY>
-__global__ void __launch_bounds__(kThreads)
-    march7_lean_kernel(const __grid_constant__ CUtensorMap map, Op op, Geo g, Bc<T> bc,
-                       const T* __restrict__ in, T* __restrict__ out, MarchGeom m,
-                       int slot_elems, int* status) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bars[kNSL];
-  __shared__ int abort_flag;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x0 = blockIdx.x * kLTX, y0 = blockIdx.y * kLTY, z0 = blockIdx.z * m.ZC;
+template <typename T, int R>
+struct Lean7Slot {
+  static constexpr int V = Vec16<T>::n;
+  static constexpr int side = (R + 2) * 32 * V;  // west cells, then east cells
+  static constexpr int elems = (side + 2 * R + V - 1) / V * V;
+};
+
+template <typename T, typename Op, int R, int D>
+__global__ void __launch_bounds__(32 * kLWarps)
+    lean7_kernel(Op op, const __grid_constant__ Geo g, const __grid_constant__ Bc<T> bc,
+                 const T* __restrict__ in, T* __restrict__ out, int zc) {
+  constexpr int V = Vec16<T>::n;
+  constexpr int WW = 32 * V;
+  using VT = typename Vec16<T>::type;
+  using Slot = Lean7Slot<T, R>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x;
+  T* ring = reinterpret_cast<T*>(smem_raw) + threadIdx.y * D * Slot::elems;
+  const int x0 = blockIdx.x * WW;
+  const int y0 = (blockIdx.y * kLWarps + threadIdx.y) * R;
+  const int z0 = blockIdx.z * zc;
   const int nz = g.n[0], ny = g.n[1], nx = g.n[2];
-  const int z1 = min(z0 + m.ZC, nz);
-  const bool xy_edge = x0 - kXOff < 0 || y0 - 1 < 0 || x0 + kLTX + kXOff > nx ||
-                       y0 + kLTY + 1 > ny;
-  PlaneRing<T, kNSL> ring{align128<T>(smem_raw), bars, slot_elems, z0 - 1};
-  const bool leader = tx == 0 && ty == 0;
-
-  if (leader) {
-    for (int i = 0; i < kNSL; ++i) mbar_init(&bars[i], 1);
-    mbar_init_fence();
-    abort_flag = 0;
-  }
-  __syncthreads();
   pdl_wait();
   pdl_launch_next();
-  const int last = z1;  // plane z1 is the upper neighbour of the last plane
-  if (leader)
-    for (int p = z0 - 1; p <= min(z0 + kNSL - 3, last); ++p)
-      issue_plane(ring, &map, g, bc, m, x0, y0, p);
-  for (int p = z0 - 1; p <= z0; ++p) {
-    if (!wait_all(ring.bar(p), ring.parity(p), &abort_flag)) {
-      report_timeout<T>(status);
-      drain(ring, p, min(z0 + kNSL - 3, last));
-      return;
-    }
-    fixup_plane(ring, in, g, bc, m, x0, y0, p, xy_edge);
-  }
-  __syncthreads();
-
-  const int ci = (ty + 1) * kLW + tx + kXOff;
-  T cm[kLQ], c0[kLQ];
-  {
-    const T* Pm = ring.plane(z0 - 1);
-    const T* P0 = ring.plane(z0);
+  if (y0 >= ny) return;  // whole warp; no block-wide barrier follows
+  const int z1 = min(z0 + zc, nz);
+  const int x = x0 + lane * V;
+  const bool vec = x + V <= nx;
+  const bool full_x = x0 + WW <= nx;
+  // bytes a lane copies of a row: the cells below nx, the rest of its vector
+  // reads zero
+  const uint32_t bytes = (uint32_t)max(0, min(V, nx - x)) * (uint32_t)sizeof(T);
+  const bool rows_in = y0 >= 1 && y0 + R + 1 <= ny;
+  const bool first = lane == 0;                             // uses the west neighbours
+  const bool last = x < nx && (lane == 31 || x + V >= nx);  // uses the east neighbours
+  const ColumnRule<T, 1, 2> wr(g, bc, x0 - 1), er(g, bc, min(x0 + WW, nx));
+  const bool x_ghost = wr.ghost || er.ghost;  // uniform across the warp
+  const bool full_y = y0 + R <= ny;
+  const int64_t out_off = (int64_t)y0 * g.pitch;
+  // this lane's element of each row of a plane (planes below 2^31 elements)
+  const uint32_t xs = x < nx ? x : 0;
+  uint32_t off[R + 2];
 #pragma unroll
-    for (int q = 0; q < kLQ; ++q) {
-      cm[q] = Pm[ci + q * 8 * kLW];
-      c0[q] = P0[ci + q * 8 * kLW];
-    }
-  }
-  T* optr = out + (int64_t)z0 * g.plane + (int64_t)(y0 + ty) * g.pitch + x0 + tx;
-  const int64_t qstride = (int64_t)8 * g.pitch;
-  const bool xin = x0 + tx < nx;
-  int nq = 0;
+  for (int j = 0; j < R + 2; ++j)
+    // rows past the ghost row feed outputs that are not stored
+    off[j] = (uint32_t)(rows_in ? y0 - 1 + j : AxisRule<T>(g, bc, 1, min(y0 - 1 + j, ny)).src) *
+                 (uint32_t)g.pitch +
+             xs;
+  // lane j < 2 R copies one side cell: west of row j, east of row j - R
+  uint32_t side_off = 0;
 #pragma unroll
-  for (int q = 0; q < kLQ; ++q) nq += (xin && y0 + ty + 8 * q < ny) ? 1 : 0;
-  const bool full = x0 + kLTX <= nx && y0 + kLTY <= ny;
-
-  // Edge tiles of a grid periodic along y and x (window cells outside the
-  // grid are plain copies of cells on the far side, at most one per thread,
-  // plane offsets below 2^31): thread tid copies window cell tid's source,
-  // found once here, into each plane's slot.
-  // EDGE_COPY: the instantiation for grids with many edge tiles (the copy
-  // costs eight registers a thread, one CTA per SM less).
-  int e_dst = -1, e_src = 0;
-  bool async_tile = false;
-  if (EDGE_COPY && xy_edge && bc.type[1] == PPF_BC_PERIODIC && bc.type[2] == PPF_BC_PERIODIC &&
-      (int64_t)ny * g.pitch < (1LL << 31)) {
-    const EdgeSet E = edge_set(m, g, x0, y0);
-    async_tile = E.count <= kThreads;
-    const int tid = tx + 32 * ty;
-    if (async_tile && tid < E.count) {
-      int ly, lx;
-      edge_cell(E, tid, ly, lx);
-      e_dst = ly * m.BX + lx + (kXOff - m.H);
-      e_src = wrap_index(y0 - m.H + ly, ny) * (int)g.pitch + wrap_index(x0 - m.H + lx, nx);
-    }
+  for (int j = 0; j < R; ++j) {
+    if (lane == j) side_off = off[j + 1] - xs + (uint32_t)wr.xi;
+    if (lane == R + j) side_off = off[j + 1] - xs + (uint32_t)er.xi;
   }
 
+  // plane p: the band's own rows, and for a plane that is advanced the rows
+  // and columns beside them
+  auto issue = [&](int p, int slot) {
+    T* s = ring + slot * Slot::elems;
+    const int zs = (unsigned)p < (unsigned)nz ? p : AxisRule<T>(g, bc, 0, p).src;
+    const T* src = in + (int64_t)zs * g.plane;
+    const bool beside = p >= z0 && p < z1;
+    const uint32_t d = smem_addr(s + lane * V);
+#pragma unroll
+    for (int j = 0; j < R + 2; ++j)
+      if ((j >= 1 && j <= R) || beside)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         d + (uint32_t)(j * WW * sizeof(T))),
+                     "l"(src + off[j]), "r"(bytes)
+                     : "memory");
+    if (beside && lane < 2 * R) cp_async_elem(s + Slot::side + lane, src + side_off);
+  };
+  auto read_row = [&](const T* s, int j, T (&v)[V]) {
+    const VT q = *reinterpret_cast<const VT*>(s + j * WW + lane * V);
+    const T* pq = reinterpret_cast<const T*>(&q);
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = pq[e];
+  };
+  auto read_own = [&](int z, const T* s, T (&v)[R][V]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) read_row(s, j + 1, v[j]);
+    if ((unsigned)z >= (unsigned)nz) {
+      const AxisRule<T> zr(g, bc, 0, z);
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[j][e] = zr.value(v[j][e]);
+    }
+  };
+
+  // one group per plane, empty ones past the end, so that the count of groups
+  // in flight is the same in every iteration
+#pragma unroll
+  for (int q = 0; q < D; ++q) {
+    if (z0 - 1 + q <= z1) issue(z0 - 1 + q, q);
+    cp_async_commit();
+  }
+  T cm[R][V], c0[R][V];
+  asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");
+  read_own(z0 - 1, ring, cm);
+  read_own(z0, ring + Slot::elems, c0);
+  int sm = 0;  // slot of plane z - 1
   for (int z = z0; z < z1; ++z) {
-    // plane z + kNSL - 2 takes the slot of plane z - 2, last read in
-    // iteration z - 2 (plane p is read in iterations p - 1 and p), which
-    // every thread finished before the barrier of iteration z - 1
-    if (leader && z + kNSL - 2 <= last) issue_plane(ring, &map, g, bc, m, x0, y0, z + kNSL - 2);
-    if (!wait_all(ring.bar(z + 1), ring.parity(z + 1), &abort_flag)) {
-      report_timeout<T>(status);
-      drain(ring, z + 1, min(z + kNSL - 2, last));
-      return;
-    }
-    // (no register prefetch of the edge values here: its registers cost
-    // this kernel more occupancy than the hidden loads gain)
-    const bool zghost = ghost_plane(g, bc, z + 1);
-    const bool async_edge = async_tile && !zghost;
-    if (zghost || (xy_edge && !async_edge)) {
-      fixup_plane(ring, in, g, bc, m, x0, y0, z + 1, xy_edge);
-      __syncthreads();
-    }
-    if (async_edge) {
-      // Iteration z reads only the own (inside) cells of plane z + 1, its
-      // cells outside the grid from iteration z + 1 on, after that
-      // iteration's barrier: they are copied into the slot (which its TMA
-      // load has filled) asynchronously during this plane's stencil, each
-      // thread waiting for its copy at the end of the iteration.
-      if (e_dst >= 0)
-        cp_async_elem(ring.plane(z + 1) + e_dst,
-                      in + (int64_t)wrap_index(z + 1, nz) * g.plane + e_src);
-      cp_async_commit();
-    }
-    const T* P0 = ring.plane(z);
-    const T* P1 = ring.plane(z + 1);
+    // planes up to z + D - 2 are issued: z + 1 has landed when D - 3 are pending
+    // (the side cells are other lanes' copies)
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 3) : "memory");
+    __syncwarp();
+    if (z + D - 1 <= z1) issue(z + D - 1, sm);
+    cp_async_commit();
+    const int s0 = sm + 1 == D ? 0 : sm + 1, sp = s0 + 1 == D ? 0 : s0 + 1;
+    const T* S0 = ring + s0 * Slot::elems;
+    T cp[R][V], c[R + 2][V], side[2 * R];
+    read_own(z + 1, ring + sp * Slot::elems, cp);
+    read_row(S0, 0, c[0]);
+    read_row(S0, R + 1, c[R + 1]);
 #pragma unroll
-    for (int q = 0; q < kLQ; ++q) {
-      const int i = ci + q * 8 * kLW;
-      const T cp = P1[i];
-      const T v = op(c0[q], P0[i - 1], P0[i + 1], P0[i - kLW], P0[i + kLW], cm[q], cp);
-      if (full || q < nq) optr[q * qstride] = v;
-      cm[q] = c0[q];
-      c0[q] = cp;
+    for (int j = 0; j < R; ++j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) c[j + 1][e] = c0[j][e];
+#pragma unroll
+    for (int q = 0; q < 2 * R / V; ++q) {
+      const VT v = *reinterpret_cast<const VT*>(S0 + Slot::side + q * V);
+      const T* pv = reinterpret_cast<const T*>(&v);
+#pragma unroll
+      for (int e = 0; e < V; ++e) side[q * V + e] = pv[e];
     }
-    optr += g.plane;
-    if (async_edge) cp_async_wait_all();
+    if (!rows_in) {  // ghost rows (uniform across the warp)
+#pragma unroll
+      for (int j = 0; j < R + 2; ++j) {
+        const AxisRule<T> r(g, bc, 1, min(y0 - 1 + j, ny));
+        if (r.ghost) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) c[j][e] = r.value(c[j][e]);
+        }
+      }
+    }
+    if (x_ghost) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        side[j] = wr.value(0, side[j]);
+        side[R + j] = er.value(0, side[R + j]);
+      }
+    }
+    T* orow = out + (int64_t)z * g.plane + out_off;
+#pragma unroll
+    for (int j = 1; j <= R; ++j) {
+      const T wv = side[j - 1], ev = side[R + j - 1];
+      if (!full_x) {  // the ghost column inside the last lane's vector
+#pragma unroll
+        for (int e = 1; e < V; ++e)
+          if (x + e == nx) c[j][e] = ev;
+      }
+      T wl = __shfl_up_sync(0xffffffffu, c[j][V - 1], 1);
+      T ee = __shfl_down_sync(0xffffffffu, c[j][0], 1);
+      if (first) wl = wv;
+      if (last) ee = ev;
+      T o[V];
+      advance(op, c[j], wl, ee, c[j - 1], c[j + 1], cm[j - 1], cp[j - 1], o);
+      if (full_y || y0 + j - 1 < ny) store_cells<T, V>(orow, x, nx, vec, o);
+      orow += g.pitch;
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) cm[j][e] = c0[j][e], c0[j][e] = cp[j][e];
+    sm = s0;
   }
+  cp_async_wait_all();
 }
 
 // ------------------------------------------------------------- Cahn-Hilliard
@@ -756,6 +841,17 @@ int zchunk_of(const PpfTiling* t, const Geo& g) {
   return zc < g.n[0] ? zc : g.n[0];
 }
 
+// The same for the lean 7-point kernel: a chunk of zc planes copies zc + 2, and a
+// warp advances one plane after the other, so chunks are as short as it takes to
+// have a dozen warps per SM (float, us per step with 2 / 4 / 8 planes: 64^3 3.8 /
+// 5.7 / 9.4, 128^3 5.2 / 5.7 / 7.9, 256^3 30 / 29 / 26, 512^3 196 / 178 / 170,
+// 16 planes 176).
+int lean_zchunk(long warps, int nz) {
+  int zc = 8;
+  while (zc > 2 && warps * ((nz + zc - 1) / zc) < 2048) zc /= 2;
+  return zc < nz ? zc : nz;
+}
+
 template <typename T>
 int32_t plane_map(CUtensorMap* map, const T* base, const Geo& g, const MarchGeom& m) {
   const uint64_t dims[3] = {(uint64_t)g.n[2], (uint64_t)g.n[1], (uint64_t)g.n[0]};
@@ -804,30 +900,29 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
   size_t smem;
   int* st = status_ptr();
   if (!st) return fail(PPF_ERR_CUDA, "status word unavailable");
-  const bool lean = !tiling || ((tiling->tile_x == 0 || tiling->tile_x == kLTX) &&
-                                (tiling->tile_y == 0 || tiling->tile_y == kLTY));
+  const bool lean = (!tiling || ((tiling->tile_x == 0 || tiling->tile_x == 32) &&
+                                 (tiling->tile_y == 0 || tiling->tile_y == 32))) &&
+                    g.plane < (1LL << 31);
   if (lean) {
     PpfTiling lt{};
     lt.depth = tiling ? tiling->depth : 0;
-    lt.tile_x = kLTX;
-    lt.tile_y = kLTY;
-    if ((rc = plan3d<T>(&lt, g, 1, kNSL, 0, &m, &slot_elems, &smem))) return rc;
-    CUtensorMap map;
-    if ((rc = plane_map<T>(&map, in, g, m))) return rc;
-    // periodic in y and x with a quarter or more of the tiles on an edge
-    // (384^3 and below): the kernel that copies the edge cells
-    // asynchronously (256^3 43.8 -> 39.5 us per step, 384^3 108.9 -> 104.8;
-    // 512^3 222.0 against 224.4 with it)
-    const long long tx_n = (g.n[2] + kLTX - 1) / kLTX, ty_n = (g.n[1] + kLTY - 1) / kLTY;
-    const long long inner = (tx_n > 2 ? tx_n - 2 : 0) * (ty_n > 2 ? ty_n - 2 : 0);
-    const bool edge_copy = bc.type[1] == PPF_BC_PERIODIC && bc.type[2] == PPF_BC_PERIODIC &&
-                           4 * (tx_n * ty_n - inner) >= tx_n * ty_n;
-    auto kern = edge_copy ? march7_lean_kernel<T, Op, true> : march7_lean_kernel<T, Op, false>;
+    lt.zchunk = tiling ? tiling->zchunk : 0;
+    if ((rc = plan3d<T>(&lt, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
+    if (((uintptr_t)in) % 16 || ((uintptr_t)out) % 16)
+      return fail(PPF_ERR_INVALID, "3-D steps need 16-byte aligned rows");
+    constexpr int WW = 32 * Vec16<T>::n;
+    // four rows per warp re-read half a row per row, two a whole one; in double,
+    // where the FP64 units bind, fewer registers win (200^3: 4 %)
+    constexpr int R = sizeof(T) == 4 ? 4 : 2, D = 4;
+    const int strips = (g.n[2] + WW - 1) / WW, bands = (g.n[1] + R * kLWarps - 1) / (R * kLWarps);
+    m.ZC = tiling && tiling->zchunk > 0 ? zchunk_of(tiling, g)
+                                        : lean_zchunk((long)strips * bands * kLWarps, g.n[0]);
+    const dim3 gd(strips, bands, (g.n[0] + m.ZC - 1) / m.ZC);
+    auto kern = lean7_kernel<T, Op, R, D>;
+    smem = (size_t)kLWarps * D * Lean7Slot<T, R>::elems * sizeof(T);
     PPF_TRY_CUDA(allow_smem(kern, smem));
-    m.ZC = zchunk_of(tiling, g);
-    dim3 gd((g.n[2] + kLTX - 1) / kLTX, (g.n[1] + kLTY - 1) / kLTY, (g.n[0] + m.ZC - 1) / m.ZC);
-    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kThreads / 32), smem, (cudaStream_t)stream,
-                        tiling && tiling->pdl, map, op, g, bc, in, out, m, slot_elems, st));
+    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kLWarps), smem, (cudaStream_t)stream,
+                        tiling && tiling->pdl, op, g, bc, in, out, m.ZC));
     return PPF_OK;
   }
   if ((rc = plan3d<T>(tiling, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
