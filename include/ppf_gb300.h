@@ -415,6 +415,61 @@ int32_t ppf_ncgpu_temperature_advance_f32(const PpfGrid* g, float* temperature, 
 int32_t ppf_ncgpu_temperature_advance_f64(const PpfGrid* g, double* temperature, double dT,
                                           void* stream);
 
+/* ---- runs of steps ------------------------------------------------------ */
+
+/* npasses passes of one model, from the field buffers a into b, back into a and
+ * so on: pass i advances depths[i] steps (1 for every model but the 2-D explicit
+ * Diffusion and Allen-Cahn steps) through the model's step entry point, with
+ * its argument checks; the first error ends the run. The result is in a when
+ * npasses is even, else in b.
+ *   PPF_RUN_CAHN_HILLIARD   step k adds its mass to mass[k] (mass may be NULL)
+ *   PPF_RUN_WARREN1995, PPF_RUN_NCGPU   step k draws the noise of step + k
+ *     (+ *step_base)
+ *   PPF_RUN_*_IMPLICIT      tmp, scratch as in the step; iterations (may be NULL)
+ *     receives the last step's count
+ *   PPF_RUN_NCGPU           tmp is the step's transfer buffer; dT != 0 raises the
+ *     temperature after every step */
+#define PPF_RUN_DIFFUSION 0
+#define PPF_RUN_ALLEN_CAHN 1
+#define PPF_RUN_CAHN_HILLIARD 2
+#define PPF_RUN_WARREN1995 3
+#define PPF_RUN_DIFFUSION_IMPLICIT 4
+#define PPF_RUN_PHASE_IMPLICIT 5
+#define PPF_RUN_NCGPU 6
+#define PPF_RUN_MAX_FIELDS 8
+typedef struct PpfRun {
+  int32_t model;      /* PPF_RUN_* */
+  int32_t elem_bytes; /* 4 or 8 */
+  const void* params; /* the model's parameter struct */
+  const PpfGrid* grid;
+  const PpfBoundary* boundary;
+  const PpfTiling* tiling; /* depth is taken from depths; may be NULL */
+  void* a[PPF_RUN_MAX_FIELDS];
+  void* b[PPF_RUN_MAX_FIELDS];
+  uint64_t seed, step;
+  const uint64_t* step_base;
+  double* mass;
+  int32_t* status;
+  void* tmp;
+  void* scratch;
+  size_t scratch_bytes;
+  void* temperature;
+  const double* tables;
+  double dT;
+} PpfRun;
+int32_t ppf_run(const PpfRun* run, const int32_t* depths, int32_t npasses, int32_t* iterations,
+                void* stream);
+
+/* One launch that ORs PPF_STATUS_NONFINITE into *status if any of the nfields
+ * fields holds NaN or Inf, moves the library's status bits into *status as
+ * ppf_status_collect does, and writes the word to *host (pinned host memory or
+ * any address the device can write). counter: a device word, zeroed once, for
+ * one call at a time. */
+int32_t ppf_watch_f32(const float* const* fields, int32_t nfields, const PpfGrid* g,
+                      int32_t* status, int32_t* counter, int32_t* host, void* stream);
+int32_t ppf_watch_f64(const double* const* fields, int32_t nfields, const PpfGrid* g,
+                      int32_t* status, int32_t* counter, int32_t* host, void* stream);
+
 /* ---- batched ensemble ------------------------------------------------- */
 
 #define PPF_MODEL_WARREN1995 1
@@ -607,6 +662,8 @@ int32_t ppf_selftest_wait_timeout(int32_t poll_limit, void* stream);
 
 /* *counter += inc on the device (stream-ordered; one thread). */
 int32_t ppf_counter_add_u64(uint64_t* counter, uint64_t inc, void* stream);
+/* *counter = value in stream order. */
+int32_t ppf_counter_set_u64(uint64_t* counter, uint64_t value, void* stream);
 
 /* ---- CUDA graphs ------------------------------------------------------ */
 

@@ -127,6 +127,27 @@ class PpfMember(C.Structure):
                 ("w95", PpfWarren1995Params), ("ac", PpfAllenCahnParams)]
 
 
+PPF_RUN_DIFFUSION = 0
+PPF_RUN_ALLEN_CAHN = 1
+PPF_RUN_CAHN_HILLIARD = 2
+PPF_RUN_WARREN1995 = 3
+PPF_RUN_DIFFUSION_IMPLICIT = 4
+PPF_RUN_PHASE_IMPLICIT = 5
+PPF_RUN_NCGPU = 6
+PPF_RUN_MAX_FIELDS = 8
+
+
+class PpfRun(C.Structure):
+    _fields_ = [("model", C.c_int32), ("elem_bytes", C.c_int32), ("params", C.c_void_p),
+                ("grid", C.POINTER(PpfGrid)), ("boundary", C.POINTER(PpfBoundary)),
+                ("tiling", C.POINTER(PpfTiling)), ("a", C.c_void_p * PPF_RUN_MAX_FIELDS),
+                ("b", C.c_void_p * PPF_RUN_MAX_FIELDS), ("seed", C.c_uint64),
+                ("step", C.c_uint64), ("step_base", C.c_void_p), ("mass", C.c_void_p),
+                ("status", C.c_void_p), ("tmp", C.c_void_p), ("scratch", C.c_void_p),
+                ("scratch_bytes", C.c_size_t), ("temperature", C.c_void_p),
+                ("tables", C.c_void_p), ("dT", C.c_double)]
+
+
 class PpfEnsemblePlan(C.Structure):
     _fields_ = [("device_table", C.c_void_p), ("n_items", C.c_int64),
                 ("n_members", C.c_int32), ("rows", C.c_int32), ("n_units", C.c_int64),
@@ -184,6 +205,10 @@ SIGNATURES: dict[str, list] = {
                                C.POINTER(I32), P],
     "ppf_periodic_solve_f64": [PG, C.c_double, C.c_double, C.c_double, P, P, P,
                                C.POINTER(I32), P],
+    "ppf_run": [C.POINTER(PpfRun), C.POINTER(I32), I32, C.POINTER(I32), P],
+    "ppf_watch_f32": [P, I32, PG, P, P, P, P],
+    "ppf_watch_f64": [P, I32, PG, P, P, P, P],
+    "ppf_counter_set_u64": [P, U64, P],
     "ppf_ensemble_plan_bytes": [C.POINTER(PpfMember), I32, PT, C.POINTER(SZ)],
     "ppf_ensemble_build": [C.POINTER(PpfMember), I32, PT, P, SZ, C.POINTER(PpfEnsemblePlan), P],
     "ppf_ensemble_step_f32": [C.POINTER(PpfEnsemblePlan), I32, U64, P, PT, P],

@@ -101,6 +101,11 @@ __global__ void counter_add_kernel(uint64_t* c, uint64_t inc) {
   *c += inc;
 }
 
+__global__ void counter_set_kernel(uint64_t* c, uint64_t value) {
+  pdl_wait();
+  *c = value;
+}
+
 // ------------------------------------------------------------ status word
 __device__ int g_status;
 
@@ -301,6 +306,14 @@ int32_t ppf_counter_add_u64(uint64_t* counter, uint64_t inc, void* stream) {
   clear_error();
   if (!counter) return fail(PPF_ERR_INVALID, "counter is NULL");
   counter_add_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(counter, inc);
+  PPF_TRY_CUDA(cudaGetLastError());
+  return PPF_OK;
+}
+
+int32_t ppf_counter_set_u64(uint64_t* counter, uint64_t value, void* stream) {
+  clear_error();
+  if (!counter) return fail(PPF_ERR_INVALID, "counter is NULL");
+  counter_set_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(counter, value);
   PPF_TRY_CUDA(cudaGetLastError());
   return PPF_OK;
 }

@@ -158,6 +158,50 @@ __global__ void __launch_bounds__(kRedThreads)
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status, PPF_STATUS_NONFINITE);
 }
 
+// The engines' watch after a chunk of steps: finite_kernel's test over every
+// field, then (the last CTA to finish) the library's status bits moved into the
+// word and the word written to the host. One launch where the sentinel per
+// field, the collecting launch and the copy were three or more, which a small
+// grid's chunk waited for one after the other.
+struct WatchFields {
+  const void* f[PPF_RUN_MAX_FIELDS];
+  int n;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads)
+    watch_kernel(WatchFields w, Geo g, int* __restrict__ status, int* __restrict__ lib,
+                 unsigned* __restrict__ counter, volatile int* host) {
+  pdl_wait();
+  const int nx = g.n[g.ndim - 1];
+  const int64_t rows = g.ndim == 2 ? (int64_t)g.n[0] : (int64_t)g.n[0] * g.n[1];
+  int bad = 0;
+  for (int k = 0; k < w.n; ++k) {
+    const T* x = (const T*)w.f[k];
+    for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+      int64_t off;
+      if (g.ndim == 2) {
+        off = r * g.pitch;
+      } else {
+        const int64_t i0 = r / g.n[1];
+        off = i0 * g.plane + (r - i0 * g.n[1]) * g.pitch;
+      }
+#pragma unroll 4
+      for (int c = threadIdx.x; c < nx; c += kRedThreads) bad |= !isfinite(x[off + c]);
+    }
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status, PPF_STATUS_NONFINITE);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(counter, 1u) == gridDim.x - 1) {
+      *counter = 0;
+      __threadfence();
+      const int v = atomicExch(lib, 0);
+      *host = atomicOr(status, v) | v;
+    }
+  }
+}
+
 template <typename T, typename Op>
 int32_t reduce_impl(Op op, const T* x, const PpfGrid* grid, const PpfBoundary* b,
                     double dx, double w, double kappa, double scale_pow_dx,
@@ -219,6 +263,32 @@ int32_t check_finite(const T* x, const PpfGrid* grid, int32_t* status, void* str
   if (rc) return rc;
   if (!x || !status) return fail(PPF_ERR_INVALID, "NULL pointer");
   finite_kernel<T><<<152 * 4, kRedThreads, 0, (cudaStream_t)stream>>>(x, g, (int*)status);
+  PPF_TRY_CUDA(cudaGetLastError());
+  return PPF_OK;
+}
+
+template <typename T>
+int32_t watch(const T* const* fields, int32_t nfields, const PpfGrid* grid, int32_t* status,
+              int32_t* counter, int32_t* host, void* stream) {
+  clear_error();
+  Geo g;
+  int32_t rc = make_geo(grid, 2, 3, &g);
+  if (rc) return rc;
+  if (!fields || !status || !counter || !host) return fail(PPF_ERR_INVALID, "NULL pointer");
+  if (nfields < 1 || nfields > PPF_RUN_MAX_FIELDS)
+    return fail(PPF_ERR_INVALID, "nfields=%d not in [1, %d]", nfields, PPF_RUN_MAX_FIELDS);
+  WatchFields w{};
+  w.n = nfields;
+  for (int32_t k = 0; k < nfields; ++k) {
+    if (!fields[k]) return fail(PPF_ERR_INVALID, "NULL field pointer");
+    w.f[k] = fields[k];
+  }
+  int* lib = status_ptr();
+  if (!lib) return fail(PPF_ERR_CUDA, "status word unavailable");
+  const int64_t rows = g.ndim == 2 ? (int64_t)g.n[0] : (int64_t)g.n[0] * g.n[1];
+  const unsigned blocks = (unsigned)(rows < 152 * 4 ? rows : 152 * 4);
+  watch_kernel<T><<<blocks, kRedThreads, 0, (cudaStream_t)stream>>>(
+      w, g, (int*)status, lib, (unsigned*)counter, (volatile int*)host);
   PPF_TRY_CUDA(cudaGetLastError());
   return PPF_OK;
 }
@@ -306,6 +376,15 @@ int32_t ppf_check_finite_f32(const float* x, const PpfGrid* grid, int32_t* statu
 int32_t ppf_check_finite_f64(const double* x, const PpfGrid* grid, int32_t* status,
                              void* stream) {
   return check_finite<double>(x, grid, status, stream);
+}
+
+int32_t ppf_watch_f32(const float* const* fields, int32_t nfields, const PpfGrid* g,
+                      int32_t* status, int32_t* counter, int32_t* host, void* stream) {
+  return watch<float>(fields, nfields, g, status, counter, host, stream);
+}
+int32_t ppf_watch_f64(const double* const* fields, int32_t nfields, const PpfGrid* g,
+                      int32_t* status, int32_t* counter, int32_t* host, void* stream) {
+  return watch<double>(fields, nfields, g, status, counter, host, stream);
 }
 
 }  // extern "C"

@@ -27,10 +27,10 @@ launch shapes on scratch copies and cache the fastest), bulk_shortcut
 check_status (bool, default True).
 
 Failure detection: after every chunk of steps (inside the captured graph)
-the engine runs the NaN/Inf sentinel over its fields (ppf_check_finite_*),
+the engine runs the NaN/Inf sentinel over its fields,
 moves the library's status bits (a bounded barrier wait that gave up, a
-Cahn-Hilliard range overflow) into its own sticky status word
-(ppf_status_collect) and copies that word to pinned host memory. The host
+Cahn-Hilliard range overflow) into its own sticky status word and writes
+that word to pinned host memory, in one launch (ppf_watch_*). The host
 reads the copy at the next chunk boundary (waiting for the chunk before the
 last, so the device stays a chunk ahead), at every autosave and in
 retrieve_fields_from_GPU, and raises EngineFault on any set bit: a run never
@@ -60,6 +60,9 @@ COMMON_DEFAULTS = dict(precision="fp32", temporal_depth=1, tile=None, pdl=True,
 
 #: captured graphs kept per engine (one per distinct parameter set)
 MAX_GRAPHS = 8
+
+#: user_data values that stand for themselves in a graph's key
+_PLAIN = frozenset((bool, int, float, str, type(None)))
 
 _STATUS_NAMES = ((L.PPF_STATUS_TIMEOUT, "a bounded barrier wait timed out (tile not written)"),
                  (L.PPF_STATUS_NONFINITE, "a field holds NaN or Inf"),
@@ -120,6 +123,15 @@ class GB300Engine:
         """Launch one pass advancing `depth` steps from buffers src to dst."""
         raise NotImplementedError
 
+    #: whether a step reads the step counter (noise drawn per step)
+    USES_STEP = False
+
+    def _ppf_run(self):
+        """PpfRun of the engine's steps (model, params, tiling and the model's
+        own buffers; the fields and the step are filled in), or None for an
+        engine whose steps are launched one by one."""
+        return None
+
     def _ppf_max_depth(self) -> int:
         return 1
 
@@ -179,7 +191,9 @@ class GB300Engine:
         self._ppf_staging = []
         self._ppf_status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._ppf_status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        self._ppf_watch_counter = torch.zeros(1, dtype=torch.int32, device=dev)
         self._ppf_status_events = collections.deque()
+        self._ppf_event_pool = []
         self._uses_gpu = True
 
     def _ppf_release_graphs(self):
@@ -189,29 +203,27 @@ class GB300Engine:
 
     # ------------------------------------------------------------ status
     def _ppf_watch(self, stream):
-        """Launches issued after a chunk of steps (captured with it): the
+        """The launch issued after a chunk of steps (captured with it): the
         NaN/Inf sentinel on the current fields, the library status bits
-        moved into the engine's word, and the word copied to pinned host
+        moved into the engine's word, and the word written to pinned host
         memory."""
         if not self.user_data.get("check_status", True):
             return
-        sp = C.c_void_p(stream.cuda_stream)
-        f = "f32" if self._ppf_dtype == torch.float32 else "f64"
-        st = ptr(self._ppf_status)
-        for t in self._ppf_bufs[self._ppf_cur]:
-            L.call(f"ppf_check_finite_{f}", ptr(t), C.byref(self._ppf_grid.grid), st, sp)
-        L.call("ppf_status_collect", st, sp)
-        with torch.cuda.stream(stream):
-            self._ppf_status_host.copy_(self._ppf_status, non_blocking=True)
+        bufs = self._ppf_bufs[self._ppf_cur]
+        L.call("ppf_watch_f32" if self._ppf_dtype == torch.float32 else "ppf_watch_f64",
+               (C.c_void_p * len(bufs))(*[t.data_ptr() for t in bufs]), len(bufs),
+               C.byref(self._ppf_grid.grid), self._ppf_status.data_ptr(),
+               self._ppf_watch_counter.data_ptr(), self._ppf_status_host.data_ptr(),
+               stream.cuda_stream)
 
     def _ppf_watch_launches(self) -> int:
-        """Kernels _ppf_watch launches (the copy is not a kernel)."""
-        return self.NFIELDS + 1 if self.user_data.get("check_status", True) else 0
+        """Kernels _ppf_watch launches."""
+        return 1 if self.user_data.get("check_status", True) else 0
 
     def _ppf_mark(self):
-        """Records the point after a chunk's status copy (host side)."""
+        """Records the point after a chunk's status word (host side)."""
         if self.user_data.get("check_status", True):
-            ev = torch.cuda.Event()
+            ev = self._ppf_event_pool.pop() if self._ppf_event_pool else torch.cuda.Event()
             ev.record(self._ppf_stream)
             self._ppf_status_events.append(ev)
 
@@ -225,10 +237,13 @@ class GB300Engine:
         if block:
             if evs:
                 evs[-1].synchronize()
+                self._ppf_event_pool.extend(evs)
                 evs.clear()
         else:
             while len(evs) > 1:
-                evs.popleft().synchronize()
+                ev = evs.popleft()
+                ev.synchronize()
+                self._ppf_event_pool.append(ev)
         bits = int(self._ppf_status_host.item())
         if bits:
             self.synchronize()
@@ -476,11 +491,31 @@ class GB300Engine:
             passes.append(nsteps % k)
         return passes
 
-    def _ppf_launch_pass(self, depth, step, step_base):
-        src = self._ppf_bufs[self._ppf_cur]
-        dst = self._ppf_bufs[1 - self._ppf_cur]
-        self._ppf_step(src, dst, depth, step, step_base, C.c_void_p(self._ppf_stream.cuda_stream))
-        self._ppf_cur ^= 1
+    def _ppf_launch_passes(self, depths, step, step_base):
+        """Launch the passes of a run of steps from absolute step `step` (plus
+        *step_base on the device): one native call, or one call per pass."""
+        cur = self._ppf_cur
+        sp = self._ppf_stream.cuda_stream
+        run = self._ppf_run()
+        if run is None:
+            for d in depths:
+                self._ppf_step(self._ppf_bufs[self._ppf_cur], self._ppf_bufs[1 - self._ppf_cur], d,
+                               step, step_base, C.c_void_p(sp))
+                self._ppf_cur ^= 1
+                step += d
+            return
+        run.elem_bytes = 4 if self._ppf_dtype == torch.float32 else 8
+        run.grid = C.pointer(self._ppf_grid.grid)
+        run.boundary = C.pointer(self._ppf_bc)
+        for j, (t, u) in enumerate(zip(self._ppf_bufs[cur], self._ppf_bufs[1 - cur])):
+            run.a[j], run.b[j] = t.data_ptr(), u.data_ptr()
+        run.step = step
+        run.step_base = step_base.data_ptr() if step_base is not None else None
+        it = C.c_int32()
+        n = len(depths)
+        L.call("ppf_run", C.byref(run), (C.c_int32 * n)(*depths), n, C.byref(it), sp)
+        self._ppf_iterations = it.value
+        self._ppf_cur ^= n & 1
 
     def _ppf_state_key(self):
         """What a captured graph bakes in besides the buffers: every
@@ -489,8 +524,11 @@ class GB300Engine:
         so editing user_data between simulate() calls never replays stale
         constants."""
         items = []
-        for k, v in sorted(self.user_data.items(), key=lambda kv: str(kv[0])):
-            if isinstance(v, np.ndarray):
+        for k, v in self.user_data.items():
+            t = type(v)
+            if t in _PLAIN:
+                v = (t, v)
+            elif isinstance(v, np.ndarray):
                 v = (v.shape, v.dtype.str,
                      hashlib.sha1(np.ascontiguousarray(v).tobytes()).hexdigest())
             elif isinstance(v, torch.Tensor):
@@ -522,11 +560,9 @@ class GB300Engine:
         try:
             with torch.cuda.stream(s):
                 self._ppf_segment_begin(total, s)
-                off = 0
-                for d in depths:
-                    self._ppf_launch_pass(d, off, self._ppf_stepctr)
-                    off += d
-                L.call("ppf_counter_add_u64", ptr(self._ppf_stepctr), C.c_uint64(total), sp)
+                self._ppf_launch_passes(depths, 0, self._ppf_stepctr if self.USES_STEP else None)
+                if self.USES_STEP:
+                    L.call("ppf_counter_add_u64", ptr(self._ppf_stepctr), C.c_uint64(total), sp)
                 self._ppf_watch(s)
         finally:
             try:
@@ -554,8 +590,8 @@ class GB300Engine:
         span = chunk * k
         if ud.get("use_graph", True) and nsteps >= span:
             g = self._ppf_graph(tuple(self._ppf_passes(span, even=True)))
-            with torch.cuda.stream(s):
-                self._ppf_stepctr.fill_(step)
+            if self.USES_STEP:
+                L.call("ppf_counter_set_u64", ptr(self._ppf_stepctr), C.c_uint64(step), sp)
             while nsteps >= span:
                 self._ppf_check_status(False)
                 with nvtx_range(f"ppf.graph {span} steps from {step}"):
@@ -569,9 +605,7 @@ class GB300Engine:
             self._ppf_check_status(False)
             with torch.cuda.stream(s), nvtx_range(f"ppf.eager {nsteps} steps from {step}"):
                 self._ppf_segment_begin(nsteps, s)
-                for d in self._ppf_passes(nsteps):
-                    self._ppf_launch_pass(d, step, None)
-                    step += d
+                self._ppf_launch_passes(self._ppf_passes(nsteps), step, None)
                 self._ppf_watch(s)
             self._ppf_mark()
             self._ppf_segment_end(nsteps, s)

@@ -30,6 +30,16 @@ from .base import GB300Engine
 _F = {torch.float32: "f32", torch.float64: "f64"}
 
 
+def _run(model, params, tiling=None, **fields) -> L.PpfRun:
+    """PpfRun of one model; the structs it points at live as long as it does."""
+    r = L.PpfRun(model=model, **fields)
+    r.params = C.addressof(params)
+    if tiling is not None:
+        r.tiling = C.pointer(tiling)
+    r.keep = (params, tiling)
+    return r
+
+
 _PHASE_SOLVERS = {"implicit": L.PPF_SOLVER_IMPLICIT, "crank-nicolson": L.PPF_SOLVER_CRANK_NICOLSON,
                   "imex": L.PPF_SOLVER_IMEX}
 
@@ -77,20 +87,28 @@ class _ImplicitPhase:
         self._ppf_scratch = torch.empty(max(16, nbytes.value), dtype=torch.uint8,
                                         device=g.device)
 
-    def _ppf_phase_step(self, src, dst, sp):
+    def _ppf_phase_params(self):
         ud = self.user_data
-        p = L.PpfImplicitPhaseParams(float(self.dx), float(self.dt), float(ud["M"]),
-                                     float(ud["W"]), float(ud["epsilon"]),
-                                     float(ud.get("implicit_tol", 0.0)), self.PHASE_MODEL,
-                                     self._ppf_phase_solver, 1 if ud.get("adi") else 0,
-                                     1 if ud.get("gmres") else 0,
-                                     int(ud.get("implicit_max_iter", 0)), 0)
+        return L.PpfImplicitPhaseParams(float(self.dx), float(self.dt), float(ud["M"]),
+                                        float(ud["W"]), float(ud["epsilon"]),
+                                        float(ud.get("implicit_tol", 0.0)), self.PHASE_MODEL,
+                                        self._ppf_phase_solver, 1 if ud.get("adi") else 0,
+                                        1 if ud.get("gmres") else 0,
+                                        int(ud.get("implicit_max_iter", 0)), 0)
+
+    def _ppf_phase_step(self, src, dst, sp):
+        p = self._ppf_phase_params()
         it = C.c_int32()
         sc = self._ppf_scratch
         L.call(f"ppf_phase_implicit_step_{_F[self._ppf_dtype]}", C.byref(p),
                C.byref(self._ppf_grid.grid), ptr(src[0]), ptr(dst[0]), ptr(self._ppf_tmp),
                ptr(sc), sc.numel(), C.byref(it), sp)
         self._ppf_iterations = it.value
+
+    def _ppf_phase_run(self):
+        return _run(L.PPF_RUN_PHASE_IMPLICIT, self._ppf_phase_params(),
+                    tmp=self._ppf_tmp.data_ptr(), scratch=self._ppf_scratch.data_ptr(),
+                    scratch_bytes=self._ppf_scratch.numel())
 
     def _ppf_phase_bc(self):
         if self._ppf_phase_solver is not None and self._boundary_conditions_type is None:
@@ -213,6 +231,13 @@ class _DiffusionMixin(GB300Engine):
                                             float(ud.get("implicit_tol", 0.0)), self._ppf_solver,
                                             1 if ud.get("adi", False) else 0)
 
+    def _ppf_run(self):
+        if self._ppf_solver != L.PPF_SOLVER_EXPLICIT:
+            return _run(L.PPF_RUN_DIFFUSION_IMPLICIT, self._ppf_implicit_params(),
+                        tmp=self._ppf_tmp.data_ptr(), scratch=self._ppf_scratch.data_ptr(),
+                        scratch_bytes=self._ppf_scratch.numel())
+        return _run(L.PPF_RUN_DIFFUSION, self._ppf_params(), self._ppf_tiling(1))
+
     def _ppf_step(self, src, dst, depth, step, step_base, sp):
         f = _F[self._ppf_dtype]
         if self._ppf_solver != L.PPF_SOLVER_EXPLICIT:
@@ -277,6 +302,11 @@ class _CahnAllenMixin(_ImplicitPhase, GB300Engine):
         ud = self.user_data
         return L.PpfAllenCahnParams(float(self.dx), float(self.dt), float(ud["M"]),
                                     float(ud["epsilon"]), float(ud["W"]))
+
+    def _ppf_run(self):
+        if self._ppf_phase_solver is not None:
+            return self._ppf_phase_run()
+        return _run(L.PPF_RUN_ALLEN_CAHN, self._ppf_params(), self._ppf_tiling(1))
 
     def _ppf_step(self, src, dst, depth, step, step_base, sp):
         if self._ppf_phase_solver is not None:
@@ -379,6 +409,15 @@ class _CahnHilliardMixin(_ImplicitPhase, GB300Engine):
             with torch.cuda.stream(stream):
                 self._ch_mass_parts.append(self._ch_mass[:nsteps].clone())
 
+    def _ppf_run(self):
+        if self._ppf_phase_solver is not None:
+            return self._ppf_phase_run()
+        track = self.user_data.get("track_mass", True)
+        # one run per segment, from its first step
+        return _run(L.PPF_RUN_CAHN_HILLIARD, self._ppf_params(), self._ppf_tiling(1),
+                    mass=self._ch_mass.data_ptr() if track else None,
+                    status=self._ppf_status.data_ptr())
+
     def _ppf_step(self, src, dst, depth, step, step_base, sp):
         if self._ppf_phase_solver is not None:
             return self._ppf_phase_step(src, dst, sp)
@@ -412,6 +451,7 @@ class _Warren1995Mixin(GB300Engine):
     """Binary Ni-Cu isothermal solidification (Engines/Warren1995.py:50-207)."""
 
     NFIELDS = 2
+    USES_STEP = True
     DEFAULTS = dict(T_mA=1728.0, T_mB=1358.0, L_A=2350000000.0, L_B=1728000000.0, s_A=0.37,
                     s_B=0.29, D_L=1e-9, D_S=1e-13, B_A=0.0033, B_B=0.0039, v_m=0.00000742,
                     R=8.314, y_e=0.04, T=1574.0, alpha=0.3, diamond_size=15)
@@ -472,6 +512,10 @@ class _Warren1995Mixin(GB300Engine):
         ud = self.user_data
         vals = dict(ud, dx=float(self.dx), dt=float(self.dt))
         return L.PpfWarren1995Params(*[float(vals[n]) for n in L.WARREN_PARAM_NAMES])
+
+    def _ppf_run(self):
+        return _run(L.PPF_RUN_WARREN1995, self._ppf_params(), self._ppf_tiling(1),
+                    seed=int(self.user_data["seed"]))
 
     def _ppf_step(self, src, dst, depth, step, step_base, sp):
         p = self._ppf_params()

@@ -159,6 +159,7 @@ def make_seed(phi, q1, q4, x, y, angle, seed_radius):
 
 class _NcgpuMixin(GB300Engine):
     NFIELDS = 4
+    USES_STEP = True
     VARIANT = L.PPF_NCGPU_VARIANT_NCGPU
 
     def __init__(self, **kwargs):
@@ -263,6 +264,15 @@ class _NcgpuMixin(GB300Engine):
         if getattr(self, "_nc_temp", None) is not None:
             self._nc_temp_staging = self._ppf_grid.upload(self._nc_temp,
                                                           self.temperature.get_cells(), s)
+
+    def _ppf_run(self):
+        r = L.PpfRun(model=L.PPF_RUN_NCGPU, tmp=self._nc_transfer.data_ptr(),
+                     seed=int(self.user_data["seed"]), temperature=self._nc_temp.data_ptr(),
+                     dT=self._nc_dT())
+        r.params = C.addressof(self._nc_params)
+        if self._nc_tables is not None:
+            r.tables = self._nc_tables.data_ptr()
+        return r
 
     def _ppf_step(self, src, dst, depth, step, step_base, sp):
         fin = (C.c_void_p * len(src))(*[ptr(t) for t in src])
