@@ -559,10 +559,11 @@ struct ChCoef {
 
 template <typename T>
 __device__ __forceinline__ T ch_mu(const ChCoef<T>& k, T c, T w, T e, T n, T s, T d, T u) {
-  const T lap = (((w + e) + (n + s)) + (d + u)) - T(6) * c;
-  // 4c^3 - 6c^2 + 2c, or in the centered variable 4u^3 - u
-  const T fp = k.centered ? c * (T(4) * c * c - T(1)) : c * (T(2) + c * (T(-6) + T(4) * c));
-  return fp - k.kap * lap;
+  const T lap = fma(T(-6), c, ((w + e) + (n + s)) + (d + u));
+  // 4c^3 - 6c^2 + 2c, or in the centered variable 4u^3 - u; the multiply-adds
+  // written out, so that the scalar and the packed form round alike
+  const T wl = k.centered ? fma(T(4) * c, c, T(-1)) : fma(c, fma(T(4), c, T(-6)), T(2));
+  return fma(c, wl, -k.kap * lap);
 }
 
 template <typename T, bool QUANT>
@@ -574,7 +575,7 @@ __device__ __forceinline__ T ch_flux(const ChCoef<T>& k, T mn, T mc) {
 
 constexpr int kNSC = 7;  // c planes z..z+2 read, z+3 .. z+5 in flight
 constexpr int kMuSlots = 3;  // mu planes z - 1, z, z + 1
-// Cahn-Hilliard tile: 32 x 32 cells, 256 threads; thread (tx, ty) owns the
+// Cahn-Hilliard tile (double): 32 x 32 cells, 256 threads; thread (tx, ty) owns the
 // kCQ = 4 xy-columns (ty + 8q, tx) and keeps, per column, c(z), c(z+1),
 // mu(z) and the flux through the face below plane z in registers while
 // marching along z (the flux through a face is computed once: the cell
@@ -611,7 +612,7 @@ __device__ __forceinline__ void ring_pos(int i, int& ly, int& lx) {
   }
 }
 
-template <typename T, bool QUANT>
+template <typename T>
 __global__ void __launch_bounds__(kThreads)
     cahn_hilliard_kernel(const __grid_constant__ CUtensorMap map, ChCoef<T> k, Geo g, Bc<T> bc,
                          const T* __restrict__ in, T* __restrict__ out, double* __restrict__ mass,
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(kThreads)
       c1[q] = P1[i];
       // flux through the face below z0, stored negated as "flux into the
       // cell below from above": the loop takes fd = -fup
-      fup[q] = -ch_flux<T, QUANT>(k, mum, mu0[q]);
+      fup[q] = -ch_flux<T, false>(k, mum, mu0[q]);
     }
     if (has_ring) M0[rmi] = mu_at(Pm1, P0, P1, rci);
   }
@@ -706,7 +707,6 @@ __global__ void __launch_bounds__(kThreads)
   // CTA-uniform: the whole tile lies inside the grid (no per-cell checks)
   const bool full = x0 + kCTX <= nx && y0 + kCTY <= ny;
 
-  long long acc_q = 0;
   double acc = 0.0;
   T vmax = T(0), vsum = T(0);
   int m0i = 0;  // mu slot of plane z
@@ -756,22 +756,20 @@ __global__ void __launch_bounds__(kThreads)
     }
     const T* M0 = mring + m0i * kMN;
     m0i = m1i;
-    int32_t quanta = 0;
 #pragma unroll
     for (int q = 0; q < kCQ; ++q) {
       const int i = mi + q * 8 * kMW;
       const T m0 = mu0[q];
-      const T fw = ch_flux<T, QUANT>(k, M0[i - 1], m0);
-      const T fe = ch_flux<T, QUANT>(k, M0[i + 1], m0);
-      const T fn = ch_flux<T, QUANT>(k, M0[i - kMW], m0);
-      const T fs = ch_flux<T, QUANT>(k, M0[i + kMW], m0);
-      const T fu = ch_flux<T, QUANT>(k, mup[q], m0);
+      const T fw = ch_flux<T, false>(k, M0[i - 1], m0);
+      const T fe = ch_flux<T, false>(k, M0[i + 1], m0);
+      const T fn = ch_flux<T, false>(k, M0[i - kMW], m0);
+      const T fs = ch_flux<T, false>(k, M0[i + kMW], m0);
+      const T fu = ch_flux<T, false>(k, mup[q], m0);
       const T fd = -fup[q];
       const T v = c0[q] + (((fw + fe) + (fn + fs)) + (fd + fu));
       if (full || q < nq) {
         optr[q * qstride] = v;
-        if (QUANT) quanta += __float2int_rn((float)(v * k.iq));  // exact: |v / q| < 2^24
-        else acc += (double)v;
+        acc += (double)v;
         vmax = fmax(vmax, fabs(v));
         vsum += v;
       }
@@ -780,17 +778,13 @@ __global__ void __launch_bounds__(kThreads)
       mu0[q] = mup[q];
       fup[q] = fu;
     }
-    acc_q += quanta;
     optr += g.plane;
   }
   int flags = 0;
-  if (QUANT && !(vmax < k.range)) flags |= PPF_STATUS_RANGE;
   if (!isfinite(vsum) || !isfinite(vmax)) flags |= PPF_STATUS_NONFINITE;
   if (status && flags) atomicOr(status, flags);
   if (mass) {
-    // QUANT: exact integer count of quanta (|sum| < 2^53), scaled by q at
-    // the end: the total is the same whatever order the CTAs add in.
-    double v = QUANT ? (double)acc_q : acc;
+    double v = acc;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (tx == 0) red[ty] = v;
@@ -799,8 +793,298 @@ __global__ void __launch_bounds__(kThreads)
       double s = tx < kThreads / 32 ? red[tx] : 0.0;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (tx == 0) atomicAdd(mass, QUANT ? s * (double)k.q : s);
+      if (tx == 0) atomicAdd(mass, s);
     }
+  }
+}
+
+// ------------------------------------------------------------- Cahn-Hilliard, float
+// A warp owns 128 columns (4 per lane) and kHR rows and marches along z, as
+// lean7_kernel does: c planes come by cp.async into a ring of its own, mu(z) and
+// mu(z + 1) of its rows and the rows beside them stay in registers, and every
+// face flux is computed once by the cell west, north or below of it and taken
+// negated by the other (x across lanes through the neighbour's mu). The columns
+// beside the strip come as 24 side cells per plane, from which lanes 0 .. 7 form
+// the eight mu values the strip's outer faces need. Nothing but a warp's own
+// copies is waited for. The arithmetic is packed (FP32x2) and rounds as
+// ch_mu / ch_flux do, so both kernels give the same bits.
+//
+// Bound: instruction issue and latency at 12 warps per SM (registers, shared
+// memory); 29.6 M warp instructions per 256^3 step where the shared-memory tiles
+// of cahn_hilliard_kernel, which this replaced in float, took 62.5 M and a block
+// barrier per plane. us per step: 256^3 87 -> 42, 384^3 235 -> 130, 128^3 33 ->
+// 12, one plane of 1500 x 2000 40 -> 13.
+constexpr int kHR = 4;              // rows per warp
+constexpr int kHWarps = 4;
+constexpr int kHRow = 128;          // elements of a row in a slot
+constexpr int kHRows = kHR + 4;     // c rows y0 - 2 .. y0 + kHR + 1
+constexpr int kHSideRows = kHR + 2; // side rows y0 - 1 .. y0 + kHR
+constexpr int kHSide = kHRows * kHRow;           // side cells: 4 columns x kHSideRows
+constexpr int kHSlot = kHSide + 32;
+static_assert(4 * kHSideRows <= 32 && 2 * kHR <= 8, "one side cell and one side mu per lane");
+constexpr int kHD = 4;                           // ring: planes z .. z + 2 in use, one coming
+template <bool FLAT>  // the ring and two sets of eight side mu values
+constexpr int kHWarpElems = (FLAT ? 1 : kHD) * kHSlot + 16;
+
+struct Quad {  // four adjacent cells of a lane
+  F2 a, b;
+};
+__device__ __forceinline__ Quad operator+(Quad x, Quad y) { return {x.a + y.a, x.b + y.b}; }
+__device__ __forceinline__ Quad operator-(Quad x, Quad y) { return {x.a - y.a, x.b - y.b}; }
+__device__ __forceinline__ Quad quad(const float4& v) { return {pk(v.x, v.y), pk(v.z, v.w)}; }
+
+__device__ __forceinline__ F2 ch_mu2(const ChCoef<float>& k, F2 c, F2 we, F2 ns, F2 du) {
+  const F2 lap = fma2(sp(-6.f), c, (we + ns) + du);
+  const F2 w = k.centered ? fma2(sp(4.f) * c, c, sp(-1.f))
+                          : fma2(c, fma2(sp(4.f), c, sp(-6.f)), sp(2.f));
+  return fma2(c, w, sp(-k.kap) * lap);
+}
+
+// Fluxes from the differences of mu across the faces, as ch_flux.
+template <bool QUANT>
+__device__ __forceinline__ float ch_scale(const ChCoef<float>& k, float d) {
+  return QUANT ? rintf(k.aiq * d) * k.q : k.a * d;
+}
+template <bool QUANT>
+__device__ __forceinline__ Quad ch_scale4(const ChCoef<float>& k, Quad d) {
+  if (!QUANT) return {sp(k.a) * d.a, sp(k.a) * d.b};
+  const F2 x = sp(k.aiq) * d.a, y = sp(k.aiq) * d.b;
+  return {pk(rintf(lo(x)), rintf(hi(x))) * sp(k.q), pk(rintf(lo(y)), rintf(hi(y))) * sp(k.q)};
+}
+template <bool QUANT>
+__device__ __forceinline__ Quad ch_flux4(const ChCoef<float>& k, Quad mn, Quad mc) {
+  return ch_scale4<QUANT>(k, mn - mc);
+}
+
+// FLAT: a single plane, its own neighbour along z (no march, no z fluxes). Off holds
+// an element's offset within a plane.
+template <bool QUANT, bool FLAT, typename Off>
+__global__ void __launch_bounds__(32 * kHWarps, 3)
+    ch_march_kernel(const __grid_constant__ ChCoef<float> k, const __grid_constant__ Geo g,
+                    const __grid_constant__ Bc<float> bc, const float* __restrict__ in,
+                    float* __restrict__ out, double* __restrict__ mass, int* __restrict__ status,
+                    int zc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x;
+  float* ring = reinterpret_cast<float*>(smem_raw) + threadIdx.y * kHWarpElems<FLAT>;
+  float* smu = ring + (FLAT ? 1 : kHD) * kHSlot;
+  const int nz = g.n[0], ny = g.n[1], nx = g.n[2];
+  const int x0 = blockIdx.x * kHRow;
+  const int y0 = (blockIdx.y * kHWarps + threadIdx.y) * kHR;
+  const int z0 = blockIdx.z * zc;
+  pdl_wait();
+  pdl_launch_next();
+  if (y0 >= ny) return;  // whole warp; no block-wide barrier follows
+  const int z1 = min(z0 + zc, nz);
+  const int x = x0 + 4 * lane;
+  // source elements within a plane; rows and columns further out than two ghost
+  // cells feed nothing that is stored
+  Off off[kHRows];
+#pragma unroll
+  for (int j = 0; j < kHRows; ++j)
+    off[j] = (Off)AxisRule<float>(g, bc, 1, min(y0 - 2 + j, ny + 1)).src * (Off)g.pitch;
+  const bool vec = x + 4 <= nx;
+  uint32_t col[4];  // a lane whose vector reaches past nx copies cell by cell
+#pragma unroll
+  for (int e = 0; e < 4; ++e) col[e] = AxisRule<float>(g, bc, 2, min(x + e, nx + 1)).src;
+  const bool used = x < nx + 2;
+  // side cell `lane`: columns x0 - 2, x0 - 1, x0 + 128, x0 + 129, kHSideRows each
+  Off side_off = 0;
+  const bool has_side = lane < 4 * kHSideRows;
+  {
+    const int q = lane / kHSideRows, j = lane - q * kHSideRows;
+    const int xc = q < 2 ? x0 - 2 + q : x0 + kHRow - 2 + q;
+    const uint32_t c = AxisRule<float>(g, bc, 2, min(xc, nx + 1)).src;
+#pragma unroll
+    for (int r = 0; r < kHSideRows; ++r)
+      if (r == j) side_off = off[r + 1] + c;
+  }
+
+  auto issue = [&](int p, int slot) {
+    float* s = ring + slot * kHSlot;
+    const int zs = (unsigned)p < (unsigned)nz ? p : AxisRule<float>(g, bc, 0, p).src;
+    const float* src = in + (int64_t)zs * g.plane;
+    if (vec) {
+      const uint32_t d = smem_addr(s + 4 * lane);
+#pragma unroll
+      for (int j = 0; j < kHRows; ++j)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4 * j * kHRow),
+                     "l"(src + off[j] + x)
+                     : "memory");
+    } else if (used) {
+#pragma unroll
+      for (int j = 0; j < kHRows; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          cp_async_elem(s + j * kHRow + 4 * lane + e, src + off[j] + col[e]);
+    }
+    if (has_side) cp_async_elem(s + kHSide + lane, src + side_off);
+  };
+  auto row = [&](const float* s, int j) {
+    return quad(*reinterpret_cast<const float4*>(s + j * kHRow + 4 * lane));
+  };
+
+  // mu of the rows y0 - 1 .. y0 + kHR of plane S1 (below it S0, above it S2);
+  // lanes 0 .. 3: of column x0 - 1, lanes 4 .. 7: of column x0 + 128, own rows
+  auto mu_rows = [&](const float* S0, const float* S1, const float* S2, Quad (&m)[kHR + 2],
+                     float& ms) {
+    Quad n = row(S1, 0), c = row(S1, 1);
+    // the columns beside the strip, for lane 0 (west) and lane 31 (east)
+    const float* sc = S1 + kHSide + (lane == 31 ? 2 : 1) * kHSideRows;
+#pragma unroll
+    for (int i = 0; i < kHR + 2; ++i) {
+      const Quad s = row(S1, i + 2);
+      const Quad du = FLAT ? c + c : row(S0, i + 1) + row(S2, i + 1);
+      const float beside = sc[i];
+      const float c0 = lo(c.a), c1 = hi(c.a), c2 = lo(c.b), c3 = hi(c.b);
+      float wl = __shfl_up_sync(0xffffffffu, c3, 1);
+      float er = __shfl_down_sync(0xffffffffu, c0, 1);
+      if (lane == 0) wl = beside;
+      if (lane == 31) er = beside;
+      const Quad ns = n + s;
+      m[i].a = ch_mu2(k, c.a, pk(wl + c1, c0 + c2), ns.a, du.a);
+      m[i].b = ch_mu2(k, c.b, pk(c1 + c3, c2 + er), ns.b, du.b);
+      n = c;
+      c = s;
+    }
+    if (lane < 2 * kHR) {
+      const int e = lane / kHR, j = lane - e * kHR;
+      const int q = (e ? 2 : 1) * kHSideRows + j + 1;  // the cell among the side cells
+      const float inner = S1[(j + 2) * kHRow + (e ? kHRow - 1 : 0)];
+      const float outer = S1[kHSide + (e ? 3 : 0) * kHSideRows + j + 1];
+      const float c1 = S1[kHSide + q];
+      ms = ch_mu(k, c1, e ? inner : outer, e ? outer : inner, S1[kHSide + q - 1],
+                 S1[kHSide + q + 1], FLAT ? c1 : S0[kHSide + q], FLAT ? c1 : S2[kHSide + q]);
+    }
+  };
+
+  Quad mu[kHR + 2], fup[kHR];
+  float ms = 0.f;
+  int s0 = 0;  // slot of plane z
+  if (FLAT) {
+    issue(0, 0);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncwarp();
+    mu_rows(ring, ring, ring, mu, ms);
+  } else {
+    // planes z0 - 2 .. z0 + 1 into slots 0 .. 3
+#pragma unroll
+    for (int q = 0; q < kHD; ++q) {
+      issue(z0 - 2 + q, q);
+      cp_async_commit();
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    Quad ml[kHR + 2];
+    float unused = 0.f;
+    mu_rows(ring, ring + kHSlot, ring + 2 * kHSlot, ml, unused);  // mu(z0 - 1)
+    __syncwarp();
+    issue(z0 + 2, 0);
+    cp_async_commit();
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    mu_rows(ring + kHSlot, ring + 2 * kHSlot, ring + 3 * kHSlot, mu, ms);  // mu(z0)
+#pragma unroll
+    for (int j = 0; j < kHR; ++j) fup[j] = ch_flux4<QUANT>(k, mu[j + 1], ml[j + 1]);
+    s0 = 2;
+  }
+  const bool full = x0 + kHRow <= nx && y0 + kHR <= ny;
+  float vmax = 0.f;
+  F2 vsum = sp(0.f);
+  long long acc_q = 0;
+  double acc = 0.0;
+  float* orow0 = out + (int64_t)z0 * g.plane + (int64_t)y0 * g.pitch + x;
+  for (int z = z0; z < z1; ++z, orow0 += g.plane) {
+    const float* S0 = ring + s0 * kHSlot;
+    // this plane's side mu to the lanes that use them
+    if (lane < 2 * kHR) smu[(z & 1) * 8 + lane] = ms;
+    Quad mun[kHR + 2];
+    if (!FLAT) {
+      const int sa = (s0 + 1) & (kHD - 1), sb = (s0 + 2) & (kHD - 1);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");  // plane z + 2
+      __syncwarp();  // every lane is done with plane z - 1, whose slot is refilled
+      if (z + 1 < z1) {
+        issue(z + 3, (s0 + 3) & (kHD - 1));
+        cp_async_commit();
+      }
+      mu_rows(S0, ring + sa * kHSlot, ring + sb * kHSlot, mun, ms);
+    } else {
+      __syncwarp();
+    }
+    const float4 side = *reinterpret_cast<const float4*>(smu + (z & 1) * 8 + (lane == 31 ? 4 : 0));
+    const float sm[4] = {side.x, side.y, side.z, side.w};
+    Quad fs = ch_flux4<QUANT>(k, mu[1], mu[0]);  // the face north of row 0
+    int32_t quanta = 0;
+    float* orow = orow0;
+#pragma unroll
+    for (int j = 0; j < kHR; ++j, orow += g.pitch) {
+      const Quad m = mu[j + 1];
+      const float m0 = lo(m.a), m1 = hi(m.a), m2 = lo(m.b), m3 = hi(m.b);
+      float mw = __shfl_up_sync(0xffffffffu, m3, 1);
+      float me = __shfl_down_sync(0xffffffffu, m0, 1);
+      if (lane == 0) mw = sm[j];
+      if (lane == 31) me = sm[j];
+      // the faces east of the cells and west of the first
+      const Quad fe = ch_scale4<QUANT>(k, {pk(m1 - m0, m2 - m1), pk(m3 - m2, me - m3)});
+      const float fw = ch_scale<QUANT>(k, m0 - mw);
+      const float e0 = lo(fe.a), e1 = hi(fe.a), e2 = lo(fe.b), e3 = hi(fe.b);
+      const Quad fx = {pk(e0 - fw, e1 - e0), pk(e2 - e1, e3 - e2)};
+      const Quad fn = fs;
+      fs = ch_flux4<QUANT>(k, mu[j + 2], m);
+      const Quad c = row(S0, j + 2);
+      Quad sum = fx + (fs - fn);
+      if (!FLAT) {
+        const Quad fu = ch_flux4<QUANT>(k, mun[j + 1], m);
+        sum = sum + (fu - fup[j]);
+        fup[j] = fu;
+      }
+      const Quad v = c + sum;
+      const float o[4] = {lo(v.a), hi(v.a), lo(v.b), hi(v.b)};
+      if (full) {
+        *reinterpret_cast<float4*>(orow) = make_float4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          vmax = fmaxf(vmax, fabsf(o[e]));
+          if (!QUANT) acc += (double)o[e];
+        }
+        if (QUANT) {  // exact: |v / q| < 2^24
+          const F2 qa = v.a * sp(k.iq), qb = v.b * sp(k.iq);
+          quanta += __float2int_rn(lo(qa)) + __float2int_rn(hi(qa));
+          quanta += __float2int_rn(lo(qb)) + __float2int_rn(hi(qb));
+        }
+        vsum = vsum + (v.a + v.b);
+      } else if (y0 + j < ny) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (x + e < nx) {
+            orow[e] = o[e];
+            vmax = fmaxf(vmax, fabsf(o[e]));
+            if (QUANT) quanta += __float2int_rn(o[e] * k.iq);
+            else acc += (double)o[e];
+            vsum = vsum + pk(o[e], 0.f);
+          }
+      }
+    }
+    acc_q += quanta;
+    if (!FLAT) {
+#pragma unroll
+      for (int i = 0; i < kHR + 2; ++i) mu[i] = mun[i];
+      s0 = (s0 + 1) & (kHD - 1);
+    }
+  }
+  cp_async_wait_all();
+  int flags = 0;
+  const float vs = lo(vsum) + hi(vsum);
+  if (QUANT && !(vmax < k.range)) flags |= PPF_STATUS_RANGE;
+  if (!isfinite(vs) || !isfinite(vmax)) flags |= PPF_STATUS_NONFINITE;
+  if (status && flags) atomicOr(status, flags);
+  if (mass) {
+    // QUANT: whole quanta (|sum| < 2^53): the same total in any order
+    double v = QUANT ? (double)acc_q : acc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) atomicAdd(mass, QUANT ? v * (double)k.q : v);
   }
 }
 
@@ -937,6 +1221,40 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
   return PPF_OK;
 }
 
+// Planes per warp: one wave of CTAs (three per SM: registers and shared memory)
+// where 2 to 32 planes make one, since a warp's planes follow one another and a
+// second wave that is nearly empty costs a whole one (256^3, us per step: 42.3 with
+// 19 planes, 46.8 with 12, 47.6 with 8, 65.6 with 32; 384^3: 130 with 32, 141 with 8).
+int32_t run_ch_march(const ChCoef<float>& k, const Geo& g, const Bc<float>& bc, const float* in,
+                     float* out, double* mass, int* status, const PpfTiling* tiling, bool quant,
+                     bool pdl, cudaStream_t s) {
+  const bool flat = g.n[0] == 1 && bc.type[0] == PPF_BC_PERIODIC;
+  const int strips = (g.n[2] + kHRow - 1) / kHRow;
+  const int bands = (g.n[1] + kHR * kHWarps - 1) / (kHR * kHWarps);
+  int zc = tiling && tiling->zchunk > 0 ? tiling->zchunk : 0;
+  if (!zc) {
+    int dev = 0, sms = 0;
+    PPF_TRY_CUDA(cudaGetDevice(&dev));
+    PPF_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long fit = 3L * sms / ((long)strips * bands);  // chunks of one wave
+    zc = fit > 0 ? (int)((g.n[0] + fit - 1) / fit) : 32;
+    zc = zc < 2 ? 2 : zc > 32 ? 32 : zc;
+  }
+  zc = zc < g.n[0] ? zc : g.n[0];
+  const dim3 gd(strips, bands, (g.n[0] + zc - 1) / zc);
+  const size_t smem = (size_t)kHWarps * (flat ? kHWarpElems<true> : kHWarpElems<false>) * sizeof(float);
+  auto pick = [&](auto off) {
+    using Off = decltype(off);
+    return quant ? (flat ? ch_march_kernel<true, true, Off> : ch_march_kernel<true, false, Off>)
+                 : (flat ? ch_march_kernel<false, true, Off> : ch_march_kernel<false, false, Off>);
+  };
+  auto kern = g.plane < (1LL << 31) ? pick(uint32_t{}) : pick(int64_t{});
+  PPF_TRY_CUDA(allow_smem(kern, smem));
+  PPF_TRY_CUDA(launch(kern, gd, dim3(32, kHWarps), smem, s, pdl, k, g, bc, in, out, mass, status,
+                      zc));
+  return PPF_OK;
+}
+
 template <typename T>
 int32_t cahn_hilliard(const PpfCahnHilliardParams* p, const PpfGrid* grid_in,
                       const PpfBoundary* b_in, const T* in, T* out, double* mass,
@@ -970,9 +1288,8 @@ int32_t cahn_hilliard(const PpfCahnHilliardParams* p, const PpfGrid* grid_in,
   ct.depth = tiling ? tiling->depth : 0;
   ct.tile_x = kCTX;
   ct.tile_y = kCTY;
+  ct.zchunk = tiling ? tiling->zchunk : 0;
   if ((rc = plan3d<T>(&ct, g, 2, kNSC, kMuSlots, &m, &slot_elems, &smem))) return rc;
-  if (slot_elems != kCSlot || m.BX != kCW || m.BY != kCH)
-    return fail(PPF_ERR_INVALID, "Cahn-Hilliard plane slot mismatch");
   ChCoef<T> k;
   k.kap = (T)(p->epsilon * p->epsilon / (p->dx * p->dx));
   k.a = (T)(p->dt * p->M / (p->dx * p->dx));
@@ -990,26 +1307,26 @@ int32_t cahn_hilliard(const PpfCahnHilliardParams* p, const PpfGrid* grid_in,
   if (p->centered != 0 && p->centered != 1)
     return fail(PPF_ERR_INVALID, "centered must be 0 or 1");
   k.centered = p->centered;
-  CUtensorMap map;
-  if ((rc = plane_map<T>(&map, in, g, m))) return rc;
-  int* st = status_ptr();
-  if (!st) return fail(PPF_ERR_CUDA, "status word unavailable");
-  dim3 gd((g.n[2] + m.TX - 1) / m.TX, (g.n[1] + m.TY - 1) / m.TY, (g.n[0] + m.ZC - 1) / m.ZC);
   const bool pdl = tiling && tiling->pdl;
-  if (quant) {
-    auto kern = cahn_hilliard_kernel<T, true>;
-    PPF_TRY_CUDA(allow_smem(kern, smem));
-    m.ZC = zchunk_of(tiling, g);
-    gd.z = (unsigned)((g.n[0] + m.ZC - 1) / m.ZC);
-    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kThreads / 32), smem, (cudaStream_t)stream, pdl,
-                        map, k, g, bc, in, out, mass, (int*)status, m, slot_elems, st));
+  if constexpr (sizeof(T) == 4) {
+    if (((uintptr_t)in) % 16 || ((uintptr_t)out) % 16)
+      return fail(PPF_ERR_INVALID, "3-D steps need 16-byte aligned rows");
+    return run_ch_march(k, g, bc, in, out, mass, (int*)status, tiling, quant, pdl,
+                        (cudaStream_t)stream);
   } else {
-    auto kern = cahn_hilliard_kernel<T, false>;
-    PPF_TRY_CUDA(allow_smem(kern, smem));
+    if (slot_elems != kCSlot || m.BX != kCW || m.BY != kCH)
+      return fail(PPF_ERR_INVALID, "Cahn-Hilliard plane slot mismatch");
+    CUtensorMap map;
+    if ((rc = plane_map<T>(&map, in, g, m))) return rc;
+    int* st = status_ptr();
+    if (!st) return fail(PPF_ERR_CUDA, "status word unavailable");
     m.ZC = zchunk_of(tiling, g);
-    gd.z = (unsigned)((g.n[0] + m.ZC - 1) / m.ZC);
-    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kThreads / 32), smem, (cudaStream_t)stream, pdl,
-                        map, k, g, bc, in, out, mass, (int*)status, m, slot_elems, st));
+    const dim3 gd((g.n[2] + m.TX - 1) / m.TX, (g.n[1] + m.TY - 1) / m.TY,
+                  (g.n[0] + m.ZC - 1) / m.ZC);
+    auto kern = cahn_hilliard_kernel<T>;
+    PPF_TRY_CUDA(allow_smem(kern, smem));
+    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kThreads / 32), smem, (cudaStream_t)stream, pdl, map, k,
+                        g, bc, in, out, mass, (int*)status, m, slot_elems, st));
   }
   return PPF_OK;
 }
