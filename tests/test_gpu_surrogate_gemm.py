@@ -1,0 +1,57 @@
+"""The surrogate's GEMM over its operand layouts and ragged tiles, and its
+depthwise kernels at channel counts with and without whole vectors."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# whole tiles, ragged multiples of 8 (the pipelined kernel), odd sizes (the other)
+@pytest.mark.parametrize("M,N,K", [(64, 64, 32), (128, 192, 96), (72, 8, 40), (8, 200, 256),
+                                   (136, 72, 24), (65, 66, 33), (63, 64, 40), (64, 62, 40)])
+@pytest.mark.parametrize("ak", [True, False])
+@pytest.mark.parametrize("bk", [True, False])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_gemm_layouts(cuda, M, N, K, ak, bk, splits):
+    import torch
+    from pyphasefield_gb300 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(M + 7 * N + K)
+    A = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    B = torch.randn(K, N, generator=g, device="cuda").bfloat16()
+    a = A.contiguous() if ak else A.t().contiguous()
+    b = B.t().contiguous() if bk else B.contiguous()
+    y = torch.ones(M, N, device="cuda")
+    bias = torch.randn(N, generator=g, device="cuda") if splits == 1 else None
+    acc = 1 if splits > 1 else 0
+    L.call("ppf_sg_gemm", C.c_void_p(a.data_ptr()), *((K, 1) if ak else (1, M)),
+           C.c_void_p(b.data_ptr()), *((1, K) if bk else (N, 1)), C.c_void_p(y.data_ptr()), N,
+           C.c_void_p(bias.data_ptr()) if bias is not None else None, acc, M, N, K, splits,
+           C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    ref = A.double() @ B.double() + (bias.double() if bias is not None else 1.0)
+    # float32 accumulation of K products of order one
+    assert float((y.double() - ref).abs().max()) < 1e-6 * K
+
+
+@pytest.mark.parametrize("Cn,E", [(6, 16), (16, 24), (18, 32), (64, 40), (72, 16)])
+def test_block_channels(cuda, Cn, E):
+    """Gradients of every parameter at channel counts of whole and of broken
+    vectors, against the float64 oracle with the same bfloat16 roundings."""
+    import torch
+    from oracle import surrogate_ref as R
+    from pyphasefield_gb300.surrogate import SurrogateNet
+    P, B, H, W = 4, 2, 20, 28
+    rng = np.random.default_rng(Cn)
+    net = SurrogateNet(P=P, C=Cn, E=E, nblocks=2, delta_scale=(2.0, 3.0))
+    net.load_params(R.random_params(P, Cn, E, 2, rng))
+    f = rng.random((2, B, 2, H, W)).astype(np.float32)
+    old, new = (torch.from_numpy(v).cuda() for v in f)
+    s = torch.cuda.current_stream()
+    net.forward(old, B, H, W, W, s)
+    net.backward(old, new, B, H, W, W, s)
+    _, ref, _ = R.loss_and_grads(net.params_numpy(), f[0].astype(np.float64),
+                                 f[1].astype(np.float64), P, 2, net.in_norm, net.delta_scale)
+    got = net.grads_numpy()
+    for n, r in ref.items():
+        assert np.linalg.norm(got[n] - r) < 1e-2 * np.linalg.norm(r), n
