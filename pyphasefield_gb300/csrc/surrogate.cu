@@ -591,7 +591,7 @@ bool tc_enabled() { return g_tc_enabled != 0; }
 
 // 5th-generation tensor-core GEMM for the GEMMs whose operands are both
 // K-contiguous bf16 (A[m][k], B stored as [n][k]): the forward 1x1
-// convolutions and the output head. One CTA (4 warps) owns a 128 x 128
+// convolutions and the output head. One CTA (8 warps) owns a 128 x 128
 // output tile whose FP32 accumulator lives in tensor memory (128 lanes x
 // 128 columns, allocated by warp 0); k advances in 64-wide tiles staged in
 // shared memory in the K-major 128-byte-swizzled layout (8-row x 128-byte
@@ -601,11 +601,11 @@ bool tc_enabled() { return g_tc_enabled != 0; }
 // loaded while the tensor core works on kt. One thread issues
 // tcgen05.mma (kind::f16, BF16 x BF16 -> F32, M = 128, N = 128, K = 16 per
 // instruction) and tcgen05.commit arrives on the stage's mbarrier; the
-// epilogue reads the accumulator with tcgen05.ld (warp w: lanes 32w..32w+31
-// = rows) and applies the storer. Every mbarrier wait is bounded; a timeout
+// epilogue reads the accumulator with tcgen05.ld (warp w: lanes
+// 32 (w % 4) .. + 31 = rows, half of the columns) and applies the storer. Every mbarrier wait is bounded; a timeout
 // sets PPF_STATUS_TIMEOUT, lets the issued MMAs finish (bounded) and frees
 // the tensor memory.
-constexpr int TCM = 128, TCN = 128, TCK = 64, kTcThreads = 128;
+constexpr int TCM = 128, TCN = 128, TCK = 64, kTcThreads = 256;
 constexpr int kTcStage = (TCM + TCN) * TCK * 2;  // bytes of one A + B stage
 constexpr uint32_t kTcIdesc = (1u << 4)                        // D: F32
                               | (1u << 7) | (1u << 10)         // A, B: BF16, K-major
@@ -645,7 +645,7 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, uint32_t
 // MMA thread (warp 1) waits for a stage, issues its four tcgen05.mma (K = 16
 // each) into the TMEM accumulator and commits onto the stage's `empty`
 // mbarrier, which frees the stage for the producer; a final commit onto
-// `done` releases the four warps into the epilogue. With three 32 KB stages
+// `done` releases the warps into the epilogue. With three 32 KB stages
 // two CTAs share an SM, so one CTA's epilogue overlaps the other's loads.
 // Every wait is bounded; a timeout sets PPF_STATUS_TIMEOUT, the issued MMAs
 // and loads are waited for (bounded) and the tensor memory is freed.
@@ -749,13 +749,16 @@ __global__ void __launch_bounds__(kTcThreads)
     // lane = row of the accumulator; 32 columns per round go through a
     // per-warp 32 x 33 shared tile so that the storer runs with consecutive
     // lanes on consecutive columns (coalesced global writes)
+    // (a warp reads the 32 accumulator rows of its number modulo four; warps w
+    // and w + 4 take half of the columns each)
+    const int q4 = warp & 3;
     float* tile = reinterpret_cast<float*>(base) + warp * 32 * 33;
 #pragma unroll 1
-    for (int c0 = 0; c0 < TCN; c0 += 32) {
+    for (int c0 = (warp >> 2) * (TCN / 2); c0 < (warp >> 2) * (TCN / 2) + TCN / 2; c0 += 32) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t r[16];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c0 + 16 * h);
+        const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(c0 + 16 * h);
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
             "%13,%14,%15}, [%16];"
@@ -770,19 +773,20 @@ __global__ void __launch_bounds__(kTcThreads)
       }
       __syncwarp();
       const long long n = n0 + c0 + lane;
-      // eight rows at a time: their reads first, then their stores (one row
-      // after the other cost the residual storer 66 us at 8192 x 192)
+      // eight rows at a time: their reads first, then their stores. The residual
+      // storer at 8192 x 192: 66 us a row at a time, 26.7 like this on four warps,
+      // 16.3 on eight (the GELU storer at 8192 x 384: 20.9 on four, 16.1)
 #pragma unroll 1
       for (int r0 = 0; r0 < 32; r0 += 8) {
         float e[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const long long m = m0 + warp * 32 + r0 + q;
+          const long long m = m0 + q4 * 32 + r0 + q;
           e[q] = m < M && n < N ? st.pre(m, n) : 0.f;
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const long long m = m0 + warp * 32 + r0 + q;
+          const long long m = m0 + q4 * 32 + r0 + q;
           if (m < M && n < N) st.put(m, n, tile[(r0 + q) * 33 + lane], e[q]);
         }
       }
@@ -1077,8 +1081,8 @@ __global__ void dwconv4_kernel(const float* __restrict__ x, const float* __restr
 // Depthwise weight and bias gradients, two channels per lane and a row of the
 // patch grid per warp: the 3 x 3 window of y moves along the row in registers
 // (three loads a token instead of nine), kDwRows rows are added up in shared
-// memory, and one atomic per CTA, channel and tap remains. 8192 x 192: 51.8 us ->
-// 20.9.
+// memory, and one atomic per CTA, channel and tap remains. The loads of eight tokens
+// are in flight together. 8192 x 192: 51.8 us -> 12.0 (20.9 a token at a time).
 constexpr int kDwRows = 4;
 __global__ void __launch_bounds__(32 * kDwRows)
     dwconv2_bwd_weight_kernel(const float* __restrict__ dh, const float* __restrict__ y,
@@ -1095,34 +1099,41 @@ __global__ void __launch_bounds__(32 * kDwRows)
     const int row = (int)(pr % gh);
     const long long t0 = pr * gw;
     const float2 zero = make_float2(0.f, 0.f);
-    float2 win[3][3];  // [dy][dx] around the token
+    auto at = [&](int j, int col) {  // y of row `row + j - 1`, column col
+      return (unsigned)(row + j - 1) < (unsigned)gh && col < gw
+                 ? __ldg(reinterpret_cast<const float2*>(
+                       y + (t0 + (long long)(j - 1) * gw + col) * C + c))
+                 : zero;
+    };
+    float2 left[3], mid[3];  // columns col - 1 and col
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      win[j][1] = zero;
-      const bool in = (unsigned)(row + j - 1) < (unsigned)gh;
-      win[j][2] = in ? __ldg(reinterpret_cast<const float2*>(
-                           y + (t0 + (long long)(j - 1) * gw) * C + c))
-                     : zero;
-    }
-#pragma unroll 4
-    for (int col = 0; col < gw; ++col) {
-      const float2 d = __ldg(reinterpret_cast<const float2*>(dh + (t0 + col) * C + c));
+    for (int j = 0; j < 3; ++j) left[j] = zero, mid[j] = at(j, 0);
+    constexpr int NT = 8;  // tokens whose loads are in flight together
+    for (int c0 = 0; c0 < gw; c0 += NT) {
+      float2 d[NT], next[3][NT];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        win[j][0] = win[j][1];
-        win[j][1] = win[j][2];
-        const bool in = (unsigned)(row + j - 1) < (unsigned)gh && col + 1 < gw;
-        win[j][2] = in ? __ldg(reinterpret_cast<const float2*>(
-                             y + (t0 + (long long)(j - 1) * gw + col + 1) * C + c))
-                       : zero;
+      for (int q = 0; q < NT; ++q) {
+        d[q] = c0 + q < gw ? __ldg(reinterpret_cast<const float2*>(dh + (t0 + c0 + q) * C + c))
+                           : zero;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          acc[3 * j + q].x = fmaf(d.x, win[j][q].x, acc[3 * j + q].x);
-          acc[3 * j + q].y = fmaf(d.y, win[j][q].y, acc[3 * j + q].y);
-        }
+        for (int j = 0; j < 3; ++j) next[j][q] = at(j, c0 + q + 1);
       }
-      acc[9].x += d.x;
-      acc[9].y += d.y;
+#pragma unroll
+      for (int q = 0; q < NT; ++q) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float2 win[3] = {left[j], mid[j], next[j][q]};
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            acc[3 * j + p].x = fmaf(d[q].x, win[p].x, acc[3 * j + p].x);
+            acc[3 * j + p].y = fmaf(d[q].y, win[p].y, acc[3 * j + p].y);
+          }
+          left[j] = mid[j];
+          mid[j] = next[j][q];
+        }
+        acc[9].x += d[q].x;
+        acc[9].y += d[q].y;
+      }
     }
   }
 #pragma unroll
