@@ -55,3 +55,38 @@ def test_block_channels(cuda, Cn, E):
     got = net.grads_numpy()
     for n, r in ref.items():
         assert np.linalg.norm(got[n] - r) < 1e-2 * np.linalg.norm(r), n
+
+
+# gathers of whole 16-byte groups (tokens: ragged tiles, one and several splits), then
+# an odd pitch, patches of 6 and channel counts without whole vectors (the other kernel)
+@pytest.mark.parametrize("P,B,gh,gw,Cn,pad", [(4, 1, 3, 5, 8, 0), (8, 2, 5, 7, 24, 4),
+                                              (16, 3, 6, 11, 72, 0), (4, 2, 21, 25, 64, 8),
+                                              (12, 1, 9, 8, 136, 0), (8, 2, 5, 7, 24, 1),
+                                              (6, 2, 5, 7, 24, 0), (8, 2, 5, 7, 18, 0)])
+def test_patch_gather(cuda, P, B, gh, gw, Cn, pad):
+    import torch
+    from pyphasefield_gb300 import _lib as L
+    H, W = gh * P, gw * P
+    T, K, pitch = B * gh * gw, 2 * P * P, W + pad
+    g = torch.Generator(device="cuda").manual_seed(P + 7 * Cn + T)
+    f = torch.randn(B, 2, H, pitch, generator=g, device="cuda")
+    w = torch.randn(Cn, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(Cn, generator=g, device="cuda")
+    dy = torch.randn(T, Cn, generator=g, device="cuda").bfloat16()
+    y, yb = torch.empty(T, Cn, device="cuda"), torch.empty(T, Cn, device="cuda").bfloat16()
+    dw, db = torch.ones(Cn, K, device="cuda"), torch.zeros(Cn, device="cuda")
+    s = L.PpfSgShape()
+    s.B, s.H, s.W, s.pitch, s.P, s.C, s.E = B, H, W, pitch, P, Cn, 8
+    s.in_off0, s.in_sc0, s.in_off1, s.in_sc1 = 0.25, 2.0, -0.5, 0.75
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    L.call("ppf_sg_patch_fwd", C.byref(s), ptr(f), ptr(w), ptr(b), ptr(y), ptr(yb), st)
+    L.call("ppf_sg_patch_bwd_weight", C.byref(s), ptr(f), ptr(dy), ptr(dw), ptr(db), st)
+    off = torch.tensor([0.25, -0.5], device="cuda").view(1, 2, 1, 1)
+    sc = torch.tensor([2.0, 0.75], device="cuda").view(1, 2, 1, 1)
+    x = ((f[..., :W] - off) * sc).bfloat16().double()
+    x = x.view(B, 2, gh, P, gw, P).permute(0, 2, 4, 1, 3, 5).reshape(T, K)
+    # float32 accumulation of K (then T) products of order one
+    assert float((y.double() - (x @ w.double().t() + b.double())).abs().max()) < 1e-6 * max(K, 64)
+    assert torch.equal(yb, y.bfloat16())
+    assert float((dw.double() - 1.0 - dy.double().t() @ x).abs().max()) < 1e-6 * max(T, 64)
