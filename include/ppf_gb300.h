@@ -572,6 +572,16 @@ int32_t ppf_sg_block_bwd(const PpfSgShape* s, const float* y, const void* h_bf16
                          void* dh_bf16, float* dy, float* dw1, float* db1,
                          float* dw2, float* db2, float* dw_dw, float* db_dw,
                          void* stream);
+/* ppf_sg_block_bwd with a bf16 copy of dy as well (dy_bf16 may be NULL, or
+ * dy_out_bf16's buffer). */
+int32_t ppf_sg_block_bwd_pair(const PpfSgShape* s, const float* y, const void* h_bf16,
+                              const float* pre, const void* act_bf16,
+                              const void* w1_bf16, const void* w2_bf16,
+                              const float* w_dw, const float* dy_out,
+                              const void* dy_out_bf16, void* dpre_bf16, float* dh,
+                              void* dh_bf16, float* dy, void* dy_bf16, float* dw1,
+                              float* db1, float* dw2, float* db2, float* dw_dw,
+                              float* db_dw, void* stream);
 int32_t ppf_sg_head_fwd(const PpfSgShape* s, const void* y_bf16,
                         const void* w_out_bf16, const float* b_out, float* out,
                         void* stream);

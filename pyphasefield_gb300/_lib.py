@@ -220,6 +220,7 @@ SIGNATURES: dict[str, list] = {
     "ppf_sg_residual": [C.POINTER(PpfSgShape), P, P, P, C.c_int32, P, P],
     "ppf_sg_block_fwd": [C.POINTER(PpfSgShape)] + [P] * 14,
     "ppf_sg_block_bwd": [C.POINTER(PpfSgShape)] + [P] * 20,
+    "ppf_sg_block_bwd_pair": [C.POINTER(PpfSgShape)] + [P] * 21,
     "ppf_sg_head_fwd": [C.POINTER(PpfSgShape), P, P, P, P, P],
     "ppf_sg_head_bwd": [C.POINTER(PpfSgShape), P, P, P, P, P, P, P, P],
     "ppf_sg_mse": [C.POINTER(PpfSgShape), P, P, P, P, P, P],

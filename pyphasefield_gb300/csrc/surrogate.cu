@@ -1045,13 +1045,13 @@ int32_t gemm(LA la, LB lb, ST st, long long M, long long N, long long K, int spl
 
 // ---------------------------------------------------------------- split-k
 // Weight gradients are GEMMs over the token axis (k = tokens, thousands),
-// split across CTAs. Each split writes its partial tile to a fixed library
-// array (16 MiB) with plain stores, and one pass adds the splits into the
-// gradient: far fewer memory operations than one atomic per split and
-// element. The array is shared by every call, so weight-gradient calls must
-// not overlap on the GPU (the network's passes run on one stream).
+// split across CTAs. Each split writes its partial tile to one of two fixed
+// library arrays (16 MiB each) with plain stores, and grad_tail_kernel adds the
+// splits into the gradient: far fewer memory operations than one atomic per
+// split and element. The arrays are shared by every call, so weight-gradient
+// calls must not overlap on the GPU (the network's passes run on one stream).
 constexpr long long kSplitkCap = 4LL << 20;  // floats
-__device__ float g_splitk[kSplitkCap];
+__device__ float g_splitk[2 * kSplitkCap];
 
 struct StorePartial {  // part[split][m][n] = acc
   float* part;
@@ -1068,17 +1068,6 @@ struct StorePartial {  // part[split][m][n] = acc
   }
 };
 
-__global__ void splitk_reduce_kernel(const float* __restrict__ part, int nz, long long mn,
-                                     float* __restrict__ y) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < mn;
-       i += (long long)gridDim.x * blockDim.x) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int z = 0; z < nz; ++z) acc += part[z * mn + i];
-    y[i] += acc;
-  }
-}
-
 // Device address of g_splitk on the current device (per device and
 // context, see SymbolCache); nullptr if the lookup failed.
 float* splitk_buffer() {
@@ -1091,26 +1080,113 @@ float* splitk_buffer() {
   return (float*)p;
 }
 
-// y[M x N] += A B with k = tokens (about 256 per split).
+// What is left of a weight gradient after its GEMM: y[mn] += the sum of nz splits.
+struct SplitSum {
+  const float* part;
+  float* y;
+  long long mn;
+  int nz;  // 0: nothing
+};
+// A bias gradient: db[n] += sum_m x[m * N + n] (x NULL: of the bf16 xb).
+struct ColSum {
+  const float* x;
+  const __nv_bfloat16* xb;
+  float* db;
+  long long M;
+  int N;
+};
+constexpr int kTailThreads = 256;
+constexpr int kColChunk = 32;  // rows added up by a thread before its atomic
+
+// The split sums and column sums of up to two weight gradients in one launch:
+// blocks of each job follow those of the job before (e0, e1, e2: where jobs 0 to 2
+// end). Each alone is a few us of latency: at 8192 tokens, 192 and 384 channels
+// a block's four were 23.2 us in four launches, 12.5 in this one (with 16 loads a
+// thread in flight; 19.5 with eight).
+__global__ void __launch_bounds__(kTailThreads)
+    grad_tail_kernel(SplitSum s0, SplitSum s1, ColSum c0, ColSum c1, unsigned e0, unsigned e1,
+                     unsigned e2) {
+  unsigned blk = blockIdx.x;
+  if (blk < e1) {
+    const bool first = blk < e0;
+    const SplitSum& s = first ? s0 : s1;
+    if (!first) blk -= e0;
+    const long long stride = (long long)(first ? e0 : e1 - e0) * kTailThreads;
+    for (long long i = (long long)blk * kTailThreads + threadIdx.x; i < s.mn; i += stride) {
+      float acc = 0.f;
+#pragma unroll 16
+      for (int z = 0; z < s.nz; ++z) acc += __ldg(s.part + z * s.mn + i);
+      s.y[i] += acc;
+    }
+    return;
+  }
+  const bool first = blk < e2;
+  const ColSum& c = first ? c0 : c1;
+  const long long i = (long long)(blk - (first ? e1 : e2)) * kTailThreads + threadIdx.x;
+  const long long chunk = i / c.N;
+  const int n = (int)(i - chunk * c.N);
+  const long long m0 = chunk * kColChunk;
+  if (m0 >= c.M) return;
+  const int rows = (int)(c.M - m0 < kColChunk ? c.M - m0 : kColChunk);
+  float acc = 0.f;
+  constexpr int NR = 16;  // rows in flight
+  for (int r = 0; r < rows; r += NR) {
+    float v[NR];
+    if (c.x) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q)
+        v[q] = r + q < rows ? __ldg(c.x + (m0 + r + q) * c.N + n) : 0.f;
+    } else {
+#pragma unroll
+      for (int q = 0; q < NR; ++q)
+        v[q] = r + q < rows ? __bfloat162float(c.xb[(m0 + r + q) * c.N + n]) : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < NR; ++q) acc += v[q];
+  }
+  atomicAdd(c.db + n, acc);
+}
+
+// Blocks of the two jobs of one weight gradient.
+inline long long tail_blocks(const SplitSum& s) {
+  const long long b = s.nz ? (s.mn + kTailThreads - 1) / kTailThreads : 0;
+  return b > 4096 ? 4096 : b;
+}
+inline long long tail_blocks(const ColSum& c) {
+  const long long t = (c.M + kColChunk - 1) / kColChunk * c.N;
+  return (t + kTailThreads - 1) / kTailThreads;
+}
+
+int32_t grad_tail(const SplitSum& s0, const ColSum& c0, const SplitSum& s1, const ColSum& c1,
+                  cudaStream_t s) {
+  const long long e0 = tail_blocks(s0), e1 = e0 + tail_blocks(s1), e2 = e1 + tail_blocks(c0),
+                  e3 = e2 + tail_blocks(c1);
+  if (e3 > (1LL << 31) - 1 || c0.M > 65535LL * kColChunk)
+    return fail(PPF_ERR_INVALID, "size out of range");
+  grad_tail_kernel<<<(unsigned)e3, kTailThreads, 0, s>>>(s0, s1, c0, c1, (unsigned)e0,
+                                                         (unsigned)e1, (unsigned)e2);
+  PPF_TRY_CUDA(cudaGetLastError());
+  return PPF_OK;
+}
+
+// y[M x N] += A B with k = tokens (about 256 per split). What the splits leave in
+// array `slot` (0 or 1) is *left, for grad_tail.
 template <typename LA, typename LB>
-int32_t gemm_wgrad(LA la, LB lb, float* y, long long M, long long N, long long K, cudaStream_t s) {
+int32_t gemm_wgrad(LA la, LB lb, float* y, long long M, long long N, long long K, int slot,
+                   SplitSum* left, cudaStream_t s) {
+  *left = SplitSum{nullptr, y, M * N, 0};
   long long splits = K / 256;
   const long long cap = kSplitkCap / (M * N);
   if (splits > cap) splits = cap;
   if (splits > 1024) splits = 1024;
   float* part = splits > 1 ? splitk_buffer() : nullptr;
   if (splits <= 1 || !part) return gemm(la, lb, StoreF32{y, nullptr, N, 1}, M, N, K, 1, s);
+  part += slot * kSplitkCap;
   long long kchunk = (K + splits - 1) / splits;
   kchunk = (kchunk + BK - 1) / BK * BK;
-  const int nz = (int)((K + kchunk - 1) / kchunk);
-  int32_t rc = gemm(la, lb, StorePartial{part, N, M * N}, M, N, K, (int)splits, s);
-  if (rc) return rc;
-  const long long mn = M * N;
-  long long blocks = (mn + 255) / 256;
-  if (blocks > 4096) blocks = 4096;
-  splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, s>>>(part, nz, mn, y);
-  PPF_TRY_CUDA(cudaGetLastError());
-  return PPF_OK;
+  left->part = part;
+  left->nz = (int)((K + kchunk - 1) / kchunk);
+  return gemm(la, lb, StorePartial{part, N, M * N}, M, N, K, (int)splits, s);
 }
 
 // ---------------------------------------------------------------- others
@@ -1201,8 +1277,9 @@ __global__ void dwconv_bwd_weight_kernel(const float* __restrict__ dh, const flo
 
 // Four channels of a token per thread (C a multiple of 4, 16-byte aligned rows):
 // the same sums in the same order, a quarter of the index arithmetic and loads.
-// DATA: dy = dy_in + the transposed convolution of x (dwconv_bwd_data_kernel),
-// else h = the convolution of x and its bf16 copy (dwconv_fwd_kernel).
+// DATA: dy = dy_in + the transposed convolution of x (dwconv_bwd_data_kernel) and,
+// with outb, its bf16 copy; else h = the convolution of x and its bf16 copy
+// (dwconv_fwd_kernel).
 // Bound: L2 traffic and latency; 8192 x 192, us: 16.2 -> 10.6, the gradient 16.1
 // and a copy of dy -> 11.5.
 template <bool DATA>
@@ -1245,10 +1322,11 @@ __global__ void dwconv4_kernel(const float* __restrict__ x, const float* __restr
       for (int e = 0; e < 4; ++e) acc[e] += wt[e * 9 + q] * p[e];
     }
   if (DATA) {
-    *reinterpret_cast<float4*>(out + t * C + c) =
-        make_float4(base.x + acc[0], base.y + acc[1], base.z + acc[2], base.w + acc[3]);
-  } else {
-    *reinterpret_cast<float4*>(out + t * C + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    acc[0] = base.x + acc[0], acc[1] = base.y + acc[1];
+    acc[2] = base.z + acc[2], acc[3] = base.w + acc[3];
+  }
+  *reinterpret_cast<float4*>(out + t * C + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  if (!DATA || outb) {
     put_pair(outb + t * C + c, acc[0], acc[1]);
     put_pair(outb + t * C + c + 2, acc[2], acc[3]);
   }
@@ -1328,49 +1406,74 @@ __global__ void __launch_bounds__(32 * kDwRows)
   }
 }
 
-// db[n] += sum_m x[m * ld + n] (bias gradient), one thread per column chunk.
-__global__ void colsum_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ xb,
-                              float* __restrict__ db, long long M, int N, long long chunk) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const long long m0 = (long long)blockIdx.y * chunk;
-  const long long m1 = m0 + chunk < M ? m0 + chunk : M;
-  float acc = 0.f;
-  for (long long m = m0; m < m1; ++m)
-    acc += x ? x[m * N + n] : __bfloat162float(xb[m * N + n]);
-  atomicAdd(db + n, acc);
-}
-
 // Loss on the network output out[t, (ch, py, px)] against the normalised
 // target change: d = out - (new - old) * scale[ch]; loss += d^2 / count;
 // grad (bf16) = 2 d / count.
-__global__ void mse_kernel(const float* __restrict__ out, const float* __restrict__ f_old,
-                           const float* __restrict__ f_new, __nv_bfloat16* __restrict__ grad,
-                           double* __restrict__ loss, long long T, int P, int H, int pitch,
-                           int gh, int gw, float s0, float s1, float inv_count) {
+//
+// V consecutive elements per thread (4: P and the pitch multiples of 4, whole 16-byte
+// vectors; else 1). The loss: each 32 elements in float, in the order of a warp's
+// xor tree over them, then in double. A CTA adds up its elements and issues one
+// atomic: one per 256 elements, all on one address, was the bound. 8 x 512 x 512,
+// us: 42.5 -> 15.8.
+constexpr int kMseThreads = 256;
+template <int V>
+__global__ void __launch_bounds__(kMseThreads)
+    mse_kernel(const float* __restrict__ out, const float* __restrict__ f_old,
+               const float* __restrict__ f_new, __nv_bfloat16* __restrict__ grad,
+               double* __restrict__ loss, long long T, int P, int H, int pitch, int gh, int gw,
+               float s0, float s1, float inv_count) {
   const int K = 2 * P * P;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  float d = 0.f;
-  if (i < T * K) {
-    const long long t = i / K;
-    const int k = (int)(i - t * K);
-    const int per = gh * gw;
-    const int b = (int)(t / per), r = (int)(t - (long long)b * per);
-    const int ty = r / gw, tx = r - ty * gw;
-    const int ch = k / (P * P), q = k - ch * P * P, py = q / P, px = q - py * P;
-    const long long o = (((long long)b * 2 + ch) * H + ty * P + py) * pitch + tx * P + px;
-    d = out[i] - (f_new[o] - f_old[o]) * (ch == 0 ? s0 : s1);
-    grad[i] = __float2bfloat16(2.f * d * inv_count);
+  const long long n = T * K, stride = (long long)gridDim.x * kMseThreads * V;
+  double sum = 0.0;
+  for (long long base = (long long)blockIdx.x * kMseThreads * V; base < n; base += stride) {
+    const long long i = base + threadIdx.x * V;
+    float v[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = 0.f;
+    if (i < n) {  // (n and K are multiples of V)
+      const long long t = i / K;
+      const int k = (int)(i - t * K);
+      const int per = gh * gw;
+      const int b = (int)(t / per), r = (int)(t - (long long)b * per);
+      const int ty = r / gw, tx = r - ty * gw;
+      const int ch = k / (P * P), q = k - ch * P * P, py = q / P, px = q - py * P;
+      const long long o = (((long long)b * 2 + ch) * H + ty * P + py) * pitch + tx * P + px;
+      const float sc = ch == 0 ? s0 : s1;
+      float a[V], x[V], y[V], d[V];
+      if (V == 4) {
+        *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(out + i);
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(f_new + o);
+        *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(f_old + o);
+      } else {
+        a[0] = out[i], x[0] = f_new[o], y[0] = f_old[o];
+      }
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        d[e] = a[e] - (x[e] - y[e]) * sc;
+        v[e] = d[e] * d[e] * inv_count;
+      }
+      if (V == 4) {
+        put_pair(grad + i, 2.f * d[0] * inv_count, 2.f * d[1] * inv_count);
+        put_pair(grad + i + 2, 2.f * d[V - 2] * inv_count, 2.f * d[V - 1] * inv_count);
+      } else {
+        grad[i] = __float2bfloat16(2.f * d[0] * inv_count);
+      }
+    }
+#pragma unroll
+    for (int o = 16 / V; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[e] += __shfl_xor_sync(0xffffffffu, v[e], o);
+    sum += V == 4 ? (v[0] + v[V / 2]) + (v[V / 4] + v[V - 1]) : v[0];
   }
-  float v = d * d * inv_count;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __shared__ float part[8];  // blockDim.x == 256
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  // every lane of a group of 32 / V holds the group's sum
+  if (threadIdx.x & (32 / V - 1)) sum = 0.0;
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  __shared__ double part[kMseThreads / 32];
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double sum = 0.0;
-    for (int w = 0; w < 8; ++w) sum += part[w];
-    if (sum != 0.0) atomicAdd(loss, sum);  // one atomic per block, not per warp
+    for (int w = 1; w < kMseThreads / 32; ++w) sum += part[w];
+    if (sum != 0.0) atomicAdd(loss, sum);
   }
 }
 
@@ -1537,11 +1640,10 @@ int32_t ppf_sg_patch_bwd_weight(const PpfSgShape* s, const float* fields, const 
   PatchGatherT lb{{fields, s->P, s->H, s->W, s->pitch, gh, gw, s->in_off0, s->in_sc0,
                    s->in_off1, s->in_sc1}};
   cudaStream_t st = (cudaStream_t)stream;
-  if ((rc = gemm_wgrad(la, lb, dw_in, s->C, K, T, st))) return rc;
-  dim3 cg((unsigned)((s->C + 127) / 128), (unsigned)((T + 31) / 32));
-  colsum_kernel<<<cg, 128, 0, st>>>(nullptr, (const __nv_bfloat16*)dy_bf16, db_in, T, s->C, 32);
-  PPF_TRY_CUDA(cudaGetLastError());
-  return PPF_OK;
+  SplitSum left;
+  if ((rc = gemm_wgrad(la, lb, dw_in, s->C, K, T, 0, &left, st))) return rc;
+  return grad_tail(left, ColSum{nullptr, (const __nv_bfloat16*)dy_bf16, db_in, T, s->C},
+                   SplitSum{}, ColSum{}, st);
 }
 
 // Depthwise conv + pointwise expand + GELU: h = dw(y), pre = h W1^T + b1,
@@ -1579,13 +1681,15 @@ int32_t ppf_sg_block_fwd(const PpfSgShape* s, const float* y, const float* w_dw,
 }
 
 // Backward of ppf_sg_block_fwd given dy_out (fp32, also bf16 copy):
-// dW2, db2, dW1, db1, dWdw, dbdw accumulate; dy (fp32) = dy_out + dwconv^T(dh).
-int32_t ppf_sg_block_bwd(const PpfSgShape* s, const float* y, const void* h_bf16,
-                         const float* pre, const void* act_bf16, const void* w1_bf16,
-                         const void* w2_bf16, const float* w_dw, const float* dy_out,
-                         const void* dy_out_bf16, void* dpre_bf16, float* dh, void* dh_bf16,
-                         float* dy, float* dw1, float* db1, float* dw2, float* db2, float* dw_dw,
-                         float* db_dw, void* stream) {
+// dW2, db2, dW1, db1, dWdw, dbdw accumulate; dy (fp32) = dy_out + dwconv^T(dh), and its
+// bf16 copy where dy_bf16 is not NULL (dy_bf16 may be dy_out_bf16).
+int32_t ppf_sg_block_bwd_pair(const PpfSgShape* s, const float* y, const void* h_bf16,
+                              const float* pre, const void* act_bf16, const void* w1_bf16,
+                              const void* w2_bf16, const float* w_dw, const float* dy_out,
+                              const void* dy_out_bf16, void* dpre_bf16, float* dh,
+                              void* dh_bf16, float* dy, void* dy_bf16, float* dw1, float* db1,
+                              float* dw2, float* db2, float* dw_dw, float* db_dw,
+                              void* stream) {
   clear_error();
   int32_t rc = sg_check(s);
   if (rc) return rc;
@@ -1595,25 +1699,21 @@ int32_t ppf_sg_block_bwd(const PpfSgShape* s, const float* y, const void* h_bf16
   // dW2[c][e] += sum_t dy_out[t][c] act[t][e]
   StridedBf16 dyT{(const __nv_bfloat16*)dy_out_bf16, 1, s->C};
   StridedBf16 act{(const __nv_bfloat16*)act_bf16, s->E, 1};
-  if ((rc = gemm_wgrad(dyT, act, dw2, s->C, s->E, T, st))) return rc;
-  const long long chunk = 32;
-  dim3 cg((s->C + 127) / 128, (unsigned)((T + chunk - 1) / chunk));
-  colsum_kernel<<<cg, 128, 0, st>>>(dy_out, nullptr, db2, T, s->C, chunk);
-  PPF_TRY_CUDA(cudaGetLastError());
+  SplitSum left2, left1;
+  if ((rc = gemm_wgrad(dyT, act, dw2, s->C, s->E, T, 0, &left2, st))) return rc;
   // d_act = dy_out W2 ; d_pre = d_act * gelu'(pre)
   StridedBf16 dyA{(const __nv_bfloat16*)dy_out_bf16, s->C, 1};
   StridedBf16 w2{(const __nv_bfloat16*)w2_bf16, s->E, 1};  // B(k=c, n=e) = W2[c][e]
   if ((rc = gemm(dyA, w2, StoreGeluGrad{pre, (__nv_bfloat16*)dpre_bf16, s->E}, T, s->E, s->C, 1,
                  st)))
     return rc;
-  // dW1[e][c] += sum_t dpre[t][e] h[t][c] ; db1
+  // dW1[e][c] += sum_t dpre[t][e] h[t][c], and both bias gradients
   StridedBf16 dpT{(const __nv_bfloat16*)dpre_bf16, 1, s->E};
   StridedBf16 hh{(const __nv_bfloat16*)h_bf16, s->C, 1};
-  if ((rc = gemm_wgrad(dpT, hh, dw1, s->E, s->C, T, st))) return rc;
-  dim3 cg1((s->E + 127) / 128, (unsigned)((T + chunk - 1) / chunk));
-  colsum_kernel<<<cg1, 128, 0, st>>>(nullptr, (const __nv_bfloat16*)dpre_bf16, db1, T, s->E,
-                                     chunk);
-  PPF_TRY_CUDA(cudaGetLastError());
+  if ((rc = gemm_wgrad(dpT, hh, dw1, s->E, s->C, T, 1, &left1, st))) return rc;
+  if ((rc = grad_tail(left2, ColSum{dy_out, nullptr, db2, T, s->C}, left1,
+                      ColSum{nullptr, (const __nv_bfloat16*)dpre_bf16, db1, T, s->E}, st)))
+    return rc;
   // dh = dpre W1
   StridedBf16 dpA{(const __nv_bfloat16*)dpre_bf16, s->E, 1};
   StridedBf16 w1{(const __nv_bfloat16*)w1_bf16, s->C, 1};  // B(k=e, n=c) = W1[e][c]
@@ -1632,20 +1732,35 @@ int32_t ppf_sg_block_bwd(const PpfSgShape* s, const float* y, const void* h_bf16
     dwconv_bwd_weight_kernel<<<wg, 128, 0, st>>>(dh, y, dw_dw, db_dw, T, s->C, gh, gw, wchunk);
   }
   PPF_TRY_CUDA(cudaGetLastError());
-  const bool four = dw_vec(s->C, 4, {dh, w_dw, dy, dy_out});
+  const bool four = dw_vec(s->C, 4, {dh, w_dw, dy, dy_out, dy_bf16});
   unsigned blocks;
   if ((rc = grid1d(four ? T * s->C / 4 : T * s->C, &blocks))) return rc;
   if (four) {
-    dwconv4_kernel<true><<<blocks, 256, 0, st>>>(dh, w_dw, nullptr, dy_out, dy, nullptr, T, s->C,
-                                                 gh, gw);
+    dwconv4_kernel<true><<<blocks, 256, 0, st>>>(dh, w_dw, nullptr, dy_out, dy,
+                                                 (__nv_bfloat16*)dy_bf16, T, s->C, gh, gw);
   } else {
     if (dy != dy_out)
       PPF_TRY_CUDA(cudaMemcpyAsync(dy, dy_out, T * s->C * sizeof(float), cudaMemcpyDeviceToDevice,
                                    st));
     dwconv_bwd_data_kernel<<<blocks, 256, 0, st>>>(dh, w_dw, dy, T, s->C, gh, gw);
+    if (dy_bf16) {
+      PPF_TRY_CUDA(cudaGetLastError());
+      cast_kernel<<<blocks, 256, 0, st>>>(dy, (__nv_bfloat16*)dy_bf16, T * s->C);
+    }
   }
   PPF_TRY_CUDA(cudaGetLastError());
   return PPF_OK;
+}
+
+int32_t ppf_sg_block_bwd(const PpfSgShape* s, const float* y, const void* h_bf16,
+                         const float* pre, const void* act_bf16, const void* w1_bf16,
+                         const void* w2_bf16, const float* w_dw, const float* dy_out,
+                         const void* dy_out_bf16, void* dpre_bf16, float* dh, void* dh_bf16,
+                         float* dy, float* dw1, float* db1, float* dw2, float* db2, float* dw_dw,
+                         float* db_dw, void* stream) {
+  return ppf_sg_block_bwd_pair(s, y, h_bf16, pre, act_bf16, w1_bf16, w2_bf16, w_dw, dy_out,
+                               dy_out_bf16, dpre_bf16, dh, dh_bf16, dy, nullptr, dw1, db1, dw2,
+                               db2, dw_dw, db_dw, stream);
 }
 
 // Output head: out = y Wout^T + bout, out [token][2 P P].
@@ -1673,11 +1788,11 @@ int32_t ppf_sg_head_bwd(const PpfSgShape* s, const void* y_bf16, const void* w_o
   cudaStream_t st = (cudaStream_t)stream;
   StridedBf16 doT{(const __nv_bfloat16*)dout_bf16, 1, K};
   StridedBf16 yy{(const __nv_bfloat16*)y_bf16, s->C, 1};
-  if ((rc = gemm_wgrad(doT, yy, dw_out, K, s->C, T, st))) return rc;
-  dim3 cg((unsigned)((K + 127) / 128), (unsigned)((T + 31) / 32));
-  colsum_kernel<<<cg, 128, 0, st>>>(nullptr, (const __nv_bfloat16*)dout_bf16, db_out, T, (int)K,
-                                    32);
-  PPF_TRY_CUDA(cudaGetLastError());
+  SplitSum left;
+  if ((rc = gemm_wgrad(doT, yy, dw_out, K, s->C, T, 0, &left, st))) return rc;
+  if ((rc = grad_tail(left, ColSum{nullptr, (const __nv_bfloat16*)dout_bf16, db_out, T, (int)K},
+                      SplitSum{}, ColSum{}, st)))
+    return rc;
   StridedBf16 doA{(const __nv_bfloat16*)dout_bf16, K, 1};
   StridedBf16 w{(const __nv_bfloat16*)w_out_bf16, s->C, 1};  // B(k=o, n=c) = Wout[o][c]
   return gemm(doA, w, StoreBf16Pair{dy, (__nv_bfloat16*)dy_bf16, nullptr, s->C}, T, s->C, K, 1,
@@ -1693,7 +1808,12 @@ int32_t ppf_sg_mse(const PpfSgShape* s, const float* out, const float* f_old, co
   const long long T = (long long)s->B * gh * gw, K = 2LL * s->P * s->P;
   unsigned blocks;
   if ((rc = grid1d(T * K, &blocks))) return rc;
-  mse_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(out, f_old, f_new,
+  const bool four = dw_vec(s->P, 4, {out, f_old, f_new}) && s->pitch % 4 == 0 &&
+                    pair_ok(grad_bf16, 2);
+  const long long per = kMseThreads * (four ? 4 : 1), need = (T * K + per - 1) / per;
+  const unsigned grid = (unsigned)(need < 1216 ? need : 1216);  // 8 CTAs per SM over 152 SMs
+  auto kern = four ? mse_kernel<4> : mse_kernel<1>;
+  kern<<<grid, kMseThreads, 0, (cudaStream_t)stream>>>(out, f_old, f_new,
                                                        (__nv_bfloat16*)grad_bf16, loss, T, s->P,
                                                        s->H, s->pitch, gh, gw, s->s0, s->s1,
                                                        1.0f / (float)(T * K));

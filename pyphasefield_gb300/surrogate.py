@@ -209,13 +209,12 @@ class SurrogateNet:
                ptr(a["dout"]), ptr(g["w_out"]), ptr(g["b_out"]), ptr(a["dy"]), ptr(a["dyb"]), sp)
         dy, dy2 = a["dy"], a["dy2"]
         for l in reversed(range(self.L)):
-            L.call("ppf_sg_block_bwd", C.byref(s), ptr(a["y"][l]), ptr(a["hb"][l]),
+            L.call("ppf_sg_block_bwd_pair", C.byref(s), ptr(a["y"][l]), ptr(a["hb"][l]),
                    ptr(a["pre"][l]), ptr(a["act"][l]), ptr(wb[f"w1_{l}"]), ptr(wb[f"w2_{l}"]),
                    ptr(w[f"dw{l}"]), ptr(dy), ptr(a["dyb"]), ptr(a["dpre"]), ptr(a["dh"]),
-                   ptr(a["dhb"]), ptr(dy2), ptr(g[f"w1_{l}"]), ptr(g[f"b1_{l}"]),
+                   ptr(a["dhb"]), ptr(dy2), ptr(a["dyb"]), ptr(g[f"w1_{l}"]), ptr(g[f"b1_{l}"]),
                    ptr(g[f"w2_{l}"]), ptr(g[f"b2_{l}"]), ptr(g[f"dw{l}"]), ptr(g[f"bdw{l}"]), sp)
             dy, dy2 = dy2, dy
-            L.call("ppf_sg_cast_bf16", ptr(dy), ptr(a["dyb"]), C.c_longlong(dy.numel()), sp)
         L.call("ppf_sg_patch_bwd_weight", C.byref(s), ptr(f_old), ptr(a["dyb"]), ptr(g["w_in"]),
                ptr(g["b_in"]), sp)
         return a["loss"]

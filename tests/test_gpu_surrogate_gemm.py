@@ -90,3 +90,67 @@ def test_patch_gather(cuda, P, B, gh, gw, Cn, pad):
     assert float((y.double() - (x @ w.double().t() + b.double())).abs().max()) < 1e-6 * max(K, 64)
     assert torch.equal(yb, y.bfloat16())
     assert float((dw.double() - 1.0 - dy.double().t() @ x).abs().max()) < 1e-6 * max(T, 64)
+
+
+# vectors of four and single elements, a ragged last CTA, more elements than one sweep
+@pytest.mark.parametrize("P,B,gh,gw,pad", [(4, 1, 1, 1, 0), (4, 3, 5, 7, 4), (6, 2, 3, 5, 0),
+                                           (8, 2, 3, 3, 1), (16, 2, 36, 40, 0), (5, 1, 90, 91, 0)])
+def test_loss_and_its_gradient(cuda, P, B, gh, gw, pad):
+    import torch
+    from pyphasefield_gb300 import _lib as L
+    H, W = gh * P, gw * P
+    T, K, pitch = B * gh * gw, 2 * P * P, W + pad
+    g = torch.Generator(device="cuda").manual_seed(T)
+    out = torch.randn(T, K, generator=g, device="cuda")
+    old, new = (torch.randn(B, 2, H, pitch, generator=g, device="cuda") for _ in range(2))
+    grad = torch.empty(T, K, device="cuda").bfloat16()
+    loss = torch.zeros(1, dtype=torch.float64, device="cuda")
+    s = L.PpfSgShape()
+    s.B, s.H, s.W, s.pitch, s.P, s.C, s.E = B, H, W, pitch, P, 8, 8
+    s.s0, s.s1 = 2.0, 3.0
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    L.call("ppf_sg_mse", C.byref(s), ptr(out), ptr(old), ptr(new), ptr(grad), ptr(loss),
+           C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    d = (new - old).double()[..., :W] * torch.tensor([2.0, 3.0], device="cuda").view(1, 2, 1, 1)
+    d = out.double() - d.view(B, 2, gh, P, gw, P).permute(0, 2, 4, 1, 3, 5).reshape(T, K)
+    # d^2 and sums of 32 in float32: 2^-24 times their few operations each
+    assert abs(float(loss) / float((d * d).mean()) - 1.0) < 1e-6
+    ref = 2.0 * d / (T * K)
+    # bfloat16 rounding of a float32 difference of numbers of order ten
+    assert float((grad.double() - ref).abs().max()) < 2.0**-8 * float(ref.abs().max())
+
+
+# channels one by one (7, 1346), then in pairs
+@pytest.mark.parametrize("Cn", [7, 1346, 6, 8])
+def test_block_gradient_pair(cuda, Cn):
+    """The bf16 copy of dy, written over dy_out's, and no copy: the same dy."""
+    import torch
+    from pyphasefield_gb300 import _lib as L
+    B, gh, gw, E = 2, 3, 5, 16
+    T = B * gh * gw
+    g = torch.Generator(device="cuda").manual_seed(Cn)
+    r = lambda *n: torch.randn(*n, generator=g, device="cuda")  # noqa: E731
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    s = L.PpfSgShape()
+    s.B, s.H, s.W, s.pitch, s.P, s.C, s.E = B, 4 * gh, 4 * gw, 4 * gw, 4, Cn, E
+    y, h, pre, act = r(T, Cn), r(T, Cn).bfloat16(), r(T, E), r(T, E).bfloat16()
+    w1, w2, wd, dyo = r(E, Cn).bfloat16(), r(Cn, E).bfloat16(), r(Cn, 9), r(T, Cn)
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def run(name, pair):
+        dyb = dyo.bfloat16()
+        dpre, dh, dhb = r(T, E).bfloat16(), r(T, Cn), r(T, Cn).bfloat16()
+        dy = torch.empty(T, Cn, device="cuda")
+        grads = [torch.zeros(n, device="cuda") for n in (E * Cn, E, Cn * E, Cn, Cn * 9, Cn)]
+        L.call(name, C.byref(s), ptr(y), ptr(h), ptr(pre), ptr(act), ptr(w1), ptr(w2), ptr(wd),
+               ptr(dyo), ptr(dyb), ptr(dpre), ptr(dh), ptr(dhb), ptr(dy),
+               *([ptr(dyb)] if pair else []), *(ptr(q) for q in grads), st)
+        # both bias gradients: a float32 sum of T numbers
+        assert torch.allclose(grads[1].double(), dpre.double().sum(0), rtol=0, atol=1e-4)
+        assert torch.allclose(grads[3].double(), dyo.double().sum(0), rtol=0, atol=1e-4)
+        return dy, dyb
+
+    dy, keep = run("ppf_sg_block_bwd", False)
+    dy2, dyb = run("ppf_sg_block_bwd_pair", True)
+    assert torch.equal(dy, dy2) and torch.equal(dyb, dy.bfloat16())
+    assert torch.equal(keep, dyo.bfloat16())
