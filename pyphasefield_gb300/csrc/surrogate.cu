@@ -1275,61 +1275,75 @@ __global__ void dwconv_bwd_weight_kernel(const float* __restrict__ dh, const flo
   atomicAdd(db + c, acc[9]);
 }
 
-// Four channels of a token per thread (C a multiple of 4, 16-byte aligned rows):
-// the same sums in the same order, a quarter of the index arithmetic and loads.
+// Two channels of kDwTokens tokens in a row per thread (C even, 8-byte aligned rows):
+// each token of y is loaded three times instead of nine, and the weights once per
+// CTA, tap by tap in shared memory (in memory a channel's nine taps are together, and
+// a warp's reads of them cost more than its tokens). The same sums in the same order.
 // DATA: dy = dy_in + the transposed convolution of x (dwconv_bwd_data_kernel) and,
 // with outb, its bf16 copy; else h = the convolution of x and its bf16 copy
-// (dwconv_fwd_kernel).
-// Bound: L2 traffic and latency; 8192 x 192, us: 16.2 -> 10.6, the gradient 16.1
-// and a copy of dy -> 11.5.
+// (dwconv_fwd_kernel). Bound: L2 traffic and latency; 8192 x 192, us: 16.2 ->
+// 9.8, the gradient 16.1 and a copy of dy -> 10.4.
+constexpr int kDwTokens = 4;
+constexpr int kDwMaxC = 1344;  // 9 C floats of shared memory
 template <bool DATA>
-__global__ void dwconv4_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                               const float* __restrict__ bd, const float* dy_in, float* out,
-                               __nv_bfloat16* __restrict__ outb, long long T, int C, int gh,
-                               int gw) {
-  const int c4 = C / 4;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= T * c4) return;
-  const long long t = i / c4;
-  const int c = (int)(i - t * c4) * 4;
-  const int per = gh * gw;
-  const int r = (int)(t % per), row = r / gw, col = r - row * gw;
-  float wt[36];
+__global__ void __launch_bounds__(256)
+    dwconv2_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                   const float* __restrict__ bd, const float* dy_in, float* out,
+                   __nv_bfloat16* __restrict__ outb, long long n, int C, int gh, int gw) {
+  extern __shared__ float wt[];  // [tap][channel]
+  const int c2 = C / 2, segs = (gw + kDwTokens - 1) / kDwTokens;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long s = i / c2;  // segment
+  const int c = (int)(i - s * c2) * 2;
+  const long long line = s / segs;  // row of a sample
+  const int col = (int)(s - line * segs) * kDwTokens, row = (int)(line % gh);
+  const long long t = line * gw + col;
+  const bool live = i < n;
+  float2 v[3][kDwTokens + 2];
 #pragma unroll
-  for (int q = 0; q < 9; ++q)
-    *reinterpret_cast<float4*>(wt + 4 * q) = __ldg(reinterpret_cast<const float4*>(w + c * 9) + q);
-  float4 v[9], base = make_float4(0.f, 0.f, 0.f, 0.f);
-  bool in[9];
+  for (int j = 0; j < 3; ++j)
 #pragma unroll
-  for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-    for (int dx = -1; dx <= 1; ++dx) {
-      const int q = (dy + 1) * 3 + dx + 1, sg = DATA ? -1 : 1;
-      in[q] = (unsigned)(row + sg * dy) < (unsigned)gh && (unsigned)(col + sg * dx) < (unsigned)gw;
-      if (in[q])
-        v[q] = __ldg(reinterpret_cast<const float4*>(
-            x + (t + (long long)(sg * dy) * gw + sg * dx) * C + c));
+    for (int q = 0; q < kDwTokens + 2; ++q) {
+      const bool in = live && (unsigned)(row + j - 1) < (unsigned)gh &&
+                      (unsigned)(col + q - 1) < (unsigned)gw;
+      v[j][q] = in ? __ldg(reinterpret_cast<const float2*>(
+                         x + (t + (long long)(j - 1) * gw + q - 1) * C + c))
+                   : make_float2(0.f, 0.f);
     }
-  if (DATA) base = *reinterpret_cast<const float4*>(dy_in + t * C + c);
-  float acc[4];
+  for (int k = threadIdx.x; k < 9 * C; k += 256) wt[k % 9 * C + k / 9] = __ldg(w + k);
+  __syncthreads();
+  if (!live) return;
+  float2 acc[kDwTokens];
+  const float2 b0 = DATA ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(bd + c);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) acc[e] = DATA ? 0.f : bd[c + e];
+  for (int q = 0; q < kDwTokens; ++q) acc[q] = b0;
 #pragma unroll
-  for (int q = 0; q < 9; ++q)
-    if (in[q]) {
-      const float* p = reinterpret_cast<const float*>(&v[q]);
+  for (int k = 0; k < 9; ++k) {
+    const int j = DATA ? 2 - k / 3 : k / 3, d = DATA ? 2 - k % 3 : k % 3;
+    const float2 wk = *reinterpret_cast<const float2*>(wt + k * C + c);
+    if ((unsigned)(row + j - 1) < (unsigned)gh) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] += wt[e * 9 + q] * p[e];
+      for (int q = 0; q < kDwTokens; ++q)
+        if ((unsigned)(col + q + d - 1) < (unsigned)gw) {
+          acc[q].x += wk.x * v[j][q + d].x;
+          acc[q].y += wk.y * v[j][q + d].y;
+        }
     }
-  if (DATA) {
-    acc[0] = base.x + acc[0], acc[1] = base.y + acc[1];
-    acc[2] = base.z + acc[2], acc[3] = base.w + acc[3];
   }
-  *reinterpret_cast<float4*>(out + t * C + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-  if (!DATA || outb) {
-    put_pair(outb + t * C + c, acc[0], acc[1]);
-    put_pair(outb + t * C + c + 2, acc[2], acc[3]);
+  float2 base[kDwTokens];
+  if (DATA) {  // dy may be dy_in: read before any is stored
+#pragma unroll
+    for (int q = 0; q < kDwTokens; ++q)
+      if (col + q < gw) base[q] = *reinterpret_cast<const float2*>(dy_in + (t + q) * C + c);
   }
+#pragma unroll
+  for (int q = 0; q < kDwTokens; ++q)
+    if (col + q < gw) {
+      const long long o = (t + q) * C + c;
+      if (DATA) acc[q] = make_float2(base[q].x + acc[q].x, base[q].y + acc[q].y);
+      put_pair(out + o, acc[q].x, acc[q].y);
+      if (!DATA || outb) put_pair(outb + o, acc[q].x, acc[q].y);
+    }
 }
 
 // Depthwise weight and bias gradients, two channels per lane and a row of the
@@ -1566,6 +1580,17 @@ bool dw_vec(int C, int n, std::initializer_list<const void*> ptrs) {
   return C % n == 0;
 }
 
+// Whether dwconv2_kernel applies (bf16 may be NULL), and its threads.
+bool dw_two(const PpfSgShape* s, std::initializer_list<const void*> ptrs, const void* bf16) {
+  for (const void* p : ptrs)
+    if ((uintptr_t)p & 7) return false;
+  return s->C % 2 == 0 && s->C <= kDwMaxC && pair_ok(bf16, 2);
+}
+long long dw_threads(const PpfSgShape* s) {
+  const int gh = s->H / s->P, gw = s->W / s->P;
+  return (long long)s->B * gh * ((gw + kDwTokens - 1) / kDwTokens) * (s->C / 2);
+}
+
 int32_t grid1d(long long n, unsigned* blocks) {
   const long long b = (n + 255) / 256;
   if (b < 1 || b > (1LL << 31) - 1) return fail(PPF_ERR_INVALID, "size out of range");
@@ -1659,11 +1684,11 @@ int32_t ppf_sg_block_fwd(const PpfSgShape* s, const float* y, const float* w_dw,
   const long long T = (long long)s->B * gh * gw;
   cudaStream_t st = (cudaStream_t)stream;
   unsigned blocks;
-  const bool four = dw_vec(s->C, 4, {y, w_dw, h, h_bf16});
-  if ((rc = grid1d(four ? T * s->C / 4 : T * s->C, &blocks))) return rc;
-  if (four)
-    dwconv4_kernel<false><<<blocks, 256, 0, st>>>(y, w_dw, b_dw, nullptr, h,
-                                                  (__nv_bfloat16*)h_bf16, T, s->C, gh, gw);
+  const bool two = dw_two(s, {y, b_dw, h}, h_bf16);
+  if ((rc = grid1d(two ? dw_threads(s) : T * s->C, &blocks))) return rc;
+  if (two)
+    dwconv2_kernel<false><<<blocks, 256, 9 * s->C * sizeof(float), st>>>(
+        y, w_dw, b_dw, nullptr, h, (__nv_bfloat16*)h_bf16, dw_threads(s), s->C, gh, gw);
   else
     dwconv_fwd_kernel<<<blocks, 256, 0, st>>>(y, w_dw, b_dw, h, (__nv_bfloat16*)h_bf16, T, s->C,
                                               gh, gw);
@@ -1732,12 +1757,12 @@ int32_t ppf_sg_block_bwd_pair(const PpfSgShape* s, const float* y, const void* h
     dwconv_bwd_weight_kernel<<<wg, 128, 0, st>>>(dh, y, dw_dw, db_dw, T, s->C, gh, gw, wchunk);
   }
   PPF_TRY_CUDA(cudaGetLastError());
-  const bool four = dw_vec(s->C, 4, {dh, w_dw, dy, dy_out, dy_bf16});
+  const bool two = dw_two(s, {dh, dy, dy_out}, dy_bf16);
   unsigned blocks;
-  if ((rc = grid1d(four ? T * s->C / 4 : T * s->C, &blocks))) return rc;
-  if (four) {
-    dwconv4_kernel<true><<<blocks, 256, 0, st>>>(dh, w_dw, nullptr, dy_out, dy,
-                                                 (__nv_bfloat16*)dy_bf16, T, s->C, gh, gw);
+  if ((rc = grid1d(two ? dw_threads(s) : T * s->C, &blocks))) return rc;
+  if (two) {
+    dwconv2_kernel<true><<<blocks, 256, 9 * s->C * sizeof(float), st>>>(
+        dh, w_dw, nullptr, dy_out, dy, (__nv_bfloat16*)dy_bf16, dw_threads(s), s->C, gh, gw);
   } else {
     if (dy != dy_out)
       PPF_TRY_CUDA(cudaMemcpyAsync(dy, dy_out, T * s->C * sizeof(float), cudaMemcpyDeviceToDevice,
