@@ -740,9 +740,9 @@ inline bool gather_operand(const PatchGather& g, long long cols, long long kspan
 
 // ---------------------------------------------------------------- tcgen05
 // The tcgen05 path is on by default for GEMMs of at least kTcMinRows rows
-// (the training batches: 8192 tokens x N 384 x K 192 runs at 74 TFLOP/s vs
-// 54 on mma.sync, 65536 tokens at 132 vs 86); below that (the 1024-token
-// prediction) its few 128 x 128 tiles leave most SMs idle and mma.sync's
+// (the training batches, N 384, K 192: 4096 tokens take 8.2 us here and on
+// mma.sync, 8192 tokens 8.3 and 12.3, 65536 tokens 41 and 59); below that (the
+// 1024-token prediction) its few tiles leave most SMs idle and mma.sync's
 // 64 x 64 tiles win. ppf_sg_set_tensor_path(0) selects mma.sync everywhere.
 int g_tc_enabled = 1;
 constexpr long long kTcMinRows = 4096;
@@ -750,25 +750,33 @@ bool tc_enabled() { return g_tc_enabled != 0; }
 
 // 5th-generation tensor-core GEMM for the GEMMs whose operands are both
 // K-contiguous bf16 (A[m][k], B stored as [n][k]): the forward 1x1
-// convolutions and the output head. One CTA (8 warps) owns a 128 x 128
+// convolutions and the output head. One CTA (8 warps) owns a 128 x TN
 // output tile whose FP32 accumulator lives in tensor memory (128 lanes x
-// 128 columns, allocated by warp 0); k advances in 64-wide tiles staged in
+// TN columns, allocated by warp 0); k advances in 64-wide tiles staged in
 // shared memory in the K-major 128-byte-swizzled layout (8-row x 128-byte
 // atoms, 1024 bytes apart along the rows: row r's 16-byte chunk j of k at
 // (r / 8) * 1024 + (r % 8) * 128 + ((j ^ (r % 8)) * 16), see tc_desc and
 // tc_load_tile). Two stages: the tile for kt + 1 is
 // loaded while the tensor core works on kt. One thread issues
-// tcgen05.mma (kind::f16, BF16 x BF16 -> F32, M = 128, N = 128, K = 16 per
+// tcgen05.mma (kind::f16, BF16 x BF16 -> F32, M = 128, N = TN, K = 16 per
 // instruction) and tcgen05.commit arrives on the stage's mbarrier; the
 // epilogue reads the accumulator with tcgen05.ld (warp w: lanes
-// 32 (w % 4) .. + 31 = rows, half of the columns) and applies the storer. Every mbarrier wait is bounded; a timeout
-// sets PPF_STATUS_TIMEOUT, lets the issued MMAs finish (bounded) and frees
-// the tensor memory.
-constexpr int TCM = 128, TCN = 128, TCK = 64, kTcThreads = 256;
-constexpr int kTcStage = (TCM + TCN) * TCK * 2;  // bytes of one A + B stage
+// 32 (w % 4) .. + 31 = rows, half of the columns) and applies the storer. Every
+// mbarrier wait is bounded; a timeout sets PPF_STATUS_TIMEOUT, lets the issued MMAs
+// finish (bounded) and frees the tensor memory.
+//
+// TN is 64, but 128 where N is a multiple of 128 from 512 on. Tiles of 64 columns
+// spread a batch more evenly over the SMs and pad N = 192 less, but read A more often.
+// us with 64 / 128 columns: 8192 x 384 8.3 / 10.2, 65536 x 192 30.8 / 36.0,
+// 65536 x 384 41.0 / 43.0, 131072 x 384 77.7 / 77.8; 8192 x 512 11.3 / 10.3,
+// 65536 x 512 (K 512) 70.4 / 67.5.
+constexpr int TCM = 128, TCK = 64, kTcThreads = 256;
+template <int TN>
+constexpr int kTcStage = (TCM + TN) * TCK * 2;  // bytes of one A + B stage
+template <int TN>
 constexpr uint32_t kTcIdesc = (1u << 4)                        // D: F32
                               | (1u << 7) | (1u << 10)         // A, B: BF16, K-major
-                              | ((uint32_t)(TCN >> 3) << 17)   // N / 8
+                              | ((uint32_t)(TN >> 3) << 17)    // N / 8
                               | ((uint32_t)(TCM >> 4) << 24);  // M / 16
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) {
@@ -798,14 +806,15 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, uint32_t
 }
 
 // Pipeline: a producer thread (warp 0) streams the k-tiles of A (128 rows)
-// and B (128 columns) into kTcStages shared-memory stages with TMA tensor
+// and B (TN columns) into kTcStages shared-memory stages with TMA tensor
 // loads (cp.async.bulk.tensor.2d, 128-byte swizzle: the K-major SW128 layout
 // the descriptors describe), completing on the stage's `full` mbarrier; an
 // MMA thread (warp 1) waits for a stage, issues its four tcgen05.mma (K = 16
 // each) into the TMEM accumulator and commits onto the stage's `empty`
 // mbarrier, which frees the stage for the producer; a final commit onto
-// `done` releases the warps into the epilogue. With three 32 KB stages
-// two CTAs share an SM, so one CTA's epilogue overlaps the other's loads.
+// `done` releases the warps into the epilogue. With three stages
+// of 24 or 32 KB two or three CTAs share an SM, so one CTA's epilogue overlaps
+// another's loads.
 // Every wait is bounded; a timeout sets PPF_STATUS_TIMEOUT, the issued MMAs
 // and loads are waited for (bounded) and the tensor memory is freed.
 constexpr int kTcStages = 3;
@@ -819,7 +828,7 @@ __device__ __forceinline__ void tc_tma_load(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-template <typename ST>
+template <int TN, typename ST>
 __global__ void __launch_bounds__(kTcThreads)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                    const __grid_constant__ CUtensorMap map_b, ST st, long long M, long long N,
@@ -829,13 +838,13 @@ __global__ void __launch_bounds__(kTcThreads)
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag, consumed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long long m0 = (long long)blockIdx.y * TCM, n0 = (long long)blockIdx.x * TCN;
+  const long long m0 = (long long)blockIdx.y * TCM, n0 = (long long)blockIdx.x * TN;
   uint8_t* const base = tc_stage + ((1024 - (tc_smem(tc_stage) & 1023)) & 1023);
-  auto sa = [&](int st_) { return base + st_ * kTcStage; };
-  auto sb = [&](int st_) { return base + st_ * kTcStage + TCM * TCK * 2; };
+  auto sa = [&](int st_) { return base + st_ * kTcStage<TN>; };
+  auto sb = [&](int st_) { return base + st_ * kTcStage<TN> + TCM * TCK * 2; };
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(tc_smem(&tmem_base)), "r"(TCN) : "memory");
+                 ::"r"(tc_smem(&tmem_base)), "r"(TN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
@@ -867,7 +876,7 @@ __global__ void __launch_bounds__(kTcThreads)
       }
       if (*(volatile int*)&abort_flag) break;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                   ::"r"(tc_smem(&full[s])), "r"((uint32_t)kTcStage) : "memory");
+                   ::"r"(tc_smem(&full[s])), "r"((uint32_t)kTcStage<TN>) : "memory");
       tc_tma_load(sa(s), &map_a, kt * TCK, (int)m0, &full[s]);
       tc_tma_load(sb(s), &map_b, kt * TCK, (int)n0, &full[s]);
       issued = kt + 1;
@@ -889,7 +898,7 @@ __global__ void __launch_bounds__(kTcThreads)
         asm volatile(
             "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
             " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-            ::"r"(tmem), "l"(da), "l"(db), "r"(kTcIdesc), "r"(acc) : "memory");
+            ::"r"(tmem), "l"(da), "l"(db), "r"(kTcIdesc<TN>), "r"(acc) : "memory");
       }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -913,7 +922,7 @@ __global__ void __launch_bounds__(kTcThreads)
     const int q4 = warp & 3;
     float* tile = reinterpret_cast<float*>(base) + warp * 32 * 33;
 #pragma unroll 1
-    for (int c0 = (warp >> 2) * (TCN / 2); c0 < (warp >> 2) * (TCN / 2) + TCN / 2; c0 += 32) {
+    for (int c0 = (warp >> 2) * (TN / 2); c0 < (warp >> 2) * (TN / 2) + TN / 2; c0 += 32) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t r[16];
@@ -934,7 +943,8 @@ __global__ void __launch_bounds__(kTcThreads)
       const long long n = n0 + c0 + lane;
       // eight rows at a time: their reads first, then their stores. The residual
       // storer at 8192 x 192: 66 us a row at a time, 26.7 like this on four warps,
-      // 16.3 on eight (the GELU storer at 8192 x 384: 20.9 on four, 16.1)
+      // 16.3 on eight (the GELU storer at 8192 x 384: 20.9 on four, 16.1), both at 128
+      // columns; 13.7 and 13.4 at 64
 #pragma unroll 1
       for (int r0 = 0; r0 < 32; r0 += 8) {
         float e[8];
@@ -963,20 +973,20 @@ __global__ void __launch_bounds__(kTcThreads)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCN)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN)
                  : "memory");
 }
 
 // Whether the tcgen05 kernel applies: both operands K-contiguous with rows
 // on 16-byte boundaries, K a multiple of 8, enough rows to fill the GPU
-// with its 128 x 128 tiles.
+// with its tiles of 128 rows.
 bool tc_eligible(const StridedBf16& la, const StridedBf16& lb, long long M, long long K) {
   return la.sj == 1 && lb.si == 1 && (la.si & 7) == 0 && (lb.sj & 7) == 0 && (K & 7) == 0 &&
          (reinterpret_cast<uintptr_t>(la.x) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(lb.x) & 15) == 0 && M >= kTcMinRows;
 }
 
-template <typename ST>
+template <int TN, typename ST>
 int32_t tc_gemm(const StridedBf16& la, const StridedBf16& lb, ST st, long long M, long long N,
                 long long K, cudaStream_t s) {
   int* status = status_ptr();
@@ -988,12 +998,12 @@ int32_t tc_gemm(const StridedBf16& la, const StridedBf16& lb, ST st, long long M
                                      (uint64_t)la.si * 2, TCK, TCM);
   if (rc) return rc;
   if ((rc = tensor_map_bf16_sw128(&mb, lb.x, (uint64_t)K, (uint64_t)N, (uint64_t)lb.sj * 2, TCK,
-                                  TCN)))
+                                  TN)))
     return rc;
-  const size_t smem = (size_t)kTcStages * kTcStage + 1024;
-  auto kern = tc_gemm_kernel<ST>;
+  const size_t smem = (size_t)kTcStages * kTcStage<TN> + 1024;
+  auto kern = tc_gemm_kernel<TN, ST>;
   PPF_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)((N + TCN - 1) / TCN), (unsigned)((M + TCM - 1) / TCM));
+  dim3 grid((unsigned)((N + TN - 1) / TN), (unsigned)((M + TCM - 1) / TCM));
   if (grid.y > 65535) return fail(PPF_ERR_INVALID, "GEMM too large");
   PPF_TRY_CUDA(launch(kern, grid, dim3(kTcThreads), smem, s, false, ma, mb, st, M, N, K, status));
   return PPF_OK;
@@ -1005,7 +1015,8 @@ int32_t gemm(LA la, LB lb, ST st, long long M, long long N, long long K, int spl
   if (M < 1 || N < 1 || K < 1) return fail(PPF_ERR_INVALID, "empty GEMM");
   if constexpr (std::is_same<LA, StridedBf16>::value && std::is_same<LB, StridedBf16>::value) {
     if (splits <= 1 && tc_enabled() && tc_eligible(la, lb, M, K))
-      return tc_gemm(la, lb, st, M, N, K, s);
+      return N >= 512 && N % 128 == 0 ? tc_gemm<128>(la, lb, st, M, N, K, s)
+                                      : tc_gemm<64>(la, lb, st, M, N, K, s);
   }
   if (splits < 1) splits = 1;
   long long kchunk = (K + splits - 1) / splits;

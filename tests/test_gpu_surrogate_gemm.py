@@ -154,3 +154,23 @@ def test_block_gradient_pair(cuda, Cn):
     dy2, dyb = run("ppf_sg_block_bwd_pair", True)
     assert torch.equal(dy, dy2) and torch.equal(dyb, dy.bfloat16())
     assert torch.equal(keep, dyo.bfloat16())
+
+
+# tcgen05 tiles of 64 columns (ragged N, and N = 520) and of 128 (512, 640); ragged M, K
+@pytest.mark.parametrize("M", [4096, 4200])
+@pytest.mark.parametrize("N,K", [(8, 64), (64, 192), (136, 40), (192, 384), (520, 72), (512, 192),
+                                 (640, 8)])
+def test_tensor_core_tiles(cuda, M, N, K):
+    import torch
+    from pyphasefield_gb300 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(M + 7 * N + K)
+    A = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    B = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    bias = torch.randn(N, generator=g, device="cuda")
+    y = torch.empty(M, N, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    L.call("ppf_sg_gemm", ptr(A), K, 1, ptr(B), 1, K, ptr(y), N, ptr(bias), 0, M, N, K, 1,
+           C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    ref = A.double() @ B.double().t() + bias.double()
+    # float32 accumulation of K products of order one
+    assert float((y.double() - ref).abs().max()) < 1e-6 * max(K, 64)
