@@ -472,6 +472,11 @@ __global__ void __launch_bounds__(32 * kMWarps, (MarchMinBlocks<T, K>::value))
 // Cells outside the grid are loaded by the boundary rule and then evolve as in
 // the marching kernel: copies (periodic wrap, no-flux mirror) follow their
 // images bit for bit, Dirichlet ghosts keep their value.
+//
+// Bound by instruction issue (0.7 of the slots at 4096^2): four cells of a row
+// take 2 shuffles and 12 arithmetic instructions a step (diffusion). Rows advanced
+// in place, and fixed ghosts looked for only where a window has some: 8192^2, us
+// per step, 33.7 -> 30.8 at 16 x 4 rows.
 template <typename Op, int R, int NW>
 __global__ void __launch_bounds__(32 * NW, 2)
     stencil2d_block_kernel(Op op, const __grid_constant__ Geo g,
@@ -535,40 +540,54 @@ __global__ void __launch_bounds__(32 * NW, 2)
 #pragma unroll
     for (int r = 0; r < R; ++r) c[r][0] = pk(v[r][0], v[r][1]), c[r][1] = pk(v[r][2], v[r][3]);
   }
+  const bool fix_x = edges && bc.type[1] == PPF_BC_DIRCHLET;
   const bool fix_y = edges && bc.type[0] == PPF_BC_DIRCHLET;
 
+  auto steps = [&](auto fixed) {
 #pragma unroll 2
-  for (int s = 1; s <= depth; ++s) {
-    float4(*eb)[2][32] = edge[s & 1];
-    eb[wid][0][lane] = make_float4(lo(c[0][0]), hi(c[0][0]), lo(c[0][1]), hi(c[0][1]));
-    eb[wid][1][lane] =
-        make_float4(lo(c[R - 1][0]), hi(c[R - 1][0]), lo(c[R - 1][1]), hi(c[R - 1][1]));
-    __syncthreads();
-    // rows s .. H - 1 - s of the window can still be computed
-    if (wid * R + R - 1 < s || wid * R > H - 1 - s) continue;
-    // the block's first and last warp read their own row: stale rows
-    const float4 a = eb[wid > 0 ? wid - 1 : 0][1][lane];
-    const float4 b = eb[wid < NW - 1 ? wid + 1 : wid][0][lane];
-    F2 prev[2] = {pk(a.x, a.y), pk(a.z, a.w)};
-    const F2 below[2] = {pk(b.x, b.y), pk(b.z, b.w)};
+    for (int s = 1; s <= depth; ++s) {
+      float4(*eb)[2][32] = edge[s & 1];
+      eb[wid][0][lane] = make_float4(lo(c[0][0]), hi(c[0][0]), lo(c[0][1]), hi(c[0][1]));
+      eb[wid][1][lane] =
+          make_float4(lo(c[R - 1][0]), hi(c[R - 1][0]), lo(c[R - 1][1]), hi(c[R - 1][1]));
+      __syncthreads();
+      // rows s .. H - 1 - s of the window can still be computed
+      if (wid * R + R - 1 < s || wid * R > H - 1 - s) continue;
+      // the block's first and last warp read their own row: stale rows
+      const float4 a = eb[wid > 0 ? wid - 1 : 0][1][lane];
+      const float4 b = eb[wid < NW - 1 ? wid + 1 : wid][0][lane];
+      const F2 below[2] = {pk(b.x, b.y), pk(b.z, b.w)};
+      // each row's sum of the rows above and below is taken before the row above
+      // changes: the rows advance in place, without copies
+      F2 ns[2] = {pk(a.x, a.y) + c[1][0], pk(a.z, a.w) + c[1][1]};
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float c0 = lo(c[r][0]), c1 = hi(c[r][0]), c2 = lo(c[r][1]), c3 = hi(c[r][1]);
-      const float wl = __shfl_up_sync(0xffffffffu, c3, 1);
-      const float er = __shfl_down_sync(0xffffffffu, c0, 1);
-      F2 nxt[2] = {op.pair(c[r][0], pk(wl + c1, c0 + c2),
-                           prev[0] + (r < R - 1 ? c[r < R - 1 ? r + 1 : r][0] : below[0])),
-                   op.pair(c[r][1], pk(c1 + c3, c2 + er),
-                           prev[1] + (r < R - 1 ? c[r < R - 1 ? r + 1 : r][1] : below[1]))};
-      if (fix) {
-        nxt[0] = pk(fix & 1u ? c0 : lo(nxt[0]), fix & 2u ? c1 : hi(nxt[0]));
-        nxt[1] = pk(fix & 4u ? c2 : lo(nxt[1]), fix & 8u ? c3 : hi(nxt[1]));
+      for (int r = 0; r < R; ++r) {
+        const float c0 = lo(c[r][0]), c1 = hi(c[r][0]), c2 = lo(c[r][1]), c3 = hi(c[r][1]);
+        const float wl = __shfl_up_sync(0xffffffffu, c3, 1);
+        const float er = __shfl_down_sync(0xffffffffu, c0, 1);
+        F2 below_ns[2];
+        if (r + 1 < R) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            below_ns[h] = c[r][h] + (r + 2 < R ? c[r + 2 < R ? r + 2 : r][h] : below[h]);
+        }
+        F2 nxt[2] = {op.pair(c[r][0], pk(wl + c1, c0 + c2), ns[0]),
+                     op.pair(c[r][1], pk(c1 + c3, c2 + er), ns[1])};
+        if constexpr (decltype(fixed)::value) {
+          if (fix) {
+            nxt[0] = pk(fix & 1u ? c0 : lo(nxt[0]), fix & 2u ? c1 : hi(nxt[0]));
+            nxt[1] = pk(fix & 4u ? c2 : lo(nxt[1]), fix & 8u ? c3 : hi(nxt[1]));
+          }
+          if (fix_y && (unsigned)(yw + r) >= (unsigned)ny) nxt[0] = c[r][0], nxt[1] = c[r][1];
+        }
+        c[r][0] = nxt[0], c[r][1] = nxt[1];
+        if (r + 1 < R) ns[0] = below_ns[0], ns[1] = below_ns[1];
       }
-      if (fix_y && (unsigned)(yw + r) >= (unsigned)ny) nxt[0] = c[r][0], nxt[1] = c[r][1];
-      prev[0] = c[r][0], prev[1] = c[r][1];
-      c[r][0] = nxt[0], c[r][1] = nxt[1];
     }
-  }
+  };
+  // fixed ghosts only where the window holds some (uniform across the CTA)
+  if (fix_x || fix_y) steps(std::true_type{});
+  else steps(std::false_type{});
   if (lane * 4 < ka || lane * 4 >= WW - ka) return;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -691,12 +710,15 @@ int32_t launch_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, 
 
 // Block shapes, smallest first. A pass takes as long as its busiest SM, and a
 // block's own time grows with its rows, so the first shape that leaves at most
-// one block per SM wins (diffusion 256^2, us per step: 0.61 with 12 x 2 rows,
-// 0.69 with 16 x 2, 0.80 and 0.89 with 12 and 16 x 4; 512^2: 0.78 with 12 x 4,
-// 0.90 with 16 x 4), then the first of the four-row shapes whose blocks are all
-// resident at two per SM (777 x 1303 Allen-Cahn: 1.28 with 12 x 4, 1.61 with
-// 16 x 4); larger grids take the tallest, which recomputes the fewest halo rows
-// (8192^2: 33.7, and 38.5 with 12 x 4).
+// one block per SM wins (diffusion 256^2, us per step: 0.55 with 12 x 2 rows,
+// 0.62 with 16 x 2, 0.71 and 0.83 with 12 and 16 x 4; 512^2: 0.71 with 12 x 4,
+// 0.84 with 16 x 4), then the first of the others whose blocks are all resident
+// at two per SM (Allen-Cahn 777 x 1303: 1.21 with 12 x 4, 1.50 with 16 x 4, 1.57
+// with 12 x 6; 1200^2: 1.61, 1.50, 1.57). Larger grids take 12 x 6, which
+// recomputes the fewest halo rows at two per SM (diffusion 1500 x 1700: 1.83, 1.92,
+// 1.62; 3001 x 2999: 4.77, 4.64, 4.06; 8192^2: 26.5 against 30.8 with 16 x 4).
+// Eight rows a lane: 4.06 with 10 warps and 25.2 at 8192^2, but Allen-Cahn 2048^2
+// 3.20 against 3.06.
 template <typename Op>
 int32_t run_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, float* out, int depth,
                   bool pdl, cudaStream_t s) {
@@ -713,7 +735,8 @@ int32_t run_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, flo
   if (blocks(24) <= sms) return launch_block<Op, 2, 12>(op, g, bc, in, out, depth, pdl, s);
   if (blocks(32) <= sms) return launch_block<Op, 2, 16>(op, g, bc, in, out, depth, pdl, s);
   if (blocks(48) <= 2 * sms) return launch_block<Op, 4, 12>(op, g, bc, in, out, depth, pdl, s);
-  return launch_block<Op, 4, 16>(op, g, bc, in, out, depth, pdl, s);
+  if (blocks(64) <= 2 * sms) return launch_block<Op, 4, 16>(op, g, bc, in, out, depth, pdl, s);
+  return launch_block<Op, 6, 12>(op, g, bc, in, out, depth, pdl, s);
 }
 
 template <typename T, typename Op>

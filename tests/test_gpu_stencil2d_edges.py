@@ -76,6 +76,19 @@ def test_block_kernel_equals_single_steps(cuda, shape, depth):
             np.testing.assert_array_equal(a, b)
 
 
+# grids of the tallest blocks (16 warps of four rows, 12 of six)
+@pytest.mark.parametrize("shape", [(1021, 1030), (1303, 1999)])
+@pytest.mark.parametrize("bc", ["PERIODIC", ["NEUMANN", "DIRCHLET"]], ids=str)
+def test_tall_blocks_equal_single_steps(cuda, shape, bc):
+    c0 = np.random.default_rng(8).random(shape)
+    vals = [[v if b == "DIRCHLET" else [0.0, 0.0]
+             for v, b in zip(face_values(bc)[0], [bc] * 2 if isinstance(bc, str) else bc)]]
+    kw = dict(M=0.1, epsilon=1.0, W=1.0, values=vals, precision="fp32")
+    a = run_single_gpu("allen_cahn", c0, 11, bc, 1.0, 0.1, **kw)
+    b = run_single_gpu("allen_cahn", c0, 11, bc, 1.0, 0.1, depth=8, **kw)
+    np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("steps", [1, 7, 50, 100, 131])
 @pytest.mark.parametrize("gradient", [0.0, 0.5])
 def test_engine_default_depth_equals_single_steps(cuda, steps, gradient):
