@@ -353,7 +353,8 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Lean 7-point kernel (the default): a warp owns 32 V columns (V cells of one
-// 16-byte vector per lane) and R rows and marches along z with planes z - 1, z
+// 16-byte vector per lane; LX = 16 or 8 lanes a row, and groups of lanes on rows of
+// their own, where x is short) and R rows and marches along z with planes z - 1, z
 // and z + 1 of its rows in registers; west / east cells come by shuffles. A
 // lane copies its own vectors of the band and of the two rows beside it, D - 1
 // planes ahead, into a ring in shared memory (cp.async) and is the only one to
@@ -369,44 +370,47 @@ __global__ void __launch_bounds__(kThreads)
 // 79, 512^3 221 -> 170; float64 200^3 309 -> 260.
 constexpr int kLWarps = 4;
 
-template <typename T, int R>
+template <typename T, int R, int LX>
 struct Lean7Slot {
   static constexpr int V = Vec16<T>::n;
-  static constexpr int side = (R + 2) * 32 * V;  // west cells, then east cells
-  static constexpr int elems = (side + 2 * R + V - 1) / V * V;
+  static constexpr int side = (R + 2) * 32 * V;  // per group: west cells, then east cells
+  static constexpr int elems = (side + 2 * R * (32 / LX) + V - 1) / V * V;
 };
 
-template <typename T, typename Op, int R, int D>
+template <typename T, typename Op, int R, int D, int LX>
 __global__ void __launch_bounds__(32 * kLWarps)
     lean7_kernel(Op op, const __grid_constant__ Geo g, const __grid_constant__ Bc<T> bc,
                  const T* __restrict__ in, T* __restrict__ out, int zc) {
   constexpr int V = Vec16<T>::n;
-  constexpr int WW = 32 * V;
+  constexpr int G = 32 / LX;  // groups of lanes, each with R rows of its own
+  constexpr int RS = 32 * V;  // elements of a row of the slot
   using VT = typename Vec16<T>::type;
-  using Slot = Lean7Slot<T, R>;
+  using Slot = Lean7Slot<T, R, LX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x;
+  const int lane = threadIdx.x, lx = G > 1 ? lane % LX : lane;
+  const int group = G > 1 ? lane / LX : 0;
   T* ring = reinterpret_cast<T*>(smem_raw) + threadIdx.y * D * Slot::elems;
-  const int x0 = blockIdx.x * WW;
-  const int y0 = (blockIdx.y * kLWarps + threadIdx.y) * R;
+  const int x0 = blockIdx.x * (LX * V);
+  const int yw = (blockIdx.y * kLWarps + threadIdx.y) * (R * G);
+  const int y0 = yw + group * R;
   const int z0 = blockIdx.z * zc;
   const int nz = g.n[0], ny = g.n[1], nx = g.n[2];
   pdl_wait();
   pdl_launch_next();
-  if (y0 >= ny) return;  // whole warp; no block-wide barrier follows
+  if (yw >= ny) return;  // whole warp; no block-wide barrier follows
   const int z1 = min(z0 + zc, nz);
-  const int x = x0 + lane * V;
+  const int x = x0 + lx * V;
   const bool vec = x + V <= nx;
-  const bool full_x = x0 + WW <= nx;
+  const bool full_x = x0 + LX * V <= nx;
   // bytes a lane copies of a row: the cells below nx, the rest of its vector
   // reads zero
   const uint32_t bytes = (uint32_t)max(0, min(V, nx - x)) * (uint32_t)sizeof(T);
-  const bool rows_in = y0 >= 1 && y0 + R + 1 <= ny;
-  const bool first = lane == 0;                             // uses the west neighbours
-  const bool last = x < nx && (lane == 31 || x + V >= nx);  // uses the east neighbours
-  const ColumnRule<T, 1, 2> wr(g, bc, x0 - 1), er(g, bc, min(x0 + WW, nx));
+  const bool rows_in = yw >= 1 && yw + R * G + 1 <= ny;     // uniform across the warp
+  const bool first = lx == 0;                               // uses the west neighbours
+  const bool last = x < nx && (lx == LX - 1 || x + V >= nx);  // uses the east neighbours
+  const ColumnRule<T, 1, 2> wr(g, bc, x0 - 1), er(g, bc, min(x0 + LX * V, nx));
   const bool x_ghost = wr.ghost || er.ghost;  // uniform across the warp
-  const bool full_y = y0 + R <= ny;
+  const bool full_y = yw + R * G <= ny;
   const int64_t out_off = (int64_t)y0 * g.pitch;
   // this lane's element of each row of a plane (planes below 2^31 elements)
   const uint32_t xs = x < nx ? x : 0;
@@ -417,12 +421,13 @@ __global__ void __launch_bounds__(32 * kLWarps)
     off[j] = (uint32_t)(rows_in ? y0 - 1 + j : AxisRule<T>(g, bc, 1, min(y0 - 1 + j, ny)).src) *
                  (uint32_t)g.pitch +
              xs;
-  // lane j < 2 R copies one side cell: west of row j, east of row j - R
+  // lane j < 2 R of a group copies one side cell: west of row j, east of row j - R
   uint32_t side_off = 0;
+  const int side_at = Slot::side + group * (2 * R);
 #pragma unroll
   for (int j = 0; j < R; ++j) {
-    if (lane == j) side_off = off[j + 1] - xs + (uint32_t)wr.xi;
-    if (lane == R + j) side_off = off[j + 1] - xs + (uint32_t)er.xi;
+    if (lx == j) side_off = off[j + 1] - xs + (uint32_t)wr.xi;
+    if (lx == R + j) side_off = off[j + 1] - xs + (uint32_t)er.xi;
   }
 
   // plane p: the band's own rows, and for a plane that is advanced the rows
@@ -437,13 +442,13 @@ __global__ void __launch_bounds__(32 * kLWarps)
     for (int j = 0; j < R + 2; ++j)
       if ((j >= 1 && j <= R) || beside)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                         d + (uint32_t)(j * WW * sizeof(T))),
+                         d + (uint32_t)(j * RS * sizeof(T))),
                      "l"(src + off[j]), "r"(bytes)
                      : "memory");
-    if (beside && lane < 2 * R) cp_async_elem(s + Slot::side + lane, src + side_off);
+    if (beside && lx < 2 * R) cp_async_elem(s + side_at + lx, src + side_off);
   };
   auto read_row = [&](const T* s, int j, T (&v)[V]) {
-    const VT q = *reinterpret_cast<const VT*>(s + j * WW + lane * V);
+    const VT q = *reinterpret_cast<const VT*>(s + j * RS + lane * V);
     const T* pq = reinterpret_cast<const T*>(&q);
 #pragma unroll
     for (int e = 0; e < V; ++e) v[e] = pq[e];
@@ -491,12 +496,12 @@ __global__ void __launch_bounds__(32 * kLWarps)
       for (int e = 0; e < V; ++e) c[j + 1][e] = c0[j][e];
 #pragma unroll
     for (int q = 0; q < 2 * R / V; ++q) {
-      const VT v = *reinterpret_cast<const VT*>(S0 + Slot::side + q * V);
+      const VT v = *reinterpret_cast<const VT*>(S0 + side_at + q * V);
       const T* pv = reinterpret_cast<const T*>(&v);
 #pragma unroll
       for (int e = 0; e < V; ++e) side[q * V + e] = pv[e];
     }
-    if (!rows_in) {  // ghost rows (uniform across the warp)
+    if (!rows_in) {  // ghost rows
 #pragma unroll
       for (int j = 0; j < R + 2; ++j) {
         const AxisRule<T> r(g, bc, 1, min(y0 - 1 + j, ny));
@@ -1169,6 +1174,46 @@ int32_t as3d(const PpfGrid* in, const PpfBoundary* bin, PpfGrid* g3, PpfBoundary
   return PPF_OK;
 }
 
+// Rows per lane: four re-read half a row per row, two a whole one; in double, where
+// the FP64 units bind, fewer registers win (200^3: 4 %).
+template <typename T>
+constexpr int kLeanRows = sizeof(T) == 4 ? 4 : 2;
+
+template <typename T>
+long lean_warps(const Geo& g, int lx) {
+  const int ww = lx * Vec16<T>::n, rows = kLeanRows<T> * (32 / lx);
+  return (long)((g.n[2] + ww - 1) / ww) * ((g.n[1] + rows - 1) / rows);
+}
+
+// Lanes per row: 32, or 16 or 8 where a row of 32 vectors would reach far past nx:
+// the fewest warps, each weighed by what its shorter rows cost (more rows and side
+// cells read beside them). In double the FP64 units bind and idle lanes cost as much
+// as busy ones: 300 x 400 x 24, us per step with 32 / 16 / 8 lanes: 208 / 115 / 116,
+// 300 x 300 x 200 566 / 493 / 468, 300 x 200 x 50 114 / 114 / 125 (the 32 x 32 tiles
+// before: 166, 581, 176). In float: 300 x 400 x 24 27 / 19 / 13, 200 x 200 x 180
+// 21.2 / 17.4 / 20.7, but 300 x 300 x 200 38.9 / 46 / 52 (48, 65, 98).
+template <typename T>
+int lean_lanes(const Geo& g) {
+  const bool f = sizeof(T) == 4;
+  const double c32 = lean_warps<T>(g, 32), c16 = (f ? 1.2 : 1.08) * lean_warps<T>(g, 16),
+               c8 = (f ? 1.5 : 1.12) * lean_warps<T>(g, 8);
+  return c32 <= c16 && c32 <= c8 ? 32 : c16 <= c8 ? 16 : 8;
+}
+
+template <typename T, typename Op, int LX>
+int32_t launch_lean7(Op op, const Geo& g, const Bc<T>& bc, const T* in, T* out, int zc, bool pdl,
+                     cudaStream_t s) {
+  constexpr int R = kLeanRows<T>, D = 4, WW = LX * Vec16<T>::n, rows = R * (32 / LX) * kLWarps;
+  const int strips = (g.n[2] + WW - 1) / WW, bands = (g.n[1] + rows - 1) / rows;
+  if (!zc) zc = lean_zchunk((long)strips * bands * kLWarps, g.n[0]);
+  const dim3 gd(strips, bands, (g.n[0] + zc - 1) / zc);
+  auto kern = lean7_kernel<T, Op, R, D, LX>;
+  const size_t smem = (size_t)kLWarps * D * Lean7Slot<T, R, LX>::elems * sizeof(T);
+  PPF_TRY_CUDA(allow_smem(kern, smem));
+  PPF_TRY_CUDA(launch(kern, gd, dim3(32, kLWarps), smem, s, pdl, op, g, bc, in, out, zc));
+  return PPF_OK;
+}
+
 template <typename T, typename Op>
 int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, const T* in,
                    T* out, const PpfTiling* tiling, void* stream) {
@@ -1194,20 +1239,14 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
     if ((rc = plan3d<T>(&lt, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
     if (((uintptr_t)in) % 16 || ((uintptr_t)out) % 16)
       return fail(PPF_ERR_INVALID, "3-D steps need 16-byte aligned rows");
-    constexpr int WW = 32 * Vec16<T>::n;
-    // four rows per warp re-read half a row per row, two a whole one; in double,
-    // where the FP64 units bind, fewer registers win (200^3: 4 %)
-    constexpr int R = sizeof(T) == 4 ? 4 : 2, D = 4;
-    const int strips = (g.n[2] + WW - 1) / WW, bands = (g.n[1] + R * kLWarps - 1) / (R * kLWarps);
-    m.ZC = tiling && tiling->zchunk > 0 ? zchunk_of(tiling, g)
-                                        : lean_zchunk((long)strips * bands * kLWarps, g.n[0]);
-    const dim3 gd(strips, bands, (g.n[0] + m.ZC - 1) / m.ZC);
-    auto kern = lean7_kernel<T, Op, R, D>;
-    smem = (size_t)kLWarps * D * Lean7Slot<T, R>::elems * sizeof(T);
-    PPF_TRY_CUDA(allow_smem(kern, smem));
-    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kLWarps), smem, (cudaStream_t)stream,
-                        tiling && tiling->pdl, op, g, bc, in, out, m.ZC));
-    return PPF_OK;
+    const cudaStream_t st7 = (cudaStream_t)stream;
+    const bool pdl = tiling && tiling->pdl;
+    const int zc = tiling && tiling->zchunk > 0 ? zchunk_of(tiling, g) : 0;
+    switch (lean_lanes<T>(g)) {
+      case 8: return launch_lean7<T, Op, 8>(op, g, bc, in, out, zc, pdl, st7);
+      case 16: return launch_lean7<T, Op, 16>(op, g, bc, in, out, zc, pdl, st7);
+      default: return launch_lean7<T, Op, 32>(op, g, bc, in, out, zc, pdl, st7);
+    }
   }
   if ((rc = plan3d<T>(tiling, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
   m.ZC = zchunk_of(tiling, g);

@@ -33,3 +33,12 @@ def test_single_step_edges(cuda, shape, bc):
             np.testing.assert_array_equal(a, b)
         ref = restate.run_single(model, c0, 3, bc, 1.0, 0.1, values=vals, **kw)
         assert rel_l2(a, ref) < 1e-12
+
+
+# short rows: groups of 16 and 8 lanes (float and double change over at different
+# widths), ragged in x and with the last groups past the grid in y
+@pytest.mark.parametrize("shape", [(3, 37, 24), (5, 70, 17), (4, 90, 40), (3, 61, 34), (2, 83, 140),
+                                   (3, 45, 64), (4, 129, 90)])
+@pytest.mark.parametrize("bc", BCS, ids=str)
+def test_short_rows(cuda, shape, bc):
+    test_single_step_edges(cuda, shape, bc)
