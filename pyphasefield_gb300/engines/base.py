@@ -184,14 +184,15 @@ class GB300Engine:
         self._ppf_cur = 0
         self._ppf_stream = torch.cuda.Stream(dev)
         self._ppf_bc = boundary_struct(self, self._ppf_grid, self.NFIELDS)
-        self._ppf_stepctr = torch.zeros(1, dtype=torch.int64, device=dev)
+        # step counter; status word and the watch's arrival counter
+        words = torch.zeros(2, dtype=torch.int64, device=dev)
+        self._ppf_stepctr = words[:1]
+        self._ppf_status, self._ppf_watch_counter = words[1:].view(torch.int32).split(1)
         # the buffers' zero fills ran on the current stream
         self._ppf_stream.wait_stream(torch.cuda.current_stream(dev))
         self._ppf_graphs = collections.OrderedDict()
         self._ppf_staging = []
-        self._ppf_status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._ppf_status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
-        self._ppf_watch_counter = torch.zeros(1, dtype=torch.int32, device=dev)
         self._ppf_status_events = collections.deque()
         self._ppf_event_pool = []
         self._uses_gpu = True
