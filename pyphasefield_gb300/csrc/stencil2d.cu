@@ -473,10 +473,11 @@ __global__ void __launch_bounds__(32 * kMWarps, (MarchMinBlocks<T, K>::value))
 // the marching kernel: copies (periodic wrap, no-flux mirror) follow their
 // images bit for bit, Dirichlet ghosts keep their value.
 //
-// Bound by instruction issue (0.7 of the slots at 4096^2): four cells of a row
-// take 2 shuffles and 12 arithmetic instructions a step (diffusion). Rows advanced
-// in place, and fixed ghosts looked for only where a window has some: 8192^2, us
-// per step, 33.7 -> 30.8 at 16 x 4 rows.
+// Bound by FP32 issue and, at two blocks per SM, the latency of a step's exchange:
+// four cells of a row take 2 shuffles and 12 arithmetic instructions a step
+// (diffusion). Rows advanced in place, and fixed ghosts looked for only where a window
+// has some: 8192^2, us per step, 33.7 -> 30.8 at 16 x 4 rows, and 22.7 with 8 warps of
+// 12 rows, whose exchange, barrier and halo rows are shared by more cells.
 template <typename Op, int R, int NW>
 __global__ void __launch_bounds__(32 * NW, 2)
     stencil2d_block_kernel(Op op, const __grid_constant__ Geo g,
@@ -708,17 +709,18 @@ int32_t launch_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, 
   return PPF_OK;
 }
 
-// Block shapes, smallest first. A pass takes as long as its busiest SM, and a
-// block's own time grows with its rows, so the first shape that leaves at most
-// one block per SM wins (diffusion 256^2, us per step: 0.55 with 12 x 2 rows,
-// 0.62 with 16 x 2, 0.71 and 0.83 with 12 and 16 x 4; 512^2: 0.71 with 12 x 4,
-// 0.84 with 16 x 4), then the first of the others whose blocks are all resident
-// at two per SM (Allen-Cahn 777 x 1303: 1.21 with 12 x 4, 1.50 with 16 x 4, 1.57
-// with 12 x 6; 1200^2: 1.61, 1.50, 1.57). Larger grids take 12 x 6, which
-// recomputes the fewest halo rows at two per SM (diffusion 1500 x 1700: 1.83, 1.92,
-// 1.62; 3001 x 2999: 4.77, 4.64, 4.06; 8192^2: 26.5 against 30.8 with 16 x 4).
-// Eight rows a lane: 4.06 with 10 warps and 25.2 at 8192^2, but Allen-Cahn 2048^2
-// 3.20 against 3.06.
+// Block shapes. A pass takes as long as its busiest SM, and a block's own time grows
+// with its rows, so the first shape that leaves at most one block per SM wins
+// (diffusion 256^2, us per step: 0.55 with 12 warps x 2 rows, 0.62 with 16 x 2, 0.71
+// and 0.83 with 12 and 16 x 4; 512^2: 0.71 with 12 x 4, 0.84 with 16 x 4), then the
+// first of 12 x 4, 16 x 4 and 12 x 6 whose blocks are all resident at two per SM
+// (Allen-Cahn 777 x 1303: 1.21, 1.50, 1.55, 1.40 with 8 x 12; 1200^2: 1.58, 1.51,
+// 1.58, 1.94; 1300^2: 1.90, 1.92, 1.59, 1.96). Larger grids, and those where it
+// leaves one block per SM (1024^2: 1.37 against 1.52 with 16 x 4), take 8 x 12: the
+// fewest halo rows, exchanges and barriers that 128 registers allow, at eight warps a
+// block (2400^2: 4.11 with 16 x 4, 4.02 with 12 x 6, 3.85; 3001 x 2999 diffusion 4.64,
+// 4.06, 3.69; 8192^2 30.8, 26.4, 22.7). 8 x 16 (8192^2 21.9, 2048^2 3.27 against
+// 3.12), 8 x 10 and 12 x 9 (24.0, 25.5) were no better.
 template <typename Op>
 int32_t run_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, float* out, int depth,
                   bool pdl, cudaStream_t s) {
@@ -735,8 +737,11 @@ int32_t run_block(Op op, const Geo& g, const Bc<float>& bc, const float* in, flo
   if (blocks(24) <= sms) return launch_block<Op, 2, 12>(op, g, bc, in, out, depth, pdl, s);
   if (blocks(32) <= sms) return launch_block<Op, 2, 16>(op, g, bc, in, out, depth, pdl, s);
   if (blocks(48) <= 2 * sms) return launch_block<Op, 4, 12>(op, g, bc, in, out, depth, pdl, s);
-  if (blocks(64) <= 2 * sms) return launch_block<Op, 4, 16>(op, g, bc, in, out, depth, pdl, s);
-  return launch_block<Op, 6, 12>(op, g, bc, in, out, depth, pdl, s);
+  if (blocks(96) > sms) {
+    if (blocks(64) <= 2 * sms) return launch_block<Op, 4, 16>(op, g, bc, in, out, depth, pdl, s);
+    if (blocks(72) <= 2 * sms) return launch_block<Op, 6, 12>(op, g, bc, in, out, depth, pdl, s);
+  }
+  return launch_block<Op, 12, 8>(op, g, bc, in, out, depth, pdl, s);
 }
 
 template <typename T, typename Op>

@@ -76,8 +76,9 @@ def test_block_kernel_equals_single_steps(cuda, shape, depth):
             np.testing.assert_array_equal(a, b)
 
 
-# grids of the tallest blocks (16 warps of four rows, 12 of six)
-@pytest.mark.parametrize("shape", [(1021, 1030), (1303, 1999)])
+# grids of the tallest blocks (8 warps of twelve rows at one and at more blocks per SM,
+# 16 of four, 12 of six)
+@pytest.mark.parametrize("shape", [(1021, 1030), (1303, 1999), (1203, 1190), (1303, 1301)])
 @pytest.mark.parametrize("bc", ["PERIODIC", ["NEUMANN", "DIRCHLET"]], ids=str)
 def test_tall_blocks_equal_single_steps(cuda, shape, bc):
     c0 = np.random.default_rng(8).random(shape)
