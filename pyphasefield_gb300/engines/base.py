@@ -21,7 +21,7 @@ User-data keys added to the reference's: precision ("fp32" | "fp64"),
 temporal_depth (steps per HBM pass, 2-D Diffusion/Allen-Cahn; 1, the
 default, leaves the steps per pass to the engine), tile
 ((tile_x, tile_y) or None; Warren1995: (0, rows per warp band), chosen by
-grid size when None), zchunk (planes per CTA, 3-D), autotune (bool: time the
+grid size when None), zchunk (planes per warp or CTA, 3-D), autotune (bool: time the
 launch shapes on scratch copies and cache the fastest), bulk_shortcut
 (bool, Warren1995), pdl (bool), use_graph (bool), graph_chunk (int),
 check_status (bool, default True).
