@@ -747,6 +747,14 @@ __global__ void __launch_bounds__(128)
 // 4.0 (8.3 -> 4.9) and double 44.5 -> 21.4 (58.8 -> 24.8), 256^3 float 82 ->
 // 30 (90 -> 44) and double 588 -> 307 (953 -> 312).
 constexpr int kFusedSegs = 128;
+// The root's rounding to the field's type shifts alpha by sqrt(alpha) ulps, and
+// line_fused takes every constant from the rounded root, where the three launches
+// take the carries' from the root in double. Errors against extended precision on
+// fields of zero mean, one launch / three: at most 1.6 (float) and 2.1 (double) up
+// to alpha 175, 3.7 and 3.3 at 700, 15 and 7 at 1e5, 50 and 30 at 1e7; from 1e15 the
+// rounded float root is 1. (On fields with a mean the one launch is the more
+// accurate throughout.)
+constexpr double kFusedMaxAlpha = 128.0;
 constexpr int kCarryW = 36;  // 33 weights, a multiple of 16 bytes
 
 // W[k] = R^k, k <= 32, in shared memory; B batches of 32 segments.
@@ -819,22 +827,28 @@ __device__ __forceinline__ void carry_scan(int mc, const CarryCoef<T>& cc, int l
   if (lane == 0) Bu[mc] = x0;
 }
 
-// Right-hand side from c and its neighbours' sum. In double the weights are
-// divided by w1 (the solution is scaled back in kappa): one operation less.
-template <typename T>
+// Right-hand side c + ea (ab - 2 c) from c and its neighbours' sum ab: a uniform
+// field comes back unchanged whatever ea is. DIVIDED: by ea, one operation less
+// (kappa scales the solution back). The weight 1/ea - 2 is rounded, an error of ea
+// ulps in every mode but the uniform one, so that form is for small ea (kMaxDivided),
+// and for double, where every operation counts: 1024 x 1400 Crank-Nicolson ADI, one
+// call of 20 steps 1014 us against 1102.
+template <bool DIVIDED, typename T>
 __device__ __forceinline__ T half_step(const LineCoef<T>& k, T c, T ab) {
-  if constexpr (sizeof(T) == 8)
-    return fma(k.w0, c, ab);
-  else
-    return k.w0 * c + k.w1 * ab;
+  return DIVIDED ? fma(k.w0, c, ab) : fma(k.w1, fma(T(-2), c, ab), c);
 }
+constexpr double kMaxDivided = 4.0;
 
-template <typename T, int LS, int B, int EXPL, bool X>
+// MODE: 0 no explicit part, 1 along the solved axis, 2 along another one; 3 and 4 as
+// 1 and 2 with the divided half step.
+template <typename T, int LS, int B, int MODE, bool X>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512)
     line_fused(const __grid_constant__ Lines L, const __grid_constant__ LineCoef<T> k,
                const __grid_constant__ CarryCoef<T> cc, const T* __restrict__ in,
                T* __restrict__ out, int nl, int vec_ok) {
   constexpr int V = 16 / (int)sizeof(T);
+  constexpr int EXPL = MODE > 2 ? MODE - 2 : MODE;
+  constexpr bool DIVIDED = MODE > 2;
   constexpr int PS = LS + V;  // a segment's elements in shared memory (x lines)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -877,7 +891,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512)
         [&](const T* row, int line, int i) {
           int64_t em, ep;
           wrap_offsets(L.e_is_y ? line % L.ny : line / L.ny, L.ne, L.estride, em, ep);
-          return half_step(k, __ldg(row + i), __ldg(row + em + i) + __ldg(row + ep + i));
+          return half_step<DIVIDED>(k, __ldg(row + i), __ldg(row + em + i) + __ldg(row + ep + i));
         });
     if (ok) {
       segment_in<T, LS>(tile + (ln * ns + sg) * PS, len, d);
@@ -913,8 +927,8 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512)
 #pragma unroll
       for (int j = 0; j < LS; ++j)
         if (j < len)
-          d[j] = half_step(k, d[j], __ldg(p + (int64_t)j * L.stride + em) +
-                                        __ldg(p + (int64_t)j * L.stride + ep));
+          d[j] = half_step<DIVIDED>(k, d[j], __ldg(p + (int64_t)j * L.stride + em) +
+                                                 __ldg(p + (int64_t)j * L.stride + ep));
     }
   }
   if (EXPL == 1) {
@@ -923,7 +937,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512)
     for (int j = 0; j < LS; ++j) {
       const T cur = d[j];
       const T nxt = j + 1 < LS ? d[j + 1 < LS ? j + 1 : j] : cp;
-      if (j < len) d[j] = half_step(k, cur, prev + (j + 1 == len ? cp : nxt));
+      if (j < len) d[j] = half_step<DIVIDED>(k, cur, prev + (j + 1 == len ? cp : nxt));
       prev = cur;
     }
   }
@@ -1136,7 +1150,7 @@ void carry_coef(double r, int n, int seglen, int nseg, CarryCoef<T>& cc) {
   for (int b = 0; b < 6; ++b) cc.Rp[b] = (T)pow(R, (double)(1 << b));
 }
 
-template <typename T, int LS, int MAXB, int EXPL, bool X>
+template <typename T, int LS, int MAXB, int MODE, bool X>
 int32_t launch_fused(Lines L, const LineCoef<T>& k, double r, const T* in, T* out,
                      cudaStream_t st) {
   constexpr int V = 16 / (int)sizeof(T);
@@ -1154,9 +1168,9 @@ int32_t launch_fused(Lines L, const LineCoef<T>& k, double r, const T* in, T* ou
                          : (int64_t)((L.nx + nl - 1) / nl) * L.no;
   if (ctas > 0x7fffffff) return fail(PPF_ERR_INVALID, "grid too large for the line solver");
   const int vec_ok = ((uintptr_t)in) % 16 == 0 && ((uintptr_t)out) % 16 == 0;
-  auto kern = L.nseg <= 33 ? line_fused<T, LS, 1, EXPL, X> : line_fused<T, LS, 2, EXPL, X>;
+  auto kern = L.nseg <= 33 ? line_fused<T, LS, 1, MODE, X> : line_fused<T, LS, 2, MODE, X>;
   if constexpr (MAXB == 4)
-    if (L.nseg > 65) kern = line_fused<T, LS, 4, EXPL, X>;
+    if (L.nseg > 65) kern = line_fused<T, LS, 4, MODE, X>;
   PPF_TRY_CUDA(allow_smem(kern, smem));
   PPF_TRY_CUDA(launch(kern, dim3((unsigned)ctas), dim3(threads), smem, st, true, L, k, cc, in, out,
                       nl, vec_ok));
@@ -1179,20 +1193,20 @@ int fused_segment(const Lines& L, bool x) {
   return 16;
 }
 
-template <typename T, int EXPL>
+template <typename T, int MODE>
 int32_t launch_fused_axis(const Lines& L, const LineCoef<T>& k, double r, const T* in, T* out,
                           cudaStream_t st) {
   const bool x = L.seglen == kXSegV;
   switch (fused_segment<T>(L, x)) {
     case 8:
-      return x ? launch_fused<T, 8, 2, EXPL, true>(L, k, r, in, out, st)
-               : launch_fused<T, 8, 2, EXPL, false>(L, k, r, in, out, st);
+      return x ? launch_fused<T, 8, 2, MODE, true>(L, k, r, in, out, st)
+               : launch_fused<T, 8, 2, MODE, false>(L, k, r, in, out, st);
     case 16:
-      return x ? launch_fused<T, 16, 4, EXPL, true>(L, k, r, in, out, st)
-               : launch_fused<T, 16, 4, EXPL, false>(L, k, r, in, out, st);
+      return x ? launch_fused<T, 16, 4, MODE, true>(L, k, r, in, out, st)
+               : launch_fused<T, 16, 4, MODE, false>(L, k, r, in, out, st);
     default:
-      return x ? launch_fused<T, 32, 4, EXPL, true>(L, k, r, in, out, st)
-               : launch_fused<T, 32, 4, EXPL, false>(L, k, r, in, out, st);
+      return x ? launch_fused<T, 32, 4, MODE, true>(L, k, r, in, out, st)
+               : launch_fused<T, 32, 4, MODE, false>(L, k, r, in, out, st);
   }
 }
 
@@ -1244,31 +1258,29 @@ int32_t line_sweep(const Geo& g, int axis, double a, int eaxis, double ea, const
   CarryCoef<T> cc{};
   carry_coef(r, L.n, L.seglen, L.nseg, cc);
   for (int b = 0; b < 8; ++b) k.rbit[b] = (T)pow(r, (double)(1 << b));
-  // whole lines in one launch while a line's segments fit a CTA; in double the
-  // explicit weights are divided by w1, which has to be far from underflow.
+  // whole lines in one launch while a line's segments fit a CTA and the root is
+  // not close to 1 (kFusedMaxAlpha).
   // Long float columns without an explicit part stay with the three launches:
   // the CTA is then one per SM with nothing to hide its loads behind (3000^2:
   // 21.4 against 18.9 us, 2048^2: 8.0 against 14.0)
   const bool long_columns = sizeof(T) == 4 && mode == 0 && L.seglen == kSeg && L.n > 2048;
-  if (L.n <= 32 * kFusedSegs && !long_columns &&
-      (mode == 0 || sizeof(T) == 4 || ea >= 1e-100)) {
-    // every constant from the root as rounded to T, and kappa from the gain
-    // the rounded constants give a uniform field, so that it comes back
-    // unscaled: a rounding of kappa itself would add up over the steps
+  if (L.n <= 32 * kFusedSegs && a <= kFusedMaxAlpha && !long_columns) {
+    // every constant from the root as rounded to T, and kappa from the gain the
+    // constants give a uniform field, so that it comes back unscaled: a
+    // rounding of kappa itself would add up over the steps
     LineCoef<T> kf = k;
     const double rt = (double)(T)r;
-    double gain = 1.0;
-    if (mode != 0) {
-      if (sizeof(T) == 8) {
-        kf.w0 = (T)((1.0 - 2.0 * ea) / ea);
-        gain = (double)kf.w0 + 2.0;
-      } else {
-        gain = (double)kf.w0 + 2.0 * (double)kf.w1;
-      }
-    }
+    const bool divided = sizeof(T) == 8 && mode != 0 && ea >= 1e-3 && ea <= kMaxDivided;
+    if (divided) kf.w0 = (T)((1.0 - 2.0 * ea) / ea);
+    const double gain = divided ? (double)kf.w0 + 2.0 : 1.0;
     kf.kappa = (T)((1.0 - rt) * (1.0 - rt) / gain);
     pw = 1.0;
     for (int i = 0; i <= 32; ++i, pw *= rt) kf.rpow[i] = (T)pw;
+    if constexpr (sizeof(T) == 8) {
+      if (divided)
+        return mode == 1 ? launch_fused_axis<T, 3>(L, kf, rt, in, out, st)
+                         : launch_fused_axis<T, 4>(L, kf, rt, in, out, st);
+    }
     switch (mode) {
       case 0: return launch_fused_axis<T, 0>(L, kf, rt, in, out, st);
       case 1: return launch_fused_axis<T, 1>(L, kf, rt, in, out, st);
