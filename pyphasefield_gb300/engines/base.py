@@ -592,7 +592,8 @@ class GB300Engine:
         if ud.get("use_graph", True) and nsteps >= span:
             g = self._ppf_graph(tuple(self._ppf_passes(span, even=True)))
             if self.USES_STEP:
-                L.call("ppf_counter_set_u64", ptr(self._ppf_stepctr), C.c_uint64(step), sp)
+                with torch.cuda.stream(s):  # a launch: the stream's device has to be current
+                    L.call("ppf_counter_set_u64", ptr(self._ppf_stepctr), C.c_uint64(step), sp)
             while nsteps >= span:
                 self._ppf_check_status(False)
                 with nvtx_range(f"ppf.graph {span} steps from {step}"):

@@ -1,0 +1,59 @@
+"""The engines' host side with the library calls recorded (no GPU)."""
+import contextlib
+
+import pytest
+import torch
+
+from pyphasefield_gb300.engines import base
+
+
+class Stream:
+    cuda_stream = 7
+
+
+class Engine(base.GB300Engine):
+    """An engine of a few fields, without device buffers."""
+
+    def __init__(self, **user_data):
+        self.user_data = dict(user_data)
+        self._ppf_stream = Stream()
+        self._ppf_stepctr = torch.zeros(1, dtype=torch.int64)
+        self._ppf_cur = 0
+
+    def _ppf_graph(self, depths):
+        return "graph"
+
+    def _ppf_check_status(self, block, where=""):
+        pass
+
+    def _ppf_mark(self):
+        pass
+
+
+@pytest.fixture
+def log(monkeypatch):
+    """Library calls and the streams they were issued under."""
+    out = []
+    active = []
+
+    @contextlib.contextmanager
+    def stream(s):
+        active.append(s)
+        yield
+        active.pop()
+
+    monkeypatch.setattr(base.torch.cuda, "stream", stream)
+    monkeypatch.setattr(base.L, "call", lambda name, *a: out.append((name, list(active))))
+    return out
+
+
+def test_counter_is_set_with_the_engines_device_current(log):
+    """A launch into a stream of another device than the current one is
+    refused; torch.cuda.stream makes the stream's device current."""
+    class Noisy(Engine):
+        USES_STEP = True
+
+    e = Noisy(graph_chunk=4, check_status=False)
+    e._ppf_advance(8, 3)
+    assert [n for n, _ in log] == ["ppf_counter_set_u64", "ppf_graph_launch", "ppf_graph_launch"]
+    assert log[0][1] == [e._ppf_stream]
