@@ -419,9 +419,9 @@ int32_t ppf_ncgpu_temperature_advance_f64(const PpfGrid* g, double* temperature,
 
 /* npasses passes of one model, from the field buffers a into b, back into a and
  * so on: pass i advances depths[i] steps (1 for every model but the 2-D explicit
- * Diffusion and Allen-Cahn steps) through the model's step entry point, with
- * its argument checks; the first error ends the run. The result is in a when
- * npasses is even, else in b.
+ * Diffusion and Allen-Cahn steps; more is refused before any launch) through the
+ * model's step entry point, with its argument checks; the first error ends the
+ * run. The result is in a when npasses is even, else in b.
  *   PPF_RUN_CAHN_HILLIARD   step k adds its mass to mass[k] (mass may be NULL)
  *   PPF_RUN_WARREN1995, PPF_RUN_NCGPU   step k draws the noise of step + k
  *     (+ *step_base)

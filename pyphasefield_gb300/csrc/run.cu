@@ -99,8 +99,13 @@ int32_t ppf_run(const PpfRun* run, const int32_t* depths, int32_t npasses, int32
   clear_error();
   if (!run || !run->params || !run->grid) return fail(PPF_ERR_INVALID, "run is NULL");
   if (npasses < 0 || (npasses > 0 && !depths)) return fail(PPF_ERR_INVALID, "bad pass list");
-  for (int32_t i = 0; i < npasses; ++i)
+  const bool deep = run->model == PPF_RUN_DIFFUSION || run->model == PPF_RUN_ALLEN_CAHN;
+  for (int32_t i = 0; i < npasses; ++i) {
     if (depths[i] < 1) return fail(PPF_ERR_INVALID, "depth=%d < 1", depths[i]);
+    if (depths[i] > 1 && !deep)
+      return fail(PPF_ERR_UNSUPPORTED, "run.model=%d advances one step per pass (depth=%d)",
+                  run->model, depths[i]);
+  }
   if (run->elem_bytes == 4) return run_passes<float>(run, depths, npasses, iterations, stream);
   if (run->elem_bytes == 8) return run_passes<double>(run, depths, npasses, iterations, stream);
   return fail(PPF_ERR_INVALID, "elem_bytes must be 4 or 8");
