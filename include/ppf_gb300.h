@@ -459,6 +459,10 @@ typedef struct PpfRun {
 } PpfRun;
 int32_t ppf_run(const PpfRun* run, const int32_t* depths, int32_t npasses, int32_t* iterations,
                 void* stream);
+/* Passes the calling thread's last ppf_run issued before it returned (npasses, or
+ * fewer after an error: the result so far is in a when their number is even, else
+ * in b). Keeps the error message. */
+int32_t ppf_run_passes(int32_t* passes);
 
 /* One launch that ORs PPF_STATUS_NONFINITE into *status if any of the nfields
  * fields holds NaN or Inf, moves the library's status bits into *status as

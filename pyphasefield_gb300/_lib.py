@@ -206,6 +206,7 @@ SIGNATURES: dict[str, list] = {
     "ppf_periodic_solve_f64": [PG, C.c_double, C.c_double, C.c_double, P, P, P,
                                C.POINTER(I32), P],
     "ppf_run": [C.POINTER(PpfRun), C.POINTER(I32), I32, C.POINTER(I32), P],
+    "ppf_run_passes": [C.POINTER(I32)],
     "ppf_watch_f32": [P, I32, PG, P, P, P, P],
     "ppf_watch_f64": [P, I32, PG, P, P, P, P],
     "ppf_counter_set_u64": [P, U64, P],

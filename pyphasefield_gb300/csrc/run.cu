@@ -68,6 +68,9 @@ int32_t one_pass(const PpfRun* r, T* const* in, T* const* out, const PpfTiling* 
   return fail(PPF_ERR_INVALID, "run.model=%d unknown", r->model);
 }
 
+// passes the thread's last run issued without an error
+thread_local int32_t g_passes = 0;
+
 template <typename T>
 int32_t run_passes(const PpfRun* r, const int32_t* depths, int32_t npasses, int32_t* iterations,
                    void* stream) {
@@ -81,6 +84,7 @@ int32_t run_passes(const PpfRun* r, const int32_t* depths, int32_t npasses, int3
     T* const* out = (T* const*)(i & 1 ? r->a : r->b);
     const int32_t rc = one_pass<T>(r, in, out, &t, done, step, iterations, stream);
     if (rc) return rc;
+    g_passes = i + 1;
     done += depths[i];
     step += (uint64_t)depths[i];
   }
@@ -97,6 +101,7 @@ extern "C" {
 int32_t ppf_run(const PpfRun* run, const int32_t* depths, int32_t npasses, int32_t* iterations,
                 void* stream) {
   clear_error();
+  g_passes = 0;
   if (!run || !run->params || !run->grid) return fail(PPF_ERR_INVALID, "run is NULL");
   if (npasses < 0 || (npasses > 0 && !depths)) return fail(PPF_ERR_INVALID, "bad pass list");
   const bool deep = run->model == PPF_RUN_DIFFUSION || run->model == PPF_RUN_ALLEN_CAHN;
@@ -109,6 +114,12 @@ int32_t ppf_run(const PpfRun* run, const int32_t* depths, int32_t npasses, int32
   if (run->elem_bytes == 4) return run_passes<float>(run, depths, npasses, iterations, stream);
   if (run->elem_bytes == 8) return run_passes<double>(run, depths, npasses, iterations, stream);
   return fail(PPF_ERR_INVALID, "elem_bytes must be 4 or 8");
+}
+
+int32_t ppf_run_passes(int32_t* passes) {
+  if (!passes) return fail(PPF_ERR_INVALID, "passes is NULL");
+  *passes = g_passes;
+  return PPF_OK;
 }
 
 }  // extern "C"

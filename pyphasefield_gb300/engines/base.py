@@ -514,7 +514,14 @@ class GB300Engine:
         run.step_base = step_base.data_ptr() if step_base is not None else None
         it = C.c_int32()
         n = len(depths)
-        L.call("ppf_run", C.byref(run), (C.c_int32 * n)(*depths), n, C.byref(it), sp)
+        try:
+            L.call("ppf_run", C.byref(run), (C.c_int32 * n)(*depths), n, C.byref(it), sp)
+        except L.PpfError:
+            # the passes before the refused one ran
+            done = C.c_int32()
+            L.call("ppf_run_passes", C.byref(done))
+            self._ppf_cur ^= done.value & 1
+            raise
         self._ppf_iterations = it.value
         self._ppf_cur ^= n & 1
 

@@ -1,9 +1,11 @@
 """The engines' host side with the library calls recorded (no GPU)."""
 import contextlib
+import types
 
 import pytest
 import torch
 
+from pyphasefield_gb300 import _lib as L
 from pyphasefield_gb300.engines import base
 
 
@@ -57,3 +59,25 @@ def test_counter_is_set_with_the_engines_device_current(log):
     e._ppf_advance(8, 3)
     assert [n for n, _ in log] == ["ppf_counter_set_u64", "ppf_graph_launch", "ppf_graph_launch"]
     assert log[0][1] == [e._ppf_stream]
+
+
+@pytest.mark.parametrize("done", [0, 1, 2, 3])
+def test_a_run_that_stops_leaves_its_last_complete_state_current(monkeypatch, done):
+    class Native(Engine):
+        def _ppf_run(self):
+            return L.PpfRun()
+
+    def call(name, *args):
+        if name == "ppf_run":
+            raise L.PpfError(L.PPF_ERR_INVALID, name, "refused")
+        assert name == "ppf_run_passes"
+        args[0]._obj.value = done
+
+    e = Native()
+    e._ppf_bufs = [[torch.zeros(4)], [torch.zeros(4)]]
+    e._ppf_grid = types.SimpleNamespace(grid=L.PpfGrid())
+    e._ppf_bc = L.PpfBoundary()
+    monkeypatch.setattr(base.L, "call", call)
+    with pytest.raises(L.PpfError, match="refused"):
+        e._ppf_launch_passes([1] * 5, 0, None)
+    assert e._ppf_cur == done % 2
