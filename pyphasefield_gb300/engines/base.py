@@ -123,14 +123,30 @@ class GB300Engine:
         """Launch one pass advancing `depth` steps from buffers src to dst."""
         raise NotImplementedError
 
-    #: whether a step reads the step counter (noise drawn per step)
-    USES_STEP = False
+    #: whether a step reads the step counter (noise drawn per step). An engine
+    #: that states False gets step_base = None, also in captured runs.
+    USES_STEP = True
 
     def _ppf_run(self):
         """PpfRun of the engine's steps (model, params, tiling and the model's
         own buffers; the fields and the step are filled in), or None for an
-        engine whose steps are launched one by one."""
+        engine whose steps are launched one by one. A run issues the same
+        passes as _ppf_step does."""
         return None
+
+    def __init_subclass__(cls, **kwargs):
+        """A class with a _ppf_step of its own is stepped through it: what it
+        inherits for another step (_ppf_run, _ppf_auto_depth, USES_STEP =
+        False) does not hold for it unless it states it again."""
+        super().__init_subclass__(**kwargs)
+
+        def owner(name):
+            return next(i for i, c in enumerate(cls.__mro__) if name in c.__dict__)
+
+        step = owner("_ppf_step")
+        for name in ("_ppf_run", "_ppf_auto_depth", "USES_STEP"):
+            if step < owner(name):
+                setattr(cls, name, GB300Engine.__dict__[name])
 
     def _ppf_max_depth(self) -> int:
         return 1

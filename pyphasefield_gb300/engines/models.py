@@ -162,6 +162,7 @@ class _DiffusionMixin(GB300Engine):
     solves (0: the library default)."""
 
     NFIELDS = 1
+    USES_STEP = False
 
     def __init__(self, **kwargs):
         super().__init__(**kwargs)
@@ -262,6 +263,7 @@ class _CahnAllenMixin(_ImplicitPhase, GB300Engine):
     "solver" / "adi" / "gmres"."""
 
     NFIELDS = 1
+    USES_STEP = False
     PHASE_MODEL = L.PPF_MODEL_ALLEN_CAHN
 
     def __init__(self, **kwargs):
@@ -336,6 +338,7 @@ class _CahnHilliardMixin(_ImplicitPhase, GB300Engine):
     c itself and track no mass."""
 
     NFIELDS = 1
+    USES_STEP = False
     PHASE_MODEL = L.PPF_MODEL_CAHN_HILLIARD
 
     def __init__(self, **kwargs):

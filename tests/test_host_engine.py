@@ -81,3 +81,40 @@ def test_a_run_that_stops_leaves_its_last_complete_state_current(monkeypatch, do
     with pytest.raises(L.PpfError, match="refused"):
         e._ppf_launch_passes([1] * 5, 0, None)
     assert e._ppf_cur == done % 2
+
+
+def test_a_step_of_its_own_is_not_bypassed():
+    """A subclass that overrides _ppf_step alone is stepped one step a pass,
+    through it, and is given the step counter."""
+    from pyphasefield_gb300 import DiffusionGB300, Warren1995GB300
+
+    class Sourced(DiffusionGB300):
+        def _ppf_step(self, *a):
+            pass
+
+    class Further(Sourced):
+        pass
+
+    class Mixed(type("Step", (), {"_ppf_step": lambda self, *a: None}), DiffusionGB300):
+        pass
+
+    class Stated(DiffusionGB300):
+        USES_STEP = False
+        _ppf_auto_depth = DiffusionGB300._ppf_auto_depth
+
+        def _ppf_step(self, *a):
+            pass
+
+    for cls in (Sourced, Further, Mixed):
+        e = cls.__new__(cls)
+        e._ppf_grid = types.SimpleNamespace(kshape=(64, 64))
+        assert e._ppf_run() is None and e._ppf_auto_depth() == 1 and e.USES_STEP
+    assert not Stated.USES_STEP and Stated._ppf_auto_depth is DiffusionGB300._ppf_auto_depth
+    assert not DiffusionGB300.USES_STEP and Warren1995GB300.USES_STEP
+
+    class Renamed(DiffusionGB300):
+        """No step of its own: everything is inherited."""
+
+    for cls in (Renamed, Warren1995GB300):
+        assert cls._ppf_run is not base.GB300Engine._ppf_run
+    assert Renamed._ppf_auto_depth is DiffusionGB300._ppf_auto_depth and not Renamed.USES_STEP
