@@ -116,18 +116,22 @@ class _ImplicitPhase:
 
 
 def _stencil_candidates(sim) -> list:
-    """Diffusion / Allen-Cahn launch shapes: temporal depth x tile (2-D),
-    tile and planes per CTA along z (3-D)."""
+    """Diffusion / Allen-Cahn launch shapes, the engine's own choice first:
+    temporal depth x tile (2-D), tile and planes per warp or CTA along z (3-D,
+    0: the kernel's choice)."""
     if len(sim._ppf_grid.kshape) == 2:
-        # depth 1: the warp-strip kernel; depth > 1 without a tile or with
-        # (0, rows): the marching kernel (segments of `rows`); with a tile:
-        # the shared-memory tile kernel
+        # depth 1 without a tile: the engine's own depth (float: eight steps a
+        # pass in register blocks; double: the warp-strip kernel); depth > 1
+        # without a tile: register blocks in float, the marching kernel in
+        # double; with (0, rows): the marching kernel (segments of `rows`);
+        # with a tile: the shared-memory tile kernel
         return [{"temporal_depth": d, "tile": None} for d in (1, 2, 4, 8)] + \
             [{"temporal_depth": d, "tile": (0, 32 * d * f)} for d in (2, 4, 8) for f in (1, 4)] + \
             [{"temporal_depth": d, "tile": t} for d in (1, 2, 4, 8)
              for t in ((128, 32), (64, 32), (256, 16), (128, 16))]
-    return [{"tile": (32, 32), "zchunk": z} for z in (8, 12, 16, 24)] + \
-        [{"tile": t} for t in ((64, 16), (32, 16), (128, 8))]
+    # without a tile: warps that march along z; with one: shared-memory tiles
+    return [{"tile": None, "zchunk": z} for z in (0, 2, 4, 8, 12, 16, 24)] + \
+        [{"tile": t, "zchunk": 0} for t in ((64, 16), (32, 16), (128, 8))]
 
 
 def _stencil_auto_depth(sim) -> int:

@@ -118,3 +118,18 @@ def test_a_step_of_its_own_is_not_bypassed():
     for cls in (Renamed, Warren1995GB300):
         assert cls._ppf_run is not base.GB300Engine._ppf_run
     assert Renamed._ppf_auto_depth is DiffusionGB300._ppf_auto_depth and not Renamed.USES_STEP
+
+
+@pytest.mark.parametrize("shape", [(64, 64), (24, 24, 24)])
+@pytest.mark.parametrize("name", ["DiffusionGB300", "CahnAllenGB300"])
+def test_the_engines_own_choice_is_a_tuning_candidate(name, shape):
+    import pyphasefield_gb300 as P
+    cls = getattr(P, name)
+    e = cls(dimensions=list(shape), dx=1.0, dt=0.1, boundary_conditions="PERIODIC")
+    e._ppf_grid = types.SimpleNamespace(kshape=shape)
+    default = {"temporal_depth": e.user_data["temporal_depth"], "tile": e.user_data["tile"],
+               "zchunk": 0}
+    cands = e._ppf_tune_candidates()
+    assert all(default[k] == v for k, v in cands[0].items())
+    # every candidate sets the same keys: none is timed with another's left-overs
+    assert len({frozenset(c) for c in cands}) == 1
