@@ -308,7 +308,10 @@ class GB300Engine:
 
         def measure(cand):
             self.user_data.update(cand)
+            # the passes a long run consists of
             depth = max(1, min(int(self.user_data.get("temporal_depth", 1)), self._ppf_max_depth()))
+            if depth == 1:
+                depth = self._ppf_auto_depth()
             flip = [0]
 
             def run():

@@ -133,3 +133,30 @@ def test_the_engines_own_choice_is_a_tuning_candidate(name, shape):
     assert all(default[k] == v for k, v in cands[0].items())
     # every candidate sets the same keys: none is timed with another's left-overs
     assert len({frozenset(c) for c in cands}) == 1
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_candidates_are_timed_at_the_depth_they_run_at(monkeypatch, precision):
+    import pyphasefield_gb300 as P
+    from pyphasefield_gb300 import autotune
+    e = P.DiffusionGB300(dimensions=[64, 64], dx=1.0, dt=0.1, boundary_conditions="PERIODIC",
+                         user_data={"precision": precision})
+    e._ppf_grid = types.SimpleNamespace(kshape=(64, 64))
+    e._ppf_bc, e._ppf_stream, e._ppf_cur = L.PpfBoundary(), Stream(), 0
+    e._ppf_bufs = [[torch.zeros(4)], [torch.zeros(4)]]
+    timed = []
+    e._ppf_step = lambda src, dst, depth, *a: timed.append(depth)
+    monkeypatch.setattr(base.torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(autotune, "time_candidate", lambda run, s: [run(), 1.0][1])
+
+    def pick(key, cands, measure):
+        for c in cands:
+            seconds = measure(c)
+            e.user_data.update(c)
+            depth = max(e._ppf_passes(64))
+            assert timed.pop() == depth and seconds == 1.0 / depth, c
+        return cands[0]
+
+    monkeypatch.setattr(autotune, "pick", pick)
+    e._ppf_autotune()
+    assert not timed
