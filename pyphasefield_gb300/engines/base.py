@@ -289,6 +289,10 @@ class GB300Engine:
         """Launch shapes the autotuner may try (user_data updates)."""
         return []
 
+    #: part of the autotuner's cache key, changed with the kernels behind the
+    #: candidates: a choice cached for others is made anew
+    TUNE_KERNELS = ""
+
     def _ppf_autotune(self):
         """Pick tile / temporal depth by timing candidates on scratch copies
         of the current fields (user_data["autotune"] = True); the choice is
@@ -299,7 +303,7 @@ class GB300Engine:
         if len(cands) < 2:
             return
         key = autotune.make_key(type(self).__name__, self._ppf_grid.kshape, self._ppf_dtype,
-                                str(len(self.dimensions)))
+                                str(len(self.dimensions)) + self.TUNE_KERNELS)
         s = self._ppf_stream
         sp = C.c_void_p(s.cuda_stream)
         with torch.cuda.stream(s):

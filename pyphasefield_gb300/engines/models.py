@@ -167,6 +167,7 @@ class _DiffusionMixin(GB300Engine):
 
     NFIELDS = 1
     USES_STEP = False
+    TUNE_KERNELS = "|register blocks, z marches"
 
     def __init__(self, **kwargs):
         super().__init__(**kwargs)
@@ -268,6 +269,7 @@ class _CahnAllenMixin(_ImplicitPhase, GB300Engine):
 
     NFIELDS = 1
     USES_STEP = False
+    TUNE_KERNELS = "|register blocks, z marches"
     PHASE_MODEL = L.PPF_MODEL_ALLEN_CAHN
 
     def __init__(self, **kwargs):

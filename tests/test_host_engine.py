@@ -160,3 +160,20 @@ def test_candidates_are_timed_at_the_depth_they_run_at(monkeypatch, precision):
     monkeypatch.setattr(autotune, "pick", pick)
     e._ppf_autotune()
     assert not timed
+
+
+def test_choices_cached_for_other_kernels_are_not_taken(monkeypatch):
+    """The Diffusion and Allen-Cahn kernels changed; the others' choices stay."""
+    import pyphasefield_gb300 as P
+    from pyphasefield_gb300 import autotune
+    keys = {}
+    monkeypatch.setattr(autotune, "pick", lambda key, cands, m: keys.update({name: key}) or cands[0])
+    monkeypatch.setattr(base.torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    for name in ("DiffusionGB300", "CahnAllenGB300", "Warren1995GB300"):
+        e = getattr(P, name)(dimensions=[64, 64], dx=1.0, dt=0.1, boundary_conditions="PERIODIC")
+        e._ppf_grid = types.SimpleNamespace(kshape=(64, 64))
+        e._ppf_stream, e._ppf_cur = Stream(), 0
+        e._ppf_bufs = [[torch.zeros(4)], [torch.zeros(4)]]
+        e._ppf_autotune()
+        old = autotune.make_key(name, (64, 64), torch.float32, "2")
+        assert (keys[name] == old) == (name == "Warren1995GB300")
