@@ -370,6 +370,10 @@ __global__ void __launch_bounds__(kThreads)
 // 79, 512^3 221 -> 170; float64 200^3 309 -> 260.
 constexpr int kLWarps = 4;
 
+// Row bands a launch holds (gridDim.y); a grid with more takes several launches,
+// each from its first row y_first on.
+constexpr int kMaxBands = 65535;
+
 template <typename T, int R, int LX>
 struct Lean7Slot {
   static constexpr int V = Vec16<T>::n;
@@ -380,7 +384,7 @@ struct Lean7Slot {
 template <typename T, typename Op, int R, int D, int LX>
 __global__ void __launch_bounds__(32 * kLWarps)
     lean7_kernel(Op op, const __grid_constant__ Geo g, const __grid_constant__ Bc<T> bc,
-                 const T* __restrict__ in, T* __restrict__ out, int zc) {
+                 const T* __restrict__ in, T* __restrict__ out, int zc, int y_first) {
   constexpr int V = Vec16<T>::n;
   constexpr int G = 32 / LX;  // groups of lanes, each with R rows of its own
   constexpr int RS = 32 * V;  // elements of a row of the slot
@@ -391,7 +395,7 @@ __global__ void __launch_bounds__(32 * kLWarps)
   const int group = G > 1 ? lane / LX : 0;
   T* ring = reinterpret_cast<T*>(smem_raw) + threadIdx.y * D * Slot::elems;
   const int x0 = blockIdx.x * (LX * V);
-  const int yw = (blockIdx.y * kLWarps + threadIdx.y) * (R * G);
+  const int yw = y_first + (blockIdx.y * kLWarps + threadIdx.y) * (R * G);
   const int y0 = yw + group * R;
   const int z0 = blockIdx.z * zc;
   const int nz = g.n[0], ny = g.n[1], nx = g.n[2];
@@ -862,20 +866,22 @@ __device__ __forceinline__ Quad ch_flux4(const ChCoef<float>& k, Quad mn, Quad m
 }
 
 // FLAT: a single plane, its own neighbour along z (no march, no z fluxes). Off holds
-// an element's offset within a plane.
+// an element's offset within a plane; 64 bits are for grids beyond 2^31 elements a
+// plane or kMaxBands row bands (only there y_first is not 0: it is left out of the
+// other form, whose registers are all taken, 1 % of 256^3).
 template <bool QUANT, bool FLAT, typename Off>
 __global__ void __launch_bounds__(32 * kHWarps, 3)
     ch_march_kernel(const __grid_constant__ ChCoef<float> k, const __grid_constant__ Geo g,
                     const __grid_constant__ Bc<float> bc, const float* __restrict__ in,
                     float* __restrict__ out, double* __restrict__ mass, int* __restrict__ status,
-                    int zc) {
+                    int zc, int y_first) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x;
   float* ring = reinterpret_cast<float*>(smem_raw) + threadIdx.y * kHWarpElems<FLAT>;
   float* smu = ring + (FLAT ? 1 : kHD) * kHSlot;
   const int nz = g.n[0], ny = g.n[1], nx = g.n[2];
   const int x0 = blockIdx.x * kHRow;
-  const int y0 = (blockIdx.y * kHWarps + threadIdx.y) * kHR;
+  const int y0 = (sizeof(Off) == 8 ? y_first : 0) + (blockIdx.y * kHWarps + threadIdx.y) * kHR;
   const int z0 = blockIdx.z * zc;
   pdl_wait();
   pdl_launch_next();
@@ -1134,10 +1140,11 @@ int zchunk_of(const PpfTiling* t, const Geo& g) {
 // warp advances one plane after the other, so chunks are as short as it takes to
 // have a dozen warps per SM (float, us per step with 2 / 4 / 8 planes: 64^3 3.8 /
 // 5.7 / 9.4, 128^3 5.2 / 5.7 / 7.9, 256^3 30 / 29 / 26, 512^3 196 / 178 / 170,
-// 16 planes 176).
+// 16 planes 176). More where gridDim.z would not hold the chunks.
 int lean_zchunk(long warps, int nz) {
   int zc = 8;
   while (zc > 2 && warps * ((nz + zc - 1) / zc) < 2048) zc /= 2;
+  if (zc < (nz + 65534) / 65535) zc = (nz + 65534) / 65535;
   return zc < nz ? zc : nz;
 }
 
@@ -1206,11 +1213,14 @@ int32_t launch_lean7(Op op, const Geo& g, const Bc<T>& bc, const T* in, T* out, 
   constexpr int R = kLeanRows<T>, D = 4, WW = LX * Vec16<T>::n, rows = R * (32 / LX) * kLWarps;
   const int strips = (g.n[2] + WW - 1) / WW, bands = (g.n[1] + rows - 1) / rows;
   if (!zc) zc = lean_zchunk((long)strips * bands * kLWarps, g.n[0]);
-  const dim3 gd(strips, bands, (g.n[0] + zc - 1) / zc);
   auto kern = lean7_kernel<T, Op, R, D, LX>;
   const size_t smem = (size_t)kLWarps * D * Lean7Slot<T, R, LX>::elems * sizeof(T);
   PPF_TRY_CUDA(allow_smem(kern, smem));
-  PPF_TRY_CUDA(launch(kern, gd, dim3(32, kLWarps), smem, s, pdl, op, g, bc, in, out, zc));
+  for (int band = 0; band < bands; band += kMaxBands) {
+    const dim3 gd(strips, min(bands - band, kMaxBands), (g.n[0] + zc - 1) / zc);
+    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kLWarps), smem, s, pdl, op, g, bc, in, out, zc,
+                        band * rows));
+  }
   return PPF_OK;
 }
 
@@ -1280,17 +1290,20 @@ int32_t run_ch_march(const ChCoef<float>& k, const Geo& g, const Bc<float>& bc, 
     zc = zc < 2 ? 2 : zc > 32 ? 32 : zc;
   }
   zc = zc < g.n[0] ? zc : g.n[0];
-  const dim3 gd(strips, bands, (g.n[0] + zc - 1) / zc);
   const size_t smem = (size_t)kHWarps * (flat ? kHWarpElems<true> : kHWarpElems<false>) * sizeof(float);
   auto pick = [&](auto off) {
     using Off = decltype(off);
     return quant ? (flat ? ch_march_kernel<true, true, Off> : ch_march_kernel<true, false, Off>)
                  : (flat ? ch_march_kernel<false, true, Off> : ch_march_kernel<false, false, Off>);
   };
-  auto kern = g.plane < (1LL << 31) ? pick(uint32_t{}) : pick(int64_t{});
+  const bool small = g.plane < (1LL << 31) && bands <= kMaxBands;
+  auto kern = small ? pick(uint32_t{}) : pick(int64_t{});
   PPF_TRY_CUDA(allow_smem(kern, smem));
-  PPF_TRY_CUDA(launch(kern, gd, dim3(32, kHWarps), smem, s, pdl, k, g, bc, in, out, mass, status,
-                      zc));
+  for (int band = 0; band < bands; band += kMaxBands) {
+    const dim3 gd(strips, min(bands - band, kMaxBands), (g.n[0] + zc - 1) / zc);
+    PPF_TRY_CUDA(launch(kern, gd, dim3(32, kHWarps), smem, s, pdl, k, g, bc, in, out, mass, status,
+                        zc, band * kHR * kHWarps));
+  }
   return PPF_OK;
 }
 
