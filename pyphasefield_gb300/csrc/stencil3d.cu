@@ -866,9 +866,10 @@ __device__ __forceinline__ Quad ch_flux4(const ChCoef<float>& k, Quad mn, Quad m
 }
 
 // FLAT: a single plane, its own neighbour along z (no march, no z fluxes). Off holds
-// an element's offset within a plane; 64 bits are for grids beyond 2^31 elements a
-// plane or kMaxBands row bands (only there y_first is not 0: it is left out of the
-// other form, whose registers are all taken, 1 % of 256^3).
+// an element's offset within a plane; 64 bits make the general form, for grids beyond
+// 2^31 elements a plane or kMaxBands row bands and for outputs off a 16-byte boundary
+// (y_first is 0 and out is aligned in the other, whose registers are all taken: the
+// row's start alone cost 1 % of 256^3).
 template <bool QUANT, bool FLAT, typename Off>
 __global__ void __launch_bounds__(32 * kHWarps, 3)
     ch_march_kernel(const __grid_constant__ ChCoef<float> k, const __grid_constant__ Geo g,
@@ -1000,7 +1001,8 @@ __global__ void __launch_bounds__(32 * kHWarps, 3)
     for (int j = 0; j < kHR; ++j) fup[j] = ch_flux4<QUANT>(k, mu[j + 1], ml[j + 1]);
     s0 = 2;
   }
-  const bool full = x0 + kHRow <= nx && y0 + kHR <= ny;
+  const bool full = x0 + kHRow <= nx && y0 + kHR <= ny &&
+                    (sizeof(Off) == 4 || ((uintptr_t)out & 15) == 0);
   float vmax = 0.f;
   F2 vsum = sp(0.f);
   long long acc_q = 0;
@@ -1239,16 +1241,14 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
   size_t smem;
   int* st = status_ptr();
   if (!st) return fail(PPF_ERR_CUDA, "status word unavailable");
-  const bool lean = (!tiling || ((tiling->tile_x == 0 || tiling->tile_x == 32) &&
-                                 (tiling->tile_y == 0 || tiling->tile_y == 32))) &&
-                    g.plane < (1LL << 31);
-  if (lean) {
+  const bool own = !tiling || ((tiling->tile_x == 0 || tiling->tile_x == 32) &&
+                               (tiling->tile_y == 0 || tiling->tile_y == 32));
+  if (own && g.plane < (1LL << 31) && (uintptr_t)out % 16 == 0) {
     PpfTiling lt{};
     lt.depth = tiling ? tiling->depth : 0;
     lt.zchunk = tiling ? tiling->zchunk : 0;
     if ((rc = plan3d<T>(&lt, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
-    if (((uintptr_t)in) % 16 || ((uintptr_t)out) % 16)
-      return fail(PPF_ERR_INVALID, "3-D steps need 16-byte aligned rows");
+    if ((uintptr_t)in % 16) return fail(PPF_ERR_INVALID, "field base not 16-byte aligned");
     const cudaStream_t st7 = (cudaStream_t)stream;
     const bool pdl = tiling && tiling->pdl;
     const int zc = tiling && tiling->zchunk > 0 ? zchunk_of(tiling, g) : 0;
@@ -1258,7 +1258,11 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
       default: return launch_lean7<T, Op, 32>(op, g, bc, in, out, zc, pdl, st7);
     }
   }
-  if ((rc = plan3d<T>(tiling, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
+  // tiles: asked for, or outputs off a 16-byte boundary and planes beyond 32-bit offsets
+  PpfTiling tt{};
+  if (tiling) tt = *tiling;
+  if (own) tt.tile_x = tt.tile_y = 32;
+  if ((rc = plan3d<T>(&tt, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
   m.ZC = zchunk_of(tiling, g);
   CUtensorMap map;
   if ((rc = plane_map<T>(&map, in, g, m))) return rc;
@@ -1296,7 +1300,7 @@ int32_t run_ch_march(const ChCoef<float>& k, const Geo& g, const Bc<float>& bc, 
     return quant ? (flat ? ch_march_kernel<true, true, Off> : ch_march_kernel<true, false, Off>)
                  : (flat ? ch_march_kernel<false, true, Off> : ch_march_kernel<false, false, Off>);
   };
-  const bool small = g.plane < (1LL << 31) && bands <= kMaxBands;
+  const bool small = g.plane < (1LL << 31) && bands <= kMaxBands && (uintptr_t)out % 16 == 0;
   auto kern = small ? pick(uint32_t{}) : pick(int64_t{});
   PPF_TRY_CUDA(allow_smem(kern, smem));
   for (int band = 0; band < bands; band += kMaxBands) {
@@ -1361,8 +1365,7 @@ int32_t cahn_hilliard(const PpfCahnHilliardParams* p, const PpfGrid* grid_in,
   k.centered = p->centered;
   const bool pdl = tiling && tiling->pdl;
   if constexpr (sizeof(T) == 4) {
-    if (((uintptr_t)in) % 16 || ((uintptr_t)out) % 16)
-      return fail(PPF_ERR_INVALID, "3-D steps need 16-byte aligned rows");
+    if ((uintptr_t)in % 16) return fail(PPF_ERR_INVALID, "field base not 16-byte aligned");
     return run_ch_march(k, g, bc, in, out, mass, (int*)status, tiling, quant, pdl,
                         (cudaStream_t)stream);
   } else {
