@@ -1246,7 +1246,6 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
   if (own && g.plane < (1LL << 31) && (uintptr_t)out % 16 == 0) {
     PpfTiling lt{};
     lt.depth = tiling ? tiling->depth : 0;
-    lt.zchunk = tiling ? tiling->zchunk : 0;
     if ((rc = plan3d<T>(&lt, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
     if ((uintptr_t)in % 16) return fail(PPF_ERR_INVALID, "field base not 16-byte aligned");
     const cudaStream_t st7 = (cudaStream_t)stream;
@@ -1261,7 +1260,7 @@ int32_t run_march7(Op op, double dx, const PpfGrid* grid, const PpfBoundary* b, 
   // tiles: asked for, or outputs off a 16-byte boundary and planes beyond 32-bit offsets
   PpfTiling tt{};
   if (tiling) tt = *tiling;
-  if (own) tt.tile_x = tt.tile_y = 32;
+  if (own) tt.tile_x = tt.tile_y = 32, tt.zchunk = 0;  // (its sign is not looked at here)
   if ((rc = plan3d<T>(&tt, g, 1, kNS7, 0, &m, &slot_elems, &smem))) return rc;
   m.ZC = zchunk_of(tiling, g);
   CUtensorMap map;
@@ -1344,7 +1343,6 @@ int32_t cahn_hilliard(const PpfCahnHilliardParams* p, const PpfGrid* grid_in,
   ct.depth = tiling ? tiling->depth : 0;
   ct.tile_x = kCTX;
   ct.tile_y = kCTY;
-  ct.zchunk = tiling ? tiling->zchunk : 0;
   if ((rc = plan3d<T>(&ct, g, 2, kNSC, kMuSlots, &m, &slot_elems, &smem))) return rc;
   ChCoef<T> k;
   k.kap = (T)(p->epsilon * p->epsilon / (p->dx * p->dx));
