@@ -827,6 +827,36 @@ __device__ __forceinline__ void carry_scan(int mc, const CarryCoef<T>& cc, int l
   if (lane == 0) Bu[mc] = x0;
 }
 
+// The same by one thread, for lines of few segments: a warp would scan 32 / nseg of
+// them one after the other, most of its lanes idle. us per solve with the scan /
+// with this (three launches): 30 x 16 double 20.4 / 4.4 (8.7), 1000 x 16 float 7.0 / 2.4
+// (4.9), 20 x 100000 columns in double 153 / 33 (125).
+constexpr int kSerialSegs = 8;
+template <typename T>
+__device__ __forceinline__ void carry_serial(int mc, const CarryCoef<T>& cc, T* F, T* Bu) {
+  T y = T(0);
+  for (int s = 0; s < mc; ++s) y = fma(cc.R, y, F[s]);
+  y = (F[mc] + cc.Rl * y) * cc.inv_close;  // y of the line's last cell
+  for (int s = 0; s < mc; ++s) {
+    const T next = fma(cc.R, y, F[s]);
+    Bu[s] = fma(y, cc.G, Bu[s]);
+    F[s] = y;
+    y = next;
+  }
+  F[mc] = y;
+  const T last = Bu[mc] + y * cc.Gl;
+  T x = last;  // with zero x past the line's end
+  for (int s = mc - 1; s >= 0; --s) x = fma(cc.R, x, Bu[s]);
+  x *= cc.inv_close;  // x of the line's first cell
+  Bu[mc] = x;
+  x = fma(cc.Rl, x, last);
+  for (int s = mc - 1; s >= 0; --s) {
+    const T next = fma(cc.R, x, Bu[s]);
+    Bu[s] = x;
+    x = next;
+  }
+}
+
 // Right-hand side c + ea (ab - 2 c) from c and its neighbours' sum ab: a uniform
 // field comes back unchanged whatever ea is. DIVIDED: by ea, one operation less
 // (kappa scales the solution back). The weight 1/ea - 2 is rounded, an error of ea
@@ -839,6 +869,7 @@ __device__ __forceinline__ T half_step(const LineCoef<T>& k, T c, T ab) {
 }
 constexpr double kMaxDivided = 4.0;
 
+// B: batches of 32 segments in pass 2's scan, 0: a thread per line.
 // MODE: 0 no explicit part, 1 along the solved axis, 2 along another one; 3 and 4 as
 // 1 and 2 with the divided half step.
 template <typename T, int LS, int B, int MODE, bool X>
@@ -857,7 +888,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512)
   T* sF = W + kCarryW;
   T* sB = sF + nl * ns;
   T* tile = sF + (2 * nl * ns + V - 1) / V * V;
-  if (tid < 33) W[tid] = pow_bits<6>(cc.Rp, tid);
+  if (B > 0 && tid < 33) W[tid] = pow_bits<6>(cc.Rp, tid);
   pdl_wait();
   pdl_launch_next();
 
@@ -957,8 +988,12 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512)
   }
   __syncthreads();
   // pass 2
-  for (int q = tid >> 5; q < nl; q += nt >> 5) 
-    carry_scan<T, B>(ns - 1, cc, tid & 31, W, sF + q * ns, sB + q * ns);
+  if constexpr (B == 0) {
+    for (int q = tid; q < nl; q += nt) carry_serial(ns - 1, cc, sF + q * ns, sB + q * ns);
+  } else {
+    for (int q = tid >> 5; q < nl; q += nt >> 5)
+      carry_scan<T, B>(ns - 1, cc, tid & 31, W, sF + q * ns, sB + q * ns);
+  }
   __syncthreads();
   // pass 3
   T y = ok ? sF[ln * ns + sg] : T(0);
@@ -1171,6 +1206,8 @@ int32_t launch_fused(Lines L, const LineCoef<T>& k, double r, const T* in, T* ou
   auto kern = L.nseg <= 33 ? line_fused<T, LS, 1, MODE, X> : line_fused<T, LS, 2, MODE, X>;
   if constexpr (MAXB == 4)
     if (L.nseg > 65) kern = line_fused<T, LS, 4, MODE, X>;
+  if constexpr (LS < 32)
+    if (L.nseg <= kSerialSegs) kern = line_fused<T, LS, 0, MODE, X>;
   PPF_TRY_CUDA(allow_smem(kern, smem));
   PPF_TRY_CUDA(launch(kern, dim3((unsigned)ctas), dim3(threads), smem, st, true, L, k, cc, in, out,
                       nl, vec_ok));

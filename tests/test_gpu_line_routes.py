@@ -1,0 +1,26 @@
+"""Periodic line solves at the edges of the one-launch kernel's rules."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_line_alpha import TOL, solve
+from tests.test_gpu_line_fused import A, reference
+
+pytestmark = pytest.mark.gpu
+
+
+def check(shape, axis, f, eaxes=(-1, 0, 1)):
+    c0 = np.random.default_rng(shape[0] + shape[1]).random(shape)
+    if f == "f32":
+        c0 = c0.astype(np.float32).astype(np.float64)
+    for eaxis in eaxes:
+        got, ref = solve(c0, axis, A, eaxis, A, f), reference(c0, axis, eaxis)
+        err = np.linalg.norm(got - ref) / np.linalg.norm(ref)
+        assert err < TOL[f], (shape, axis, eaxis, err)
+
+
+# eight segments (a thread per line closes the carries) and nine, of 8 and of 16 cells
+@pytest.mark.parametrize("n, lines", [(3, 300), (63, 7), (64, 130), (65, 33), (128, 9000), (129, 9000)])
+@pytest.mark.parametrize("f", ["f32", "f64"])
+def test_short_lines(cuda, n, lines, f):
+    check((n, lines), 0, f)
+    check((lines, n), 1, f)
