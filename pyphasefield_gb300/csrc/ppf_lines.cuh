@@ -31,7 +31,8 @@ __device__ __forceinline__ void copy16_async(T* dst, const T* src) {
 // Rows line0 .. line0 + nl - 1 (those below nlines; row = z * ny + y) of n cells
 // to the tile, `ns` segments per row. vec_ok: 16-byte aligned rows (a vector
 // that starts below n lies inside the row's pitch, a multiple of 4).
-// cell(row pointer, line, i, dst): forms a cell's value itself where given.
+// COPY: the cells themselves; else cell.at(row, line, i), or cell.vec(row, line, i, v)
+// for a whole vector.
 template <typename T, int LS, bool COPY, typename Cell>
 __device__ __forceinline__ void rows_in(T* tile, const T* __restrict__ in, int line0, int nl,
                                         int nlines, int n, int ns, int ny, int64_t pitch,
@@ -46,10 +47,14 @@ __device__ __forceinline__ void rows_in(T* tile, const T* __restrict__ in, int l
     T* dst = tile + (r * ns + c0 / LS) * PS + c0 % LS;
     if (COPY && vec_ok) {
       copy16_async(dst, row + c0);
+    } else if (!COPY && vec_ok && c0 + V <= n) {
+      typename LineVec<T>::type v;
+      cell.vec(row, line, c0, reinterpret_cast<T*>(&v));
+      *reinterpret_cast<typename LineVec<T>::type*>(dst) = v;
     } else {
 #pragma unroll
       for (int e = 0; e < V; ++e)
-        if (c0 + e < n) dst[e] = COPY ? __ldg(row + c0 + e) : cell(row, line, c0 + e);
+        if (c0 + e < n) dst[e] = COPY ? __ldg(row + c0 + e) : cell.at(row, line, c0 + e);
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");

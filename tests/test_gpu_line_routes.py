@@ -24,3 +24,11 @@ def check(shape, axis, f, eaxes=(-1, 0, 1)):
 def test_short_lines(cuda, n, lines, f):
     check((n, lines), 0, f)
     check((lines, n), 1, f)
+
+
+# the half step along another axis: vectors, a row's ragged end, rows off the boundary
+# (a pitch that is a multiple of 4 keeps every row of a 16-byte aligned field on it)
+@pytest.mark.parametrize("n", [4, 5, 127, 128, 130, 1100, 2047])
+@pytest.mark.parametrize("f", ["f32", "f64"])
+def test_half_step_along_another_axis(cuda, n, f):
+    check((37, n), 1, f, eaxes=(0,))
