@@ -1250,9 +1250,33 @@ template <typename T>
 int fused_segment(const Lines& L, bool x) {
   const int64_t cells = (int64_t)L.nlines * L.n;
   if (L.n <= 512 && cells < (1 << 20)) return 8;
-  if (L.n > 1536) return 32;
+  if (L.n > (x && L.nlines < 300 ? 2048 : 1536)) return 32;
   if (sizeof(T) == 4 && (cells >= (1 << 22) || (!x && L.n > 1024))) return 32;
   return 16;
+}
+
+// Where the three launches are the faster ones: long lines of which a CTA holds one
+// (x) or a sector of columns, with too few of them to hide a thread's chain of 32
+// cells, or so many cells that loads bind. us per solve, one launch / three:
+//   x, beyond 2048 cells: double 30 x 3000 18.6 / 17.3, 30 x 4000 23.5 / 18.2,
+//     60 x 4000 20.5 / 18.1 but 100 x 4000 23.5 / 24.6, 500 x 3000 9 / 24; float
+//     without an explicit part 30 x 4000 6.7 / 6.2, 1000 x 2500 12.7 / 10.9 but
+//     300 x 4000 6.9 / 7.3. (A line alone takes one launch: 1 x 3000 1.2 times faster.)
+//   columns without an explicit part: float 3000^2 21.4 / 18.9, 2048^2 8.0 / 14.0,
+//     1500 x 8000 1.3 times slower than three; double 4000 x 30 31.2 / 22.6, 3000 x
+//     100 23.6 / 21.7, 2300 x 100 faster, 3000 x 8000 331 / 299, 1300 x 16000 1.23
+//     times slower, 700 x 16000 faster. With one: double 4000 x 30 40.9 / 36.4.
+template <typename T>
+bool three_launches(const Lines& L, int mode) {
+  const int64_t cells = (int64_t)L.nlines * L.n;
+  if (L.seglen == kXSegV) {
+    if (L.n <= 2048 || L.nlines == 1) return false;
+    return sizeof(T) == 8 ? L.nlines < 64 : mode == 0 && (L.nlines < 100 || L.nlines > 600);
+  }
+  if (mode == 2) return false;
+  if (sizeof(T) == 4) return mode == 0 && L.n > (cells > (1 << 23) ? 1200 : 2048);
+  if (mode == 1) return L.n > 3500 && L.nlines < 128;
+  return (L.n > 2560 && L.nlines < 256) || (L.n > 800 && cells > (1 << 23));
 }
 
 template <typename T, int MODE>
@@ -1320,13 +1344,9 @@ int32_t line_sweep(const Geo& g, int axis, double a, int eaxis, double ea, const
   CarryCoef<T> cc{};
   carry_coef(r, L.n, L.seglen, L.nseg, cc);
   for (int b = 0; b < 8; ++b) k.rbit[b] = (T)pow(r, (double)(1 << b));
-  // whole lines in one launch while a line's segments fit a CTA and the root is
-  // not close to 1 (kFusedMaxAlpha).
-  // Long float columns without an explicit part stay with the three launches:
-  // the CTA is then one per SM with nothing to hide its loads behind (3000^2:
-  // 21.4 against 18.9 us, 2048^2: 8.0 against 14.0)
-  const bool long_columns = sizeof(T) == 4 && mode == 0 && L.seglen == kSeg && L.n > 2048;
-  if (L.n <= 32 * kFusedSegs && a <= kFusedMaxAlpha && !long_columns) {
+  // whole lines in one launch while a line's segments fit a CTA, the root is not close
+  // to 1 and the three launches are not the faster ones
+  if (L.n <= 32 * kFusedSegs && a <= kFusedMaxAlpha && !three_launches<T>(L, mode)) {
     // every constant from the root as rounded to T, and kappa from the gain the
     // constants give a uniform field, so that it comes back unscaled: a
     // rounding of kappa itself would add up over the steps

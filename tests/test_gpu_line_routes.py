@@ -32,3 +32,16 @@ def test_short_lines(cuda, n, lines, f):
 @pytest.mark.parametrize("f", ["f32", "f64"])
 def test_half_step_along_another_axis(cuda, n, f):
     check((37, n), 1, f, eaxes=(0,))
+
+
+# lines of 1537 to 2048 cells by 16 (below 300 lines) and by 32 cells; longer ones on
+# both sides of the three launches' rule
+@pytest.mark.parametrize("n, lines", [(1600, 299), (1600, 300), (2048, 3), (2049, 1), (2049, 2),
+                                      (2100, 63), (2100, 64), (2100, 99), (2100, 100), (2100, 601),
+                                      (2561, 255), (2561, 256), (3501, 127), (3501, 128),
+                                      (1201, 7000), (801, 10500)])
+@pytest.mark.parametrize("f", ["f32", "f64"])
+def test_long_lines(cuda, n, lines, f):
+    eaxes = (-1, 0, 1) if lines >= 3 else (-1,)
+    check((n, lines), 0, f, eaxes=eaxes)
+    check((lines, n), 1, f, eaxes=eaxes)
