@@ -158,7 +158,10 @@ __global__ void __launch_bounds__(kThreads)
 // loaded by its first and last lane), and writes each output row as one
 // vector per lane: no shared memory, no barriers.
 //
-// Bound: HBM on grids beyond L2, the latency of one round of loads below.
+// Bound: HBM on grids beyond L2, the latency of one round of loads below; in double the
+// FP64 units. (So the ghost columns' rule is applied where a strip has one alone: as an
+// addition of zero elsewhere it was a sixth of the double additions, 8192^2 656 us with
+// the tiles before, 772 with it, 649 without.)
 // The grid's edges therefore take the same path: a ghost row is read from
 // its source row and fixed after the load (AxisRule), a ghost column is one
 // more load of the lane beside it (ColumnRule), and a vector that reaches
@@ -171,7 +174,7 @@ __global__ void __launch_bounds__(kThreads)
 // Two rows per warp: the halo rows are shared through the caches, and the
 // four times as many warps hide the latency better than eight rows' deeper
 // batch of loads does (eight rows: 256^2 3.2 us, 1024^2 3.3, 4096^2 22.0,
-// 8192^2 79.7; float64 1024^2 17.6 against 14.7).
+// 8192^2 79.7; float64 1024^2 17.6 against 14.7, 13.5 since).
 constexpr int kRB = 2;
 
 template <typename T, typename Op>
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(kThreads)
   const bool first = lane == 0;                                // loads the west neighbour
   const bool last = x < nx && (lane == 31 || x + V >= nx);     // loads the east neighbour
   const ColumnRule<T, 1> wr(g, bc, x0 - 1), er(g, bc, min(x0 + WW, nx));
+  const bool x_ghost = wr.ghost || er.ghost;  // uniform across the warp
   T c[RB + 2][V], wv[RB], ev[RB];
 #pragma unroll
   for (int j = 0; j < RB + 2; ++j) {
@@ -218,8 +222,10 @@ __global__ void __launch_bounds__(kThreads)
   }
 #pragma unroll
   for (int j = 0; j < RB; ++j) {
-    wv[j] = wr.value(0, wv[j]);
-    ev[j] = er.value(0, ev[j]);
+    if (x_ghost) {
+      wv[j] = wr.value(0, wv[j]);
+      ev[j] = er.value(0, ev[j]);
+    }
     if (last) {  // the ghost column inside the last lane's vector
 #pragma unroll
       for (int e = 1; e < V; ++e)
