@@ -558,7 +558,7 @@ class GB300Engine:
         for k, v in self.user_data.items():
             t = type(v)
             if t in _PLAIN:
-                v = (t, v)
+                v = (t, v or repr(v))  # 0.0 == -0.0, which are not the same constant
             elif isinstance(v, np.ndarray):
                 v = (v.shape, v.dtype.str,
                      hashlib.sha1(np.ascontiguousarray(v).tobytes()).hexdigest())

@@ -177,3 +177,13 @@ def test_choices_cached_for_other_kernels_are_not_taken(monkeypatch):
         e._ppf_autotune()
         old = autotune.make_key(name, (64, 64), torch.float32, "2")
         assert (keys[name] == old) == (name == "Warren1995GB300")
+
+
+def test_the_state_key_tells_zeros_apart():
+    e = Engine()
+    e.dt, e.dx, e._ppf_bc = 0.1, 1.0, L.PpfBoundary()
+    keys = []
+    for v in (0.0, -0.0, 0, False, None, "", "0.0", 1, 1.0, True):
+        e.user_data["v"] = v
+        keys.append(e._ppf_state_key())
+    assert len(set(keys)) == len(keys)
