@@ -11,6 +11,7 @@ from pyphasefield_gb300.engines import base
 
 class Stream:
     cuda_stream = 7
+    device = types.SimpleNamespace(index=1)
 
 
 class Engine(base.GB300Engine):
@@ -32,33 +33,28 @@ class Engine(base.GB300Engine):
         pass
 
 
-@pytest.fixture
-def log(monkeypatch):
-    """Library calls and the streams they were issued under."""
-    out = []
-    active = []
-
-    @contextlib.contextmanager
-    def stream(s):
-        active.append(s)
-        yield
-        active.pop()
-
-    monkeypatch.setattr(base.torch.cuda, "stream", stream)
-    monkeypatch.setattr(base.L, "call", lambda name, *a: out.append((name, list(active))))
-    return out
-
-
-def test_counter_is_set_with_the_engines_device_current(log):
-    """A launch into a stream of another device than the current one is
-    refused; torch.cuda.stream makes the stream's device current."""
+@pytest.mark.parametrize("current", [0, 1])
+def test_counter_is_set_with_the_engines_device_current(monkeypatch, current):
+    """A launch into a stream of another device than the current one is refused."""
     class Noisy(Engine):
         USES_STEP = True
 
+    log, devices = [], [current]
+
+    @contextlib.contextmanager
+    def enter(s):
+        devices.append(getattr(s, "device", s).index)
+        yield
+        devices.pop()
+
+    monkeypatch.setattr(base.torch.cuda, "current_device", lambda: devices[-1])
+    monkeypatch.setattr(base.torch.cuda, "device", enter)
+    monkeypatch.setattr(base.torch.cuda, "stream", enter)
+    monkeypatch.setattr(base.L, "call", lambda name, *a: log.append((name, devices[-1])))
     e = Noisy(graph_chunk=4, check_status=False)
     e._ppf_advance(8, 3)
     assert [n for n, _ in log] == ["ppf_counter_set_u64", "ppf_graph_launch", "ppf_graph_launch"]
-    assert log[0][1] == [e._ppf_stream]
+    assert log[0][1] == 1 and devices == [current]
 
 
 @pytest.mark.parametrize("done", [0, 1, 2, 3])
