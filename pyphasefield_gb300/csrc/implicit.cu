@@ -11,10 +11,11 @@
 //   x_i = y_i + r x_{i+1}           (cyclic backward recurrence)
 // Both recurrences contract (|r| < 1). Each line is cut into segments; a
 // segment's local sums with zero carry (pass 1), a short per-line pass that
-// closes the cyclic carries in double (pass 2), and a pass that recomputes
-// each segment from its true carries (pass 3) give the exact solution with
-// three streaming kernels (12 bytes of traffic per cell and float); lines of up
-// to 4096 cells run the three passes in one launch (line_fused).
+// closes the cyclic carries in the field's type, from constants formed in double
+// (pass 2), and a pass that recomputes each segment from its true carries (pass 3)
+// give the exact solution with three streaming kernels (12 bytes of traffic per
+// cell and float). Lines of up to 4096 cells run the three passes in one launch
+// (line_fused) where that is as exact (alpha up to 128) and faster (three_launches).
 //   - lines along y or z: one thread per (column, 32-cell segment), threads
 //     of a warp on adjacent columns, so every load and store is coalesced;
 //   - lines along x: one warp per 256-cell segment, cell i of a 32-cell
@@ -732,7 +733,8 @@ __global__ void __launch_bounds__(128)
 //   pass 1  every thread: the segment's local sums F, Bu (as line_sums_yz)
 //   pass 2  a warp per line: the cyclic carries, one weighted scan up and one
 //           down over the segments, closed afterwards by what the closing
-//           adds (R^(s+1) times the start value) instead of a second scan
+//           adds (R^(s+1) times the start value) instead of a second scan; lines
+//           of few segments by a thread each (carry_serial)
 //   pass 3  every thread: the segment from its true carries
 // Lines along y / z: `nl` adjacent columns per CTA (at least one 32-byte sector
 // wide), read and written directly. Lines along x: rows come through shared
@@ -740,8 +742,10 @@ __global__ void __launch_bounds__(128)
 // both the 16-byte row accesses and the threads' 16-byte segment accesses are
 // free of bank conflicts).
 //
-// Bound: the FP64 units in double (seven operations per cell with an explicit
-// half step, five without), latency and L2 in float. us per solve with the
+// Bound: in double the FP64 units (seven operations per cell with a divided
+// explicit half step, five without), busy for half of a 1024 x 1400 solve's time,
+// and the threads' chains at a quarter of the SMs' warps in one wave and a
+// remainder; latency and L2 in float. us per solve with the
 // explicit half step, three launches -> one: 256^2 float 11.2 -> 2.3 (along
 // x 5.4 -> 2.5) and double 32.8 -> 5.0 (13.9 -> 6.4), 1024^2 float 11.9 ->
 // 4.0 (8.3 -> 4.9) and double 44.5 -> 21.4 (58.8 -> 24.8), 256^3 float 82 ->

@@ -583,10 +583,8 @@ __device__ __forceinline__ double ch_mu(const ChCoef<double>& k, double c, doubl
   return fp - k.kap * lap;
 }
 
-template <typename T, bool QUANT>
+template <typename T>
 __device__ __forceinline__ T ch_flux(const ChCoef<T>& k, T mn, T mc) {
-  // (a d) / q == (a / q) d bit for bit: scaling by a power of two is exact
-  if (QUANT) return rint(k.aiq * (mn - mc)) * k.q;
   return k.a * (mn - mc);
 }
 
@@ -707,7 +705,7 @@ __global__ void __launch_bounds__(kThreads)
       c1[q] = P1[i];
       // flux through the face below z0, stored negated as "flux into the
       // cell below from above": the loop takes fd = -fup
-      fup[q] = -ch_flux<T, false>(k, mum, mu0[q]);
+      fup[q] = -ch_flux(k, mum, mu0[q]);
     }
     if (has_ring) M0[rmi] = mu_at(Pm1, P0, P1, rci);
   }
@@ -777,11 +775,11 @@ __global__ void __launch_bounds__(kThreads)
     for (int q = 0; q < kCQ; ++q) {
       const int i = mi + q * 8 * kMW;
       const T m0 = mu0[q];
-      const T fw = ch_flux<T, false>(k, M0[i - 1], m0);
-      const T fe = ch_flux<T, false>(k, M0[i + 1], m0);
-      const T fn = ch_flux<T, false>(k, M0[i - kMW], m0);
-      const T fs = ch_flux<T, false>(k, M0[i + kMW], m0);
-      const T fu = ch_flux<T, false>(k, mup[q], m0);
+      const T fw = ch_flux(k, M0[i - 1], m0);
+      const T fe = ch_flux(k, M0[i + 1], m0);
+      const T fn = ch_flux(k, M0[i - kMW], m0);
+      const T fs = ch_flux(k, M0[i + kMW], m0);
+      const T fu = ch_flux(k, mup[q], m0);
       const T fd = -fup[q];
       const T v = c0[q] + (((fw + fe) + (fn + fs)) + (fd + fu));
       if (full || q < nq) {
@@ -823,11 +821,11 @@ __global__ void __launch_bounds__(kThreads)
 // negated by the other (x across lanes through the neighbour's mu). The columns
 // beside the strip come as 24 side cells per plane, from which lanes 0 .. 7 form
 // the eight mu values the strip's outer faces need. Nothing but a warp's own
-// copies is waited for. The arithmetic is packed (FP32x2) and rounds as
-// ch_mu / ch_flux do, so both kernels give the same bits.
+// copies is waited for. The arithmetic is packed (FP32x2) and rounds as ch_mu and
+// ch_flux do.
 //
 // Bound: instruction issue and latency at 12 warps per SM (registers, shared
-// memory); 29.6 M warp instructions per 256^3 step where the shared-memory tiles
+// memory); 26.5 M warp instructions per 256^3 step where the shared-memory tiles
 // of cahn_hilliard_kernel, which this replaced in float, took 62.5 M and a block
 // barrier per plane. us per step: 256^3 87 -> 42, 384^3 235 -> 130, 128^3 33 ->
 // 12, one plane of 1500 x 2000 40 -> 13.
@@ -857,7 +855,8 @@ __device__ __forceinline__ F2 ch_mu2(const ChCoef<float>& k, F2 c, F2 we, F2 ns,
   return fma2(c, w, sp(-k.kap) * lap);
 }
 
-// Fluxes from the differences of mu across the faces, as ch_flux.
+// Fluxes from the differences of mu across the faces, as ch_flux; QUANT: rounded to the
+// quantum ((a d) / q == (a / q) d bit for bit: scaling by a power of two is exact).
 template <bool QUANT>
 __device__ __forceinline__ float ch_scale(const ChCoef<float>& k, float d) {
   return QUANT ? rintf(k.aiq * d) * k.q : k.a * d;

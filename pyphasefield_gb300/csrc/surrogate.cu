@@ -509,7 +509,8 @@ __device__ __forceinline__ void store_pairs(const float (&acc)[2][4][4], const S
         const long long m = m0 + i * 16 + g + 8 * h, n = n0 + j * 8 + 2 * t;
         if (m < M && n < N) st.put2(m, n, acc[i][j][2 * h], acc[i][j][2 * h + 1], e[j][h]);
       }
-  }}
+  }
+}
 
 template <bool AK, bool BKC, typename ST>
 __global__ void __launch_bounds__(kGemmThreads)
@@ -1305,7 +1306,7 @@ __global__ void dwconv_bwd_weight_kernel(const float* __restrict__ dh, const flo
 }
 
 // Two channels of kDwTokens tokens in a row per thread (C even, 8-byte aligned rows):
-// each token of y is loaded three times instead of nine, and the weights once per
+// a segment's tokens take 18 loads of y instead of 36, and the weights one per
 // CTA, tap by tap in shared memory (in memory a channel's nine taps are together, and
 // a warp's reads of them cost more than its tokens). The same sums in the same order.
 // DATA: dy = dy_in + the transposed convolution of x (dwconv_bwd_data_kernel) and,
