@@ -130,10 +130,10 @@ __device__ __forceinline__ StridedIdx strided_index(const Lines& L) {
 }
 
 // Two adjacent cells (the second 0 when the column does not exist); the
-// offset is even, so the vector load is aligned.
-template <typename T>
+// offset is even, so the vector load is aligned where the field is (VEC).
+template <bool VEC, typename T>
 __device__ __forceinline__ void load2(const T* __restrict__ p, bool pair, T (&v)[2]) {
-  if (pair) {
+  if (VEC && pair) {
     if constexpr (sizeof(T) == 4) {
       const float2 q = __ldg(reinterpret_cast<const float2*>(p));
       v[0] = q.x, v[1] = q.y;
@@ -143,19 +143,20 @@ __device__ __forceinline__ void load2(const T* __restrict__ p, bool pair, T (&v)
     }
   } else {
     v[0] = __ldg(p);
-    v[1] = T(0);
+    v[1] = !VEC && pair ? __ldg(p + 1) : T(0);
   }
 }
 
-template <typename T>
+template <bool VEC, typename T>
 __device__ __forceinline__ void store2(T* p, bool pair, T a, T b) {
-  if (pair) {
+  if (VEC && pair) {
     if constexpr (sizeof(T) == 4)
       *reinterpret_cast<float2*>(p) = make_float2(a, b);
     else
       *reinterpret_cast<double2*>(p) = make_double2(a, b);
   } else {
     *p = a;
+    if (!VEC && pair) p[1] = b;
   }
 }
 
@@ -180,26 +181,26 @@ __device__ __forceinline__ EOff strided_eoffsets(const Lines& L, const StridedId
 }
 
 // Right-hand side of the cell pair at line position i (pointer p).
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 __device__ __forceinline__ void rhs2(const T* __restrict__ p, const Lines& L,
                                      const LineCoef<T>& k, const StridedIdx& id, int i,
                                      const EOff& e, T (&d)[2]) {
-  load2(p, id.pair, d);
+  load2<VEC>(p, id.pair, d);
   if (EXPL == 0) return;
   T a[2], b[2];
   if (EXPL == 1) {
     int64_t om, op;
     wrap_offsets(i, L.n, L.stride, om, op);
-    load2(p + om, id.pair, a);
-    load2(p + op, id.pair, b);
+    load2<VEC>(p + om, id.pair, a);
+    load2<VEC>(p + op, id.pair, b);
   } else if (L.e_is_x) {
     a[0] = __ldg(p + e.m[0]);
     b[0] = __ldg(p + e.p[0]);
     a[1] = id.pair ? __ldg(p + 1 + e.m[1]) : T(0);
     b[1] = id.pair ? __ldg(p + 1 + e.p[1]) : T(0);
   } else {
-    load2(p + e.m[0], id.pair, a);
-    load2(p + e.p[0], id.pair, b);
+    load2<VEC>(p + e.m[0], id.pair, a);
+    load2<VEC>(p + e.p[0], id.pair, b);
   }
 #pragma unroll
   for (int c = 0; c < 2; ++c) d[c] = k.w0 * d[c] + k.w1 * (a[c] + b[c]);
@@ -207,7 +208,7 @@ __device__ __forceinline__ void rhs2(const T* __restrict__ p, const Lines& L,
 
 // Pass 1: per segment, y's end value with zero carry (F) and the sum of
 // r^(i - start) y_i over the segment (Bu).
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 __global__ void __launch_bounds__(kLineThreads)
     line_sums_yz(Lines L, LineCoef<T> k, const T* __restrict__ in,
                  typename V2<T>::type* __restrict__ seg) {
@@ -222,12 +223,12 @@ __global__ void __launch_bounds__(kLineThreads)
   T d[kSeg][2];
   if (len == kSeg) {
 #pragma unroll
-    for (int j = 0; j < kSeg; ++j) rhs2<T, EXPL>(p + (int64_t)j * L.stride, L, k, id, i0 + j, e, d[j]);
+    for (int j = 0; j < kSeg; ++j) rhs2<T, EXPL, VEC>(p + (int64_t)j * L.stride, L, k, id, i0 + j, e, d[j]);
   } else {
 #pragma unroll
     for (int j = 0; j < kSeg; ++j) {
       if (j < len)
-        rhs2<T, EXPL>(p + (int64_t)j * L.stride, L, k, id, i0 + j, e, d[j]);
+        rhs2<T, EXPL, VEC>(p + (int64_t)j * L.stride, L, k, id, i0 + j, e, d[j]);
       else
         d[j][0] = d[j][1] = T(0);
     }
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(kLineThreads)
 }
 
 // Pass 3: the segment again, from its true carries.
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 __global__ void __launch_bounds__(kLineThreads)
     line_solve_yz(Lines L, LineCoef<T> k, const T* __restrict__ in,
                   const typename V2<T>::type* __restrict__ seg, T* __restrict__ out) {
@@ -267,12 +268,12 @@ __global__ void __launch_bounds__(kLineThreads)
   if (len == kSeg) {
 #pragma unroll
     for (int j = 0; j < kSeg; ++j)
-      rhs2<T, EXPL>(in + off0 + (int64_t)j * L.stride, L, k, id, i0 + j, e, y[j]);
+      rhs2<T, EXPL, VEC>(in + off0 + (int64_t)j * L.stride, L, k, id, i0 + j, e, y[j]);
   } else {
 #pragma unroll
     for (int j = 0; j < kSeg; ++j) {
       if (j < len)
-        rhs2<T, EXPL>(in + off0 + (int64_t)j * L.stride, L, k, id, i0 + j, e, y[j]);
+        rhs2<T, EXPL, VEC>(in + off0 + (int64_t)j * L.stride, L, k, id, i0 + j, e, y[j]);
       else
         y[j][0] = y[j][1] = T(0);
     }
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(kLineThreads)
     if (j < len) {
       x0 = fma(k.r, x0, y[j][0]);
       x1 = fma(k.r, x1, y[j][1]);
-      store2(out + off0 + (int64_t)j * L.stride, id.pair, k.kappa * x0, k.kappa * x1);
+      store2<VEC>(out + off0 + (int64_t)j * L.stride, id.pair, k.kappa * x0, k.kappa * x1);
     }
   }
 }
@@ -323,10 +324,15 @@ __device__ __forceinline__ XIdx x_index(const Lines& L) {
 }
 
 // Cells i .. i+3 of a row (i a multiple of 4, so the 16 or 32 bytes are
-// aligned: the pitch is a multiple of 4). Cells at or past n read 0; a
-// vector that starts below n lies inside the row's pitch.
-template <typename T>
+// aligned where the field is, VEC: the pitch is a multiple of 4). Cells at or past n
+// read 0; a vector that starts below n lies inside the row's pitch.
+template <bool VEC, typename T>
 __device__ __forceinline__ void load4(const T* __restrict__ row, int i, int n, T (&v)[4]) {
+  if constexpr (!VEC) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = i + k < n ? __ldg(row + i + k) : T(0);
+    return;
+  }
   if (i >= n) {
     v[0] = v[1] = v[2] = v[3] = T(0);
     return;
@@ -345,14 +351,14 @@ __device__ __forceinline__ void load4(const T* __restrict__ row, int i, int n, T
 }
 
 // Right-hand side of the segment's cells: d[c][k] = cell 128c + 4 lane + k.
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 __device__ __forceinline__ void x_rhs(const T* __restrict__ in, const Lines& L,
                                       const LineCoef<T>& k, const XIdx& id,
                                       T (&d)[kXC][4]) {
   const T* row = in + id.row;
   const int i0 = id.s * kXSegV;
 #pragma unroll
-  for (int c = 0; c < kXC; ++c) load4(row, i0 + 128 * c + 4 * id.lane, L.n, d[c]);
+  for (int c = 0; c < kXC; ++c) load4<VEC>(row, i0 + 128 * c + 4 * id.lane, L.n, d[c]);
   if (EXPL == 0) return;
   if (EXPL == 2) {
     int64_t em, ep;
@@ -362,8 +368,8 @@ __device__ __forceinline__ void x_rhs(const T* __restrict__ in, const Lines& L,
     for (int c = 0; c < kXC; ++c) {
       T a[4], b[4];
       const int i = i0 + 128 * c + 4 * id.lane;
-      load4(row + em, i, L.n, a);
-      load4(row + ep, i, L.n, b);
+      load4<VEC>(row + em, i, L.n, a);
+      load4<VEC>(row + ep, i, L.n, b);
 #pragma unroll
       for (int q = 0; q < 4; ++q) d[c][q] = k.w0 * d[c][q] + k.w1 * (a[q] + b[q]);
     }
@@ -444,7 +450,7 @@ __device__ __forceinline__ T x_forward(const T (&d)[4], T carry, int nv, T w4j,
   return __shfl_sync(kFull, sel, (nv - 1) >> 2);
 }
 
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 __global__ void __launch_bounds__(kLineThreads)
     line_sums_x(Lines L, LineCoef<T> k, const T* __restrict__ in,
                 typename V2<T>::type* __restrict__ seg) {
@@ -453,7 +459,7 @@ __global__ void __launch_bounds__(kLineThreads)
   const XIdx id = x_index(L);
   if (!id.ok) return;
   T d[kXC][4];
-  x_rhs<T, EXPL>(in, L, k, id, d);
+  x_rhs<T, EXPL, VEC>(in, L, k, id, d);
   const int i0 = id.s * kXSegV;
   const T w4j = pow_bits<5>(k.rbit + 2, id.lane);  // r^(4 lane)
   T carry = 0, bu = 0, pwk = 1;
@@ -480,7 +486,7 @@ __global__ void __launch_bounds__(kLineThreads)
   if (id.lane == 0) seg[(int64_t)id.s * L.nlines + id.line] = {carry, bu};
 }
 
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 __global__ void __launch_bounds__(kLineThreads)
     line_solve_x(Lines L, LineCoef<T> k, const T* __restrict__ in,
                  const typename V2<T>::type* __restrict__ seg, T* __restrict__ out) {
@@ -489,7 +495,7 @@ __global__ void __launch_bounds__(kLineThreads)
   const XIdx id = x_index(L);
   if (!id.ok) return;
   T y[kXC][4];
-  x_rhs<T, EXPL>(in, L, k, id, y);
+  x_rhs<T, EXPL, VEC>(in, L, k, id, y);
   const typename V2<T>::type cr = seg[(int64_t)id.s * L.nlines + id.line];
   const int i0 = id.s * kXSegV;
   const int base = 4 * id.lane;
@@ -532,7 +538,7 @@ __global__ void __launch_bounds__(kLineThreads)
       }
       carry = __shfl_sync(kFull, x[0], 0);
       const int i = i0 + 128 * c + base;
-      if (base + 3 < nv) {
+      if (VEC && base + 3 < nv) {
         if constexpr (sizeof(T) == 4) {
           *reinterpret_cast<float4*>(row + i) =
               make_float4(k.kappa * x[0], k.kappa * x[1], k.kappa * x[2], k.kappa * x[3]);
@@ -1176,17 +1182,18 @@ cudaError_t launch_carry(const Lines& L, const CarryCoef<T>& cc, typename V2<T>:
   return launch(line_carry<T>, grid, block, 0, st, true, L, cc, seg);
 }
 
-template <typename T, int EXPL>
+template <typename T, int EXPL, bool VEC>
 int32_t launch_line(const Lines& L, const LineCoef<T>& k, const CarryCoef<T>& cc, const T* in,
                     T* out, typename V2<T>::type* seg, cudaStream_t st) {
   if (L.seglen == kXSegV) {
     const int64_t warps = (int64_t)L.nlines * L.nseg;
     const dim3 grid((unsigned)((warps + kLineThreads / 32 - 1) / (kLineThreads / 32)));
     if (grid.x > 0x7fffffffu) return fail(PPF_ERR_INVALID, "grid too large");
-    PPF_TRY_CUDA(launch(line_sums_x<T, EXPL>, grid, dim3(kLineThreads), 0, st, true, L, k, in, seg));
-    PPF_TRY_CUDA(launch_carry<T>(L, cc, seg, st));
     PPF_TRY_CUDA(
-        launch(line_solve_x<T, EXPL>, grid, dim3(kLineThreads), 0, st, true, L, k, in, seg, out));
+        launch(line_sums_x<T, EXPL, VEC>, grid, dim3(kLineThreads), 0, st, true, L, k, in, seg));
+    PPF_TRY_CUDA(launch_carry<T>(L, cc, seg, st));
+    PPF_TRY_CUDA(launch(line_solve_x<T, EXPL, VEC>, grid, dim3(kLineThreads), 0, st, true, L, k,
+                        in, seg, out));
     return PPF_OK;
   }
   const int64_t so = (int64_t)L.nseg * L.no;
@@ -1195,11 +1202,23 @@ int32_t launch_line(const Lines& L, const LineCoef<T>& k, const CarryCoef<T>& cc
   if (gz > 65535) return fail(PPF_ERR_INVALID, "grid too large for the line solver");
   const int pairs = (L.nx + 1) / 2;
   const dim3 grid((pairs + kLineThreads - 1) / kLineThreads, gy, gz);
-  PPF_TRY_CUDA(launch(line_sums_yz<T, EXPL>, grid, dim3(kLineThreads), 0, st, true, L, k, in, seg));
-  PPF_TRY_CUDA(launch_carry<T>(L, cc, seg, st));
   PPF_TRY_CUDA(
-      launch(line_solve_yz<T, EXPL>, grid, dim3(kLineThreads), 0, st, true, L, k, in, seg, out));
+      launch(line_sums_yz<T, EXPL, VEC>, grid, dim3(kLineThreads), 0, st, true, L, k, in, seg));
+  PPF_TRY_CUDA(launch_carry<T>(L, cc, seg, st));
+  PPF_TRY_CUDA(launch(line_solve_yz<T, EXPL, VEC>, grid, dim3(kLineThreads), 0, st, true, L, k, in,
+                      seg, out));
   return PPF_OK;
+}
+
+// The same with vectors of two cells (columns) or four (x, as 16 bytes each) where the
+// fields lie on their boundary, else cell by cell.
+template <typename T, int EXPL>
+int32_t launch_line_any(const Lines& L, const LineCoef<T>& k, const CarryCoef<T>& cc, const T* in,
+                        T* out, typename V2<T>::type* seg, cudaStream_t st) {
+  const uintptr_t need = L.seglen == kXSegV ? 16 : 2 * sizeof(T);
+  const bool vec = (uintptr_t)in % need == 0 && (uintptr_t)out % need == 0;
+  return vec ? launch_line<T, EXPL, true>(L, k, cc, in, out, seg, st)
+             : launch_line<T, EXPL, false>(L, k, cc, in, out, seg, st);
 }
 
 template <typename T>
@@ -1349,8 +1368,10 @@ int32_t line_sweep(const Geo& g, int axis, double a, int eaxis, double ea, const
   carry_coef(r, L.n, L.seglen, L.nseg, cc);
   for (int b = 0; b < 8; ++b) k.rbit[b] = (T)pow(r, (double)(1 << b));
   // whole lines in one launch while a line's segments fit a CTA, the root is not close
-  // to 1 and the three launches are not the faster ones
-  if (L.n <= 32 * kFusedSegs && a <= kFusedMaxAlpha && !three_launches<T>(L, mode)) {
+  // to 1 and the three launches are not the faster ones (they need the scratch aligned)
+  const bool seg_ok = (uintptr_t)scratch % (2 * sizeof(T)) == 0;
+  if (L.n <= 32 * kFusedSegs && a <= kFusedMaxAlpha &&
+      !(seg_ok && three_launches<T>(L, mode))) {
     // every constant from the root as rounded to T, and kappa from the gain the
     // constants give a uniform field, so that it comes back unscaled: a
     // rounding of kappa itself would add up over the steps
@@ -1373,11 +1394,13 @@ int32_t line_sweep(const Geo& g, int axis, double a, int eaxis, double ea, const
       default: return launch_fused_axis<T, 2>(L, kf, rt, in, out, st);
     }
   }
+  if (!seg_ok)
+    return fail(PPF_ERR_INVALID, "scratch must be %zu-byte aligned", 2 * sizeof(T));
   auto* seg = static_cast<typename V2<T>::type*>(scratch);
   switch (mode) {
-    case 0: return launch_line<T, 0>(L, k, cc, in, out, seg, st);
-    case 1: return launch_line<T, 1>(L, k, cc, in, out, seg, st);
-    default: return launch_line<T, 2>(L, k, cc, in, out, seg, st);
+    case 0: return launch_line_any<T, 0>(L, k, cc, in, out, seg, st);
+    case 1: return launch_line_any<T, 1>(L, k, cc, in, out, seg, st);
+    default: return launch_line_any<T, 2>(L, k, cc, in, out, seg, st);
   }
 }
 
