@@ -70,9 +70,10 @@ def time_candidate(run, stream: torch.cuda.Stream, warmup: int = 2, reps: int = 
     return e0.elapsed_time(e1) / 1e3 / reps
 
 
-def pick(key: str, candidates: list, measure) -> dict:
+def pick(key: str, candidates: list, measure, slack: float = 0.0) -> dict:
     """Return the cached best candidate for `key`, or time every candidate
-    with measure(candidate) -> seconds per unit of work and cache the best."""
+    with measure(candidate) -> seconds per unit of work and cache the best:
+    the fastest, or the first that takes no more than 1 + slack of its time."""
     mkey = (str(cache_path()), key)
     with _lock:
         hit = _memory.get(mkey)
@@ -89,7 +90,8 @@ def pick(key: str, candidates: list, measure) -> dict:
             continue
     if not results:
         raise RuntimeError(f"no autotune candidate ran for {key}")
-    best_t, best = min(results, key=lambda r: r[0])
+    fastest = min(t for t, _ in results)
+    best_t, best = next(r for r in results if r[0] <= fastest * (1.0 + slack))
     entry = {"config": best, "seconds": best_t,
              "tried": [{"config": c, "seconds": t} for t, c in results]}
     with _lock:
