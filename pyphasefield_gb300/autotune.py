@@ -70,10 +70,9 @@ def time_candidate(run, stream: torch.cuda.Stream, warmup: int = 2, reps: int = 
     return e0.elapsed_time(e1) / 1e3 / reps
 
 
-def pick(key: str, candidates: list, measure, slack: float = 0.0) -> dict:
+def pick(key: str, candidates: list, measure) -> dict:
     """Return the cached best candidate for `key`, or time every candidate
-    with measure(candidate) -> seconds per unit of work and cache the best:
-    the fastest, or the first that takes no more than 1 + slack of its time."""
+    with measure(candidate) -> seconds per unit of work and cache the best."""
     mkey = (str(cache_path()), key)
     with _lock:
         hit = _memory.get(mkey)
@@ -90,8 +89,7 @@ def pick(key: str, candidates: list, measure, slack: float = 0.0) -> dict:
             continue
     if not results:
         raise RuntimeError(f"no autotune candidate ran for {key}")
-    fastest = min(t for t, _ in results)
-    best_t, best = next(r for r in results if r[0] <= fastest * (1.0 + slack))
+    best_t, best = min(results, key=lambda r: r[0])
     entry = {"config": best, "seconds": best_t,
              "tried": [{"config": c, "seconds": t} for t, c in results]}
     with _lock:

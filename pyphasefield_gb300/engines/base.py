@@ -300,9 +300,6 @@ class GB300Engine:
     #: part of the autotuner's cache key, changed with the kernels behind the
     #: candidates: a choice cached for others is made anew
     TUNE_KERNELS = ""
-    #: what the first candidates, the engine's own choice, may take more than
-    #: the fastest: candidates of the same passes differ by the timer's spread
-    TUNE_SLACK = 0.0
 
     def _ppf_autotune(self):
         """Pick tile / temporal depth by timing candidates on scratch copies
@@ -336,7 +333,7 @@ class GB300Engine:
             return autotune.time_candidate(run, s) / depth
 
         try:
-            best = autotune.pick(key, cands, measure, self.TUNE_SLACK)
+            best = autotune.pick(key, cands, measure)
         finally:
             self.user_data.update(saved)
         self.user_data.update(best)

@@ -168,7 +168,6 @@ class _DiffusionMixin(GB300Engine):
     NFIELDS = 1
     USES_STEP = False
     TUNE_KERNELS = "|register blocks, z marches"
-    TUNE_SLACK = 0.05
 
     def __init__(self, **kwargs):
         super().__init__(**kwargs)
@@ -271,7 +270,6 @@ class _CahnAllenMixin(_ImplicitPhase, GB300Engine):
     NFIELDS = 1
     USES_STEP = False
     TUNE_KERNELS = "|register blocks, z marches"
-    TUNE_SLACK = 0.05
     PHASE_MODEL = L.PPF_MODEL_ALLEN_CAHN
 
     def __init__(self, **kwargs):
