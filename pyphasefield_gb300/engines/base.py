@@ -318,6 +318,8 @@ class GB300Engine:
             scratch = [[t.clone() for t in self._ppf_bufs[self._ppf_cur]] for _ in range(2)]
         saved = {k: self.user_data.get(k) for c in cands for k in c}
 
+        timed = {}  # seconds per step of the passes timed so far
+
         def measure(cand):
             self.user_data.update(cand)
             # the passes a long run consists of
@@ -330,7 +332,12 @@ class GB300Engine:
                 self._ppf_step(scratch[flip[0]], scratch[1 - flip[0]], depth, 0, None, sp)
                 flip[0] ^= 1
 
-            return autotune.time_candidate(run, s) / depth
+            # candidates of the same passes (a depth that is the engine's own) tie,
+            # and the first of them is taken
+            passes = repr((depth, self.user_data.get("tile"), self.user_data.get("zchunk")))
+            if passes not in timed:
+                timed[passes] = autotune.time_candidate(run, s) / depth
+            return timed[passes]
 
         try:
             best = autotune.pick(key, cands, measure)
