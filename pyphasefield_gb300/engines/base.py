@@ -336,7 +336,9 @@ class GB300Engine:
             # and the first of them is taken
             passes = repr((depth, self.user_data.get("tile"), self.user_data.get("zchunk")))
             if passes not in timed:
-                timed[passes] = autotune.time_candidate(run, s) / depth
+                with torch.cuda.stream(s):
+                    run()  # a shape the kernel refuses ends here
+                timed[passes] = self._ppf_time(run) / depth
             return timed[passes]
 
         try:
@@ -345,6 +347,21 @@ class GB300Engine:
             self.user_data.update(saved)
         self.user_data.update(best)
         self._ppf_graphs_reset()
+
+    def _ppf_time(self, run, passes: int = 8) -> float:
+        """Seconds of one run() on the engine's stream, `passes` of them issued
+        as a captured graph where the engine's runs are: launched one by one a
+        small grid's passes would be timed by the host."""
+        from .. import autotune
+        if not self.user_data.get("use_graph", True):
+            return autotune.time_candidate(run, self._ppf_stream)
+        g = self._ppf_capture(lambda: [run() for _ in range(passes)])
+        try:
+            sp = C.c_void_p(self._ppf_stream.cuda_stream)
+            return autotune.time_candidate(lambda: L.call("ppf_graph_launch", g, sp),
+                                           self._ppf_stream, reps=5) / passes
+        finally:
+            L.call("ppf_graph_destroy", g)
 
     def _ppf_graphs_reset(self):
         self._ppf_release_graphs()
@@ -584,18 +601,10 @@ class GB300Engine:
             items.append((str(k), v))
         return (tuple(items), repr(self.dt), repr(self.dx), bytes(self._ppf_bc))
 
-    def _ppf_graph(self, depths: tuple[int, ...]):
-        key = (self._ppf_cur, depths, self._ppf_state_key())
-        g = self._ppf_graphs.get(key)
-        if g is not None:
-            self._ppf_graphs.move_to_end(key)
-            return g
-        while len(self._ppf_graphs) >= MAX_GRAPHS:
-            L.call("ppf_graph_destroy", self._ppf_graphs.popitem(last=False)[1])
+    def _ppf_capture(self, issue):
+        """Executable graph of the launches issue() makes on the engine's stream."""
         s = self._ppf_stream
         sp = C.c_void_p(s.cuda_stream)
-        cur0 = self._ppf_cur
-        total = sum(depths)
         # No Python garbage collection while capturing: collecting another
         # engine would free its pinned staging buffers and graphs, and those
         # CUDA calls would invalidate the capture.
@@ -605,18 +614,39 @@ class GB300Engine:
         exec_ = C.c_void_p()
         try:
             with torch.cuda.stream(s):
-                self._ppf_segment_begin(total, s)
-                self._ppf_launch_passes(depths, 0, self._ppf_stepctr if self.USES_STEP else None)
-                if self.USES_STEP:
-                    L.call("ppf_counter_add_u64", ptr(self._ppf_stepctr), C.c_uint64(total), sp)
-                self._ppf_watch(s)
+                issue()
         finally:
             try:
                 L.call("ppf_graph_end", sp, C.byref(exec_))
             finally:
-                self._ppf_cur = cur0
                 if gc_was_enabled:
                     gc.enable()
+        return exec_
+
+    def _ppf_graph(self, depths: tuple[int, ...]):
+        key = (self._ppf_cur, depths, self._ppf_state_key())
+        g = self._ppf_graphs.get(key)
+        if g is not None:
+            self._ppf_graphs.move_to_end(key)
+            return g
+        while len(self._ppf_graphs) >= MAX_GRAPHS:
+            L.call("ppf_graph_destroy", self._ppf_graphs.popitem(last=False)[1])
+        s = self._ppf_stream
+        cur0 = self._ppf_cur
+        total = sum(depths)
+
+        def issue():
+            self._ppf_segment_begin(total, s)
+            self._ppf_launch_passes(depths, 0, self._ppf_stepctr if self.USES_STEP else None)
+            if self.USES_STEP:
+                L.call("ppf_counter_add_u64", ptr(self._ppf_stepctr), C.c_uint64(total),
+                       C.c_void_p(s.cuda_stream))
+            self._ppf_watch(s)
+
+        try:
+            exec_ = self._ppf_capture(issue)
+        finally:
+            self._ppf_cur = cur0
         self._ppf_graphs[key] = exec_
         return exec_
 

@@ -136,7 +136,7 @@ def test_candidates_are_timed_at_the_depth_they_run_at(monkeypatch, precision):
     import pyphasefield_gb300 as P
     from pyphasefield_gb300 import autotune
     e = P.DiffusionGB300(dimensions=[64, 64], dx=1.0, dt=0.1, boundary_conditions="PERIODIC",
-                         user_data={"precision": precision})
+                         user_data={"precision": precision, "use_graph": False})
     e._ppf_grid = types.SimpleNamespace(kshape=(64, 64))
     e._ppf_bc, e._ppf_stream, e._ppf_cur = L.PpfBoundary(), Stream(), 0
     e._ppf_bufs = [[torch.zeros(4)], [torch.zeros(4)]]
@@ -153,7 +153,8 @@ def test_candidates_are_timed_at_the_depth_they_run_at(monkeypatch, precision):
             depth = max(e._ppf_passes(64))
             assert seconds == 1.0 / depth, c
             if (depth, c["tile"]) not in seen:
-                assert timed.pop() == depth, c
+                assert timed == [depth, depth], c  # once before it is timed
+                timed.clear()
             seen.add((depth, c["tile"]))
         return cands[0]
 
@@ -170,10 +171,12 @@ def test_the_engines_own_choice_wins_against_its_own_passes(monkeypatch, tmp_pat
     monkeypatch.setenv("PPF_AUTOTUNE_CACHE", str(tmp_path / "tune.json"))
     monkeypatch.setattr(autotune, "_memory", {})
     monkeypatch.setattr(base.torch.cuda, "stream", lambda s: contextlib.nullcontext())
-    e = P.DiffusionGB300(dimensions=[64, 64], dx=1.0, dt=0.1, boundary_conditions="PERIODIC")
+    e = P.DiffusionGB300(dimensions=[64, 64], dx=1.0, dt=0.1, boundary_conditions="PERIODIC",
+                         user_data={"use_graph": False})
     e._ppf_grid, e._ppf_bc = types.SimpleNamespace(kshape=(64, 64)), L.PpfBoundary()
     e._ppf_stream, e._ppf_cur = Stream(), 0
     e._ppf_bufs = [[torch.zeros(4)], [torch.zeros(4)]]
+    e._ppf_step = lambda *a: None
     spread = iter([2.0, 1.9])
 
     def time_candidate(run, s):
@@ -210,3 +213,27 @@ def test_the_state_key_tells_zeros_apart():
         e.user_data["v"] = v
         keys.append(e._ppf_state_key())
     assert len(set(keys)) == len(keys)
+
+
+def test_candidates_are_timed_as_graphs(monkeypatch):
+    """Passes launched one by one would be timed by the host on a small grid."""
+    import pyphasefield_gb300 as P
+    from pyphasefield_gb300 import autotune
+    e = P.DiffusionGB300(dimensions=[64, 64, 64], dx=1.0, dt=0.1, boundary_conditions="PERIODIC")
+    e._ppf_grid, e._ppf_bc = types.SimpleNamespace(kshape=(64, 64, 64)), L.PpfBoundary()
+    e._ppf_stream, e._ppf_cur = Stream(), 0
+    e._ppf_bufs = [[torch.zeros(4)], [torch.zeros(4)]]
+    log = []
+    e._ppf_step = lambda *a: log.append("step")
+    monkeypatch.setattr(base.torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(base.L, "call", lambda name, *a: log.append(name))
+    monkeypatch.setattr(autotune, "time_candidate", lambda run, s, reps: [run(), 16.0][1])
+
+    def pick(key, cands, measure):
+        assert measure(cands[0]) == 2.0
+        return cands[0]
+
+    monkeypatch.setattr(autotune, "pick", pick)
+    e._ppf_autotune()
+    assert log == ["step", "ppf_graph_begin"] + ["step"] * 8 + [
+        "ppf_graph_end", "ppf_graph_launch", "ppf_graph_destroy"]
